@@ -18,6 +18,7 @@
 #include <type_traits>
 
 #include "mps_device.cuh"
+#include "mps_group.cuh"
 
 namespace mps {
 
@@ -39,10 +40,12 @@ template <class R, class RN> struct FluidKeySrc {
         int id = pid[t];
         int s = nscene > 1 ? scene_of(sc, nscene, id) : 0;
         V4<R> p = pos[t];
-        if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) atomicAdd(&cnt->err_nan, 1);
+        const bool fin = isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
+        if (!fin) atomicAdd(&cnt->err_nan, 1);
         bool ok;
         const int c = fine_cell(sc[s], p.x, p.y, p.z, ok);
         if (!ok) atomicAdd(&cnt->err_cell, 1);
+        if (!ok || !fin) cnt->off_grid = 1;
         return c;
     }
     __device__ __forceinline__ int id(int t) const { return pid[t]; }
@@ -684,14 +687,20 @@ __global__ void __launch_bounds__(T) k_fine_rows_write(FineRows f,
 // ---------------------------------------------------------------------------------------
 // neighbour passes
 // ---------------------------------------------------------------------------------------
-// Entry k of slot s's neighbour list. The 32 slots of a warp own one contiguous tile of
-// K x 32 entries, entry-major (a warp's entry k is one 128-byte line). A layout strided by the
-// slot count instead spreads a warp's lines over the whole list, so that each line leaves L2
-// between its lanes' partial writes and is written back several times (measured: about three
-// times the list's bytes in DRAM writes at 2.9M particles).
-__device__ __forceinline__ size_t list_at(int s, int k, int K) {
-    return (size_t(s >> 5) * size_t(K) + size_t(k)) * 32 + size_t(s & 31);
+// Entry k of slot s's neighbour list, T slots sharing runs of 32-entry lines with E = 32 / T
+// entries each (lt = log2 T). With one thread per slot T = 32: the warp's entries k are one line.
+// With a group of lanes per slot T = 4: a slot's next eight entries are one 32-byte sector, which
+// the group writes and reads whole. (A layout strided by the slot count spreads a warp's lines
+// over the whole list, so that each line leaves L2 between its lanes' partial writes: measured
+// about three times the list's bytes in DRAM writes at 2.9M particles.)
+constexpr int kListThread = 5, kListGroup = 2;
+__host__ __device__ __forceinline__ size_t list_at(int s, int k, int K, int lt) {
+    const int le = 5 - lt, e = (1 << le) - 1;
+    return (size_t(s >> lt) * size_t((K + e) >> le) + size_t(k >> le)) * 32 +
+           size_t(((s & ((1 << lt) - 1)) << le) + (k & e));
 }
+// entries that the lists of n slots at capacity K take, in either layout
+inline size_t list_size(size_t n, int K) { return (n + 31) / 32 * 32 * size_t((K + 7) / 8 * 8); }
 
 // Resident blocks per SM asked of a kernel tuned in FP32: half as many in FP64, whose values
 // take two registers each (at the FP32 bound the FP64 kernels spill).
@@ -735,11 +744,11 @@ template <class R, class RN> struct PassArgs {
     int32_t* diag;
     RN* ndens;
     // neighbour lists: entry k of slot s (its k-th neighbour in visiting order) is
-    // nb[list_at(s, k, nbK)]; nbcnt[s] is the list's length (lists longer than nbK fall back
+    // nb[list_at(s, k, nbK, lt)]; nbcnt[s] is the list's length (lists longer than nbK fall back
     // to a scan)
     int* nb;
     int* nbcnt;
-    int nbK;
+    int nbK, lt;
     const int8_t* near_wall;  // per bucket: a wall lies in the 27 buckets around it
     // per bucket: a mirror of the view `m` lies in the 27 buckets around it (null: walk
     // the mirrors everywhere). The wall and mirror walks visit only a particle's 27 buckets,
@@ -793,7 +802,7 @@ __device__ __forceinline__ bool near_flag(const int8_t* f, const SceneDev<R, RN>
 
 // Phase 1 of a neighbour pass: the fluid neighbours j != s with d2 <= thr, in visiting
 // order, into the slot's list. Returns the neighbour count (may exceed nbK).
-template <class R, class RN, bool COUNT = false>
+template <class R, class RN, bool COUNT, int LT>
 __device__ __forceinline__ int build_list(const PassArgs<R, RN>& a, const SceneDev<R, RN>& sc,
                                           const RowCtx<R>& c, int s, R x, R y, R z, R thr, R B,
                                           int* ncand = nullptr) {
@@ -811,7 +820,7 @@ __device__ __forceinline__ int build_list(const PassArgs<R, RN>& a, const SceneD
             R dx = q.x - x, dy = q.y - y, dz = q.z - z;
             const int j = w_slot(q.w);
             if (j != s && dot3(dx, dy, dz, dx, dy, dz) <= thr) {
-                if (cnt < K) nb[list_at(s, cnt, K)] = j;
+                if (cnt < K) nb[list_at(s, cnt, K, LT)] = j;
                 ++cnt;
             }
         };
@@ -864,19 +873,6 @@ struct StageHdr {
     int base[kStageRows + 1];  // staged index of each row's first candidate
     int tab[kStageRows * kStageCols];  // staged index of each fine cell start
 };
-
-__device__ __forceinline__ unsigned ord_bits(float f) {
-    const unsigned u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float ord_float(unsigned u) {
-    return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
-}
-// distance from [v0, v1] to fine cell f along one axis (fine_gap of the nearer end)
-__device__ __forceinline__ float fine_gap_box(float v0, float v1, int f, float hf) {
-    const float lo = float(f - 3) * hf;
-    return fmaxf(fmaxf(lo - v1, v0 - (lo + hf)), 0.0f);
-}
 
 template <class R> __host__ __device__ constexpr size_t stage_smem_bytes(int cap, bool vel) {
     return ((sizeof(StageHdr) + 15) / 16) * 16 + size_t(cap) * sizeof(V4<R>) * (vel ? 2 : 1);
@@ -1050,7 +1046,7 @@ __device__ __forceinline__ void visc_walk(const PassArgs<R, RN>& a, const SceneD
         sx = fmaR(u.x - v.x, w, sx);
         sy = fmaR(u.y - v.y, w, sy);
         sz = fmaR(u.z - v.z, w, sz);
-        if (TAPE && cf < K) nb[list_at(s, cf, K)] = j;
+        if (TAPE && cf < K) nb[list_at(s, cf, K, a.lt)] = j;
         ++cf;
     };
     const V4<R> z4{R(0), R(0), R(0), R(0)};
@@ -1089,17 +1085,13 @@ __device__ __forceinline__ void warp_add_u64(unsigned long long* dst, int v) {
     if ((threadIdx.x & 31) == __ffs(m) - 1) atomicAdd(dst, (unsigned long long)tot);
 }
 
-// the rest of pass A for one particle once its fluid sum is known: mirrors (VelM = 0),
-// acceleration with gravity, kick/drift (UpPcl1) and ChkPcl, the scratch outputs
+// the rest of pass A for one particle once its sum is known: acceleration with gravity,
+// kick/drift (UpPcl1) and ChkPcl, the scratch outputs
 template <class R, class RN, bool DIAG, bool TAPE>
 __device__ __forceinline__ void pass_a_finish(const PassArgs<R, RN>& a, const SceneDev<R, RN>& sc,
                                               int s, int pid, const V4<R>& p, const V4<R>& v,
-                                              const RowCtx<R>& c, R sx, R sy, R sz, int cf) {
-    int cm = 0;
+                                              R sx, R sy, R sz, int cf, int cm) {
     if (TAPE) a.nbcnt[s] = cf;  // the recorded list (complete while cf <= nbK)
-    if (near_flag(a.near_m, sc, c))
-        visc_sum_mirrors(sc, c, p.x, p.y, p.z, v.x, v.y, v.z, a.m, MPS_INF_SKIP(a, sc.skip_r), sx,
-                         sy, sz, cm);
     R ax = fmaR(sc.kn, sx, sc.g[0]), ay = fmaR(sc.kn, sy, sc.g[1]), az = fmaR(sc.kn, sz, sc.g[2]);
     R ux = fmaR(ax, sc.dt, v.x), uy = fmaR(ay, sc.dt, v.y), uz = fmaR(az, sc.dt, v.z);
     R x = fmaR(ux, sc.dt, p.x), y = fmaR(uy, sc.dt, p.y), z = fmaR(uz, sc.dt, p.z);
@@ -1130,19 +1122,9 @@ __device__ __forceinline__ void pass_a_unlisted(const PassArgs<R, RN>& a, int s,
     }
 }
 
-// pass A: VscTrm (kernel.cu:1013-1119) + UpPcl1/ChkPcl (kernel.cu:1138-1149, 481-513), each
-// particle walking its candidates in global memory (posf through L1).
-// TAPE (recorded rollouts): also keeps the list length and the velocity before the clamp.
-template <class R, class RN, bool DIAG, bool TAPE = false, int NB = 4, bool ALT = false>
-__global__ void __launch_bounds__(128, pass_a_blocks<R>(ALT))
-    k_pass_a(const __grid_constant__ PassArgs<R, RN> a) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.nF) return;
-    const int nalive = __ldg(a.cs + a.dead);
-    if (s >= nalive) {  // unlisted particles are carried over unchanged
-        pass_a_unlisted(a, s, TAPE);
-        return;
-    }
+// Pass A for one slot, walking its candidates in global memory (posf through L1)
+template <class R, class RN, bool DIAG, bool TAPE, int NB>
+__device__ __forceinline__ void pass_a_walk(const PassArgs<R, RN>& a, int s) {
     const int pid = a.pid[s];
     const SceneDev<R, RN>& sc = scene_ref(a, pid);
     V4<R> p = ldg4(a.pos + s), v = ldg4(a.vel + s);
@@ -1150,7 +1132,7 @@ __global__ void __launch_bounds__(128, pass_a_blocks<R>(ALT))
     cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
     RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
     R sx = 0, sy = 0, sz = 0;
-    int cf = 0, ncand = 0;
+    int cf = 0, cm = 0, ncand = 0;
     const V4<R>* __restrict__ posf = a.posf;
     const V4<R>* __restrict__ vel = a.vel;
     visc_walk<R, RN, TAPE, DIAG, NB>(
@@ -1158,7 +1140,25 @@ __global__ void __launch_bounds__(128, pass_a_blocks<R>(ALT))
         [&](auto&& f) { for_fluid_ranges(sc, a.csr, c, MPS_INF_SKIP(a, sc.skip_r), f); },
         [&](int k) { return ldg4(posf + k); }, [&](int, int j) { return ldg4(vel + j); });
     if (DIAG) warp_add_u64(&a.cnt->work[0], ncand);
-    pass_a_finish<R, RN, DIAG, TAPE>(a, sc, s, pid, p, v, c, sx, sy, sz, cf);
+    if (near_flag(a.near_m, sc, c))
+        visc_sum_mirrors(sc, c, p.x, p.y, p.z, v.x, v.y, v.z, a.m, MPS_INF_SKIP(a, sc.skip_r), sx,
+                         sy, sz, cm);
+    pass_a_finish<R, RN, DIAG, TAPE>(a, sc, s, pid, p, v, sx, sy, sz, cf, cm);
+}
+
+// pass A: VscTrm (kernel.cu:1013-1119) + UpPcl1/ChkPcl (kernel.cu:1138-1149, 481-513), each
+// particle walking its candidates with one thread.
+// TAPE (recorded rollouts): also keeps the list length and the velocity before the clamp.
+template <class R, class RN, bool DIAG, bool TAPE = false, int NB = 4, bool ALT = false>
+__global__ void __launch_bounds__(128, pass_a_blocks<R>(ALT))
+    k_pass_a(const __grid_constant__ PassArgs<R, RN> a) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= a.nF) return;
+    if (s >= __ldg(a.cs + a.dead)) {  // unlisted particles are carried over unchanged
+        pass_a_unlisted(a, s, TAPE);
+        return;
+    }
+    pass_a_walk<R, RN, DIAG, TAPE, NB>(a, s);
 }
 
 // pass A with the block's neighbourhood staged in shared memory (stage_fluid): positions,
@@ -1218,7 +1218,10 @@ __global__ void __launch_bounds__(128) k_pass_a_st(const __grid_constant__ PassA
             [&](int k) { return ldg4(posf + k); }, [&](int, int j) { return ldg4(vel + j); });
     }
     if (DIAG) warp_add_u64(&a.cnt->work[0], ncand);
-    pass_a_finish<R, RN, DIAG, false>(a, sc, s, pid, p, v, c, sx, sy, sz, cf);
+    int cm = 0;
+    if (near_flag(a.near_m, sc, c))
+        visc_sum_mirrors(sc, c, p.x, p.y, p.z, v.x, v.y, v.z, a.m, B, sx, sy, sz, cm);
+    pass_a_finish<R, RN, DIAG, false>(a, sc, s, pid, p, v, sx, sy, sz, cf, cm);
 }
 
 // pass B's stores: velocity after ChkCol, pressure from MkPrs's EOS, diagnostics
@@ -1259,19 +1262,9 @@ __device__ __noinline__ void pass_b_long(const PassArgs<R, RN>& a, int s) {
     pass_b_store<R, RN, DIAG>(a, sc, s, pid, wx, wy, wz, ni, cnt5);
 }
 
-// pass B: ChkCol (kernel.cu:1168-1287) + MkPrs (kernel.cu:1306-1411) at x*; leaves the
-// list of fluid neighbours inside max(rp, rlim) for pass C (same positions, same slots)
-template <class R, class RN, bool DIAG, bool ALT = false>
-__global__ void __launch_bounds__(128, pass_b_blocks<R>(ALT))
-    k_pass_b(const __grid_constant__ PassArgs<R, RN> a) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.nF) return;
-    const int nalive = __ldg(a.cs + a.dead);
-    if (s >= nalive) {
-        a.tvel[s] = a.vel[s];
-        a.tprs[s] = R(0);
-        return;
-    }
+// Pass B for one slot with one thread; LT: the lists' layout (list_at)
+template <class R, class RN, bool DIAG, int LT>
+__device__ __forceinline__ void pass_b_walk(const PassArgs<R, RN>& a, int s) {
     const int pid = a.pid[s];
     const SceneDev<R, RN>& sc = scene_ref(a, pid);
     V4<R> p = ldg4(a.pos + s), v = ldg4(a.vel + s);
@@ -1279,7 +1272,7 @@ __global__ void __launch_bounds__(128, pass_b_blocks<R>(ALT))
     cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
     RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
     int ncand = 0;
-    const int n = build_list<R, RN, DIAG>(a, sc, c, s, p.x, p.y, p.z, sc.list_thr,
+    const int n = build_list<R, RN, DIAG, LT>(a, sc, c, s, p.x, p.y, p.z, sc.list_thr,
                                           MPS_INF_SKIP(a, sc.skip_rc), &ncand);
     a.nbcnt[s] = n;
     if (DIAG) {
@@ -1293,10 +1286,10 @@ __global__ void __launch_bounds__(128, pass_b_blocks<R>(ALT))
     R wx = v.x, wy = v.y, wz = v.z;
     RN ni = 0;
     int cnt5[5] = {0, 0, 0, 0, 0};
-    const int* __restrict__ nb = a.nb + list_at(s, 0, a.nbK);
+    const int* __restrict__ nb = a.nb + list_at(s, 0, a.nbK, LT);
     const V4<R>* __restrict__ pos = a.pos;
     const V4<R>* __restrict__ vel = a.vel;
-    const int st = 32;
+    auto at = [](int k) { return (k >> (5 - LT)) * 32 + (k & ((32 >> LT) - 1)); };
     const R rlim2 = sc.rlim2, rp_lt = sc.rp_lt, colfac = sc.colfac, rp = sc.rp;
     const RN rp_n = sc.rp_n;
     auto add = [&](int j, const V4<R>& q) {
@@ -1314,8 +1307,8 @@ __global__ void __launch_bounds__(128, pass_b_blocks<R>(ALT))
     };
     int k = 0;
     for (; k + 4 <= n; k += 4) {
-        const int j0 = nb[k * st], j1 = nb[(k + 1) * st], j2 = nb[(k + 2) * st],
-                  j3 = nb[(k + 3) * st];
+        const int j0 = nb[at(k)], j1 = nb[at(k + 1)], j2 = nb[at(k + 2)],
+                  j3 = nb[at(k + 3)];
         V4<R> q0 = ldg4(pos + j0), q1 = ldg4(pos + j1), q2 = ldg4(pos + j2), q3 = ldg4(pos + j3);
         add(j0, q0);
         add(j1, q1);
@@ -1323,7 +1316,7 @@ __global__ void __launch_bounds__(128, pass_b_blocks<R>(ALT))
         add(j3, q3);
     }
     for (; k < n; ++k) {
-        const int j = nb[k * st];
+        const int j = nb[at(k)];
         add(j, ldg4(pos + j));
     }
     col_dens_walls_mirrors<R, RN, true, true>(sc, c, p.x, p.y, p.z, v.x, v.y, v.z, a.wl, a.m,
@@ -1331,6 +1324,21 @@ __global__ void __launch_bounds__(128, pass_b_blocks<R>(ALT))
                                               near_flag(a.near_wall, sc, c),
                                               near_flag(a.near_m, sc, c));
     pass_b_store<R, RN, DIAG>(a, sc, s, pid, wx, wy, wz, ni, cnt5);
+}
+
+// pass B: ChkCol (kernel.cu:1168-1287) + MkPrs (kernel.cu:1306-1411) at x*; leaves the
+// list of fluid neighbours inside max(rp, rlim) for pass C (same positions, same slots)
+template <class R, class RN, bool DIAG, bool ALT = false>
+__global__ void __launch_bounds__(128, pass_b_blocks<R>(ALT))
+    k_pass_b(const __grid_constant__ PassArgs<R, RN> a) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= a.nF) return;
+    if (s >= __ldg(a.cs + a.dead)) {
+        a.tvel[s] = a.vel[s];
+        a.tprs[s] = R(0);
+        return;
+    }
+    pass_b_walk<R, RN, DIAG, kListThread>(a, s);
 }
 
 // pass C's end for one slot: acceleration from the gradient sums, UpPcl2 (kick and drift),
@@ -1416,7 +1424,7 @@ __global__ void __launch_bounds__(128, pass_c_blocks<R>(ALT, CORR))
     RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
     G g;
     int cf = 0, cm = 0;
-    const int* __restrict__ nb = a.nb + list_at(s, 0, a.nbK);
+    const int* __restrict__ nb = a.nb + list_at(s, 0, a.nbK, kListThread);
     const V4<R>* __restrict__ pos = a.pos;
     const R* __restrict__ prs = a.tprs;
     const int st = 32;
@@ -1472,6 +1480,699 @@ __global__ void __launch_bounds__(128, pass_c_blocks<R>(ALT, CORR))
     if (near_flag(a.near_m, sc, c))
         grad_sum_mirrors(sc, c, pid - sc.pbase, p.x, p.y, p.z, pmin, a.m, a.skip != 0, g, cm);
     pass_c_finish<R, RN, DIAG, TAPE>(a, sc, s, pid, p, pi, g, cf, cm);
+}
+
+// ---------------------------------------------------------------------------------------
+// neighbour passes with a group of G lanes per particle (mps_group.cuh): small scenes
+// ---------------------------------------------------------------------------------------
+// Pair terms inside the common range by mps_exact.cuh (d2 >= lo), else by the general operations:
+// VscTrm's weight 2 l0 / (d^2 d) (kernel.cu:1062-1064), WEI_grad(d, re) (const.cuh:46)
+template <class R> __device__ __forceinline__ R visc_weight(R two_l0, R d2, R lo) {
+    if (d2 >= lo) return div_in(two_l0, d2 * sqrt_in(d2));
+    return two_l0 / (d2 * sqrtR(d2));
+}
+template <class R> __device__ __forceinline__ R wei_in(R d, R re, R inv_re) {
+    return div_in(re, d) - div_by(d, re, inv_re);
+}
+// MkPrs's term (kernel.cu:1346-1348)
+template <class R, class RN>
+__device__ __forceinline__ RN dens_term(const SceneDev<R, RN>& sc, R d2) {
+    RN t = RN(0);
+    if (!(d2 >= sc.pair_lo)) dens_add(sc, d2, t);
+    else if (sizeof(RN) == sizeof(R)) t = RN(wei_in(sqrt_in(d2), sc.rp, sc.inv_rp));
+    else t = wei_in(sqrt_in(RN(d2)), sc.rp_n, sc.inv_rp_n);
+    return t;
+}
+// PrsGrdTrm's weight WEI_grad(d, rp) / d^2 (kernel.cu:1731-1735)
+template <class R, class RN>
+__device__ __forceinline__ R grad_weight(const SceneDev<R, RN>& sc, R d2) {
+    if (d2 >= sc.pair_lo) return div_in(wei_in(sqrt_in(d2), sc.rp, sc.inv_rp), d2);
+    return wei_grad(sqrtR(d2), sc.rp) / d2;
+}
+
+// What a lane knows of its group's particle
+template <class R, class RN> struct GroupSlot {
+    const SceneDev<R, RN>* sc;
+    V4<R> p;
+    RowCtx<R> c;
+    int s, pid, row;
+    bool act;
+};
+// this group's slot, if it is listed
+template <class R, class RN, int G>
+__device__ __forceinline__ int group_slot(const Group<G>& gr) {
+    return int((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * Group<G>::P + gr.g;
+}
+template <class R, class RN>
+__device__ __forceinline__ GroupSlot<R, RN> group_load(const PassArgs<R, RN>& a, int s, bool act,
+                                                       const V4<R>* pos) {
+    GroupSlot<R, RN> t;
+    t.s = s;
+    t.act = act;
+    t.pid = act ? a.pid[s] : 0;
+    t.sc = &a.sc[act && a.nscene > 1 ? scene_of(a.sc, a.nscene, t.pid) : 0];
+    t.p = act ? ldg4(pos + s) : V4<R>{R(0), R(0), R(0), R(0)};
+    int ix = 0, iy = 0, iz = 0;
+    if (act) cell_of(*t.sc, t.p.x, t.p.y, t.p.z, ix, iy, iz);
+    t.c = row_ctx(*t.sc, t.p.x, t.p.y, t.p.z, ix, iy, iz);
+    t.row = t.sc->cbase + iz * t.sc->nbxy + iy * t.sc->nbx;
+    return t;
+}
+// whether the group walk does not cover this slot: a position off the grid, whose rows the union
+// would widen, or a scene whose sizes leave the range of mps_exact.cuh
+template <class R, class RN>
+__device__ __forceinline__ bool group_off(const PassArgs<R, RN>& a, int s) {
+    return a.cnt->off_grid != 0 || !scene_ref(a, a.pid[s]).pairs_ok;
+}
+// the scene of a set (its lanes share their bucket row)
+template <class R, class RN>
+__device__ __forceinline__ const SceneDev<R, RN>& group_scene(const PassArgs<R, RN>& a,
+                                                              const SceneDev<R, RN>* mine,
+                                                              const GroupSet& t) {
+    return a.sc[__shfl_sync(kFull, int(mine - a.sc), __ffs(t.lanes) - 1)];
+}
+template <class R> __device__ __forceinline__ R pair_d2(const V4<R>& q, const V4<R>& p) {
+    const R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+    return dot3(dx, dy, dz, dx, dy, dz);
+}
+
+template <class R, class RN, bool DIAG, bool TAPE>
+__device__ __noinline__ void pass_a_single(const PassArgs<R, RN>& a, int s) {
+    pass_a_walk<R, RN, DIAG, TAPE, 2>(a, s);
+}
+
+// pass A, G lanes per particle
+template <class R, class RN, bool DIAG, bool TAPE, int G>
+__global__ void __launch_bounds__(128) k_pass_a_g(const __grid_constant__ PassArgs<R, RN> a) {
+    using Mem = GroupMem<R, 32 / G, 4>;
+    __shared__ Mem mem[4];
+    Mem& m = mem[threadIdx.x >> 5];
+    const Group<G> gr;
+    const int s = group_slot<R, RN>(gr);
+    bool act = s < a.nF && s < __ldg(a.cs + a.dead);
+    if (s < a.nF && !act && gr.l == 0) pass_a_unlisted(a, s, TAPE);
+    if (act && group_off(a, s)) {
+        if (gr.l == 0) pass_a_single<R, RN, DIAG, TAPE>(a, s);
+        act = false;
+    }
+    unsigned pend = __ballot_sync(kFull, act);
+    if (pend == 0u) return;
+    const GroupSlot<R, RN> me = group_load(a, s, act, a.pos);
+    const SceneDev<R, RN>& sc = *me.sc;
+    const V4<R> p = me.p, v = act ? ldg4(a.vel + s) : p;
+    const bool nearm = act && near_flag(a.near_m, sc, me.c);
+    if (DIAG) {
+        int ncand = 0;
+        if (act && gr.l == 0)
+            for_fluid_ranges(sc, a.csr, me.c, MPS_INF_SKIP(a, sc.skip_r),
+                             [&](int lo, int hi) { ncand += hi - lo; });
+        warp_add_u64(&a.cnt->work[0], ncand);
+    }
+    const R two_l0 = sc.two_l0, lo = sc.pair_lo;
+    R sum = R(0);
+    int cf = 0, cm = 0;
+    while (pend) {
+        const GroupSet t = group_next(pend, me.row, me.c);
+        pend &= ~t.lanes;
+        const bool in = (t.lanes >> gr.lane) & 1u;
+        const SceneDev<R, RN>& ts = group_scene(a, me.sc, t);
+        const R B = MPS_INF_SKIP(a, ts.skip_r), r_le = ts.r_le, hi = ts.pair_hi;
+        const bool mirrors = __any_sync(kFull, in && nearm);
+        const GroupPts<R, 32 / G> pts(gr, p, s, t.lanes);
+        // the fluid, then the mirrors (VelM = 0, kernel.cu:834-836): one loop, one copy of the
+        // code in the instruction cache
+#pragma unroll 1
+        for (int kind = 0; kind < (mirrors ? 2 : 1); ++kind) {
+            const V4<R>* table = kind == 0 ? a.posf : a.m.pos;
+            int nrow, total;
+            if (kind == 0) group_fluid_rows(m, ts, a.csr, t, B, nrow, total);
+            else group_bucket_rows(m, ts, a.m.cs, t, B, nrow, total);
+#pragma unroll 1
+            for (int w0 = 0; w0 < total; w0 += Mem::kWindow) {
+                const int nl = group_list<G>(m, nrow, total, w0);
+                const int n = group_test(m, gr, table, nl, [&](int i, const V4<R>& q) {
+                    const R d2 = pts.d2(i, q);
+                    bool ok = pts.on(i) && d2 <= r_le && (kind == 1 || w_slot(q.w) != pts.s[i]);
+                    if (ok && d2 > hi)
+                        ok = bucket_adjacent(ts, pts.x[i], pts.y[i], pts.z[i], q.x, q.y, q.z);
+                    return ok;
+                });
+                group_sum(m, gr, n, sum, [&](int h, bool on, int k) {
+                    V4<R> x{R(0), R(0), R(0), R(0)};
+                    if (on) {
+                        const V4<R> q = ldg4(table + k);
+                        if (kind == 0) {
+                            const int j = w_slot(q.w);
+                            x = ldg4(a.vel + j);
+                            if (TAPE && cf + h < a.nbK) a.nb[list_at(s, cf + h, a.nbK, kListGroup)] = j;
+                        }
+                        x = V4<R>{x.x - v.x, x.y - v.y, x.z - v.z, visc_weight(two_l0, pair_d2(q, p), lo)};
+                    }
+                    return x;
+                });
+                if (kind == 0) cf += n;
+                else cm += n;
+            }
+        }
+    }
+    const R sx = gr.from(sum, 0), sy = gr.from(sum, 1), sz = gr.from(sum, 2);
+    if (act && gr.l == 0) pass_a_finish<R, RN, DIAG, TAPE>(a, sc, s, me.pid, p, v, sx, sy, sz, cf, cm);
+}
+
+// scratch of pass B: also MkPrs's terms, in its own arithmetic
+template <class R, class RN, int P> struct GroupMemB : GroupMem<R, P, 4> {
+    alignas(16) RN dens[P][kGroupPitch];
+};
+
+// ChkCol (with the velocity velo(k, q)) and, with `dens`, MkPrs over the cnt accepted candidates:
+// the collision terms that act (f > 0) are compacted and added by lanes 0-2, the density terms
+// by lane 3. keep(h, k, q) sees every accepted candidate.
+template <bool DIAG, int G, class R, class RN, class Velo, class Keep>
+__device__ __forceinline__ void group_col_dens(GroupMemB<R, RN, 32 / G>& m, const Group<G>& gr,
+                                               const SceneDev<R, RN>& sc, const V4<R>& p,
+                                               const V4<R>& v, const V4<R>* __restrict__ table,
+                                               int cnt, R rcol2, bool dens, R& sum, RN& ni, int& ncol,
+                                               int& nden, Keep&& keep, Velo&& velo) {
+    const int most = __reduce_max_sync(kFull, cnt);
+#pragma unroll 1
+    for (int h0 = 0; h0 < most; h0 += kGroupChunk) {
+        const int n = min(kGroupChunk, most - h0);
+        int nc = 0;
+#pragma unroll 1
+        for (int u = 0; u < n; u += G) {
+            const int h = h0 + u + gr.l;
+            V4<R> e{R(0), R(0), R(0), R(0)};
+            RN t = RN(0);
+            bool hit = false;
+            if (h < cnt) {
+                const int k = m.kidx[m.hit[gr.g][h]];
+                const V4<R> q = ldg4(table + k);
+                keep(h, k, q);
+                const R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+                const R d2 = dot3(dx, dy, dz, dx, dy, dz);
+                if (d2 < rcol2) {
+                    if (DIAG) ++ncol;
+                    const V4<R> w = velo(k, q);
+                    const R f = dot3(v.x - w.x, v.y - w.y, v.z - w.z, dx, dy, dz);
+                    hit = f > R(0);
+                    e = V4<R>{-dx, -dy, -dz, f * (sc.colfac / d2)};
+                }
+                if (dens && d2 <= sc.rp_lt) {
+                    t = dens_term(sc, d2);
+                    if (DIAG) ++nden;
+                }
+            }
+            m.dens[gr.g][u + gr.l] = t;
+            const unsigned all = __ballot_sync(kFull, hit);
+            if (all) {
+                const unsigned b = gr.mine(all);
+                if (hit) {
+                    const int at = nc + __popc(b & gr.below());
+                    m.term[0][gr.g][at] = e.x;
+                    m.term[1][gr.g][at] = e.y;
+                    m.term[2][gr.g][at] = e.z;
+                    m.term[3][gr.g][at] = e.w;
+                }
+                nc += __popc(b);
+            }
+        }
+        __syncwarp();
+        if (gr.l < 3) {
+            for (int i = 0; i < nc; ++i) sum = fmaR(m.term[gr.l][gr.g][i], m.term[3][gr.g][i], sum);
+        } else if (dens && gr.l == 3) {
+            for (int i = 0; i < n; i += 4) ni = add4(&m.dens[gr.g][i], ni);
+        }
+        __syncwarp();
+    }
+}
+
+template <class R, class RN, bool DIAG>
+__device__ __noinline__ void pass_b_single(const PassArgs<R, RN>& a, int s) {
+    pass_b_walk<R, RN, DIAG, kListGroup>(a, s);
+}
+
+// pass B, G lanes per particle
+template <class R, class RN, bool DIAG, int G>
+__global__ void __launch_bounds__(128) k_pass_b_g(const __grid_constant__ PassArgs<R, RN> a) {
+    using Mem = GroupMemB<R, RN, 32 / G>;
+    __shared__ Mem mem[4];
+    Mem& m = mem[threadIdx.x >> 5];
+    const Group<G> gr;
+    const int s = group_slot<R, RN>(gr);
+    bool act = s < a.nF && s < __ldg(a.cs + a.dead);
+    if (s < a.nF && !act && gr.l == 0) {
+        a.tvel[s] = a.vel[s];
+        a.tprs[s] = R(0);
+    }
+    if (act && group_off(a, s)) {
+        if (gr.l == 0) pass_b_single<R, RN, DIAG>(a, s);
+        act = false;
+    }
+    unsigned pend = __ballot_sync(kFull, act);
+    if (pend == 0u) return;
+    const GroupSlot<R, RN> me = group_load(a, s, act, a.pos);
+    const SceneDev<R, RN>& sc = *me.sc;
+    const V4<R> p = me.p, v = act ? ldg4(a.vel + s) : p;
+    const bool nearm = act && near_flag(a.near_m, sc, me.c),
+               nearw = act && near_flag(a.near_wall, sc, me.c);
+    if (DIAG) {
+        int ncand = 0;
+        if (act && gr.l == 0)
+            for_fluid_ranges(sc, a.csr, me.c, MPS_INF_SKIP(a, sc.skip_rc),
+                             [&](int lo, int hi) { ncand += hi - lo; });
+        warp_add_u64(&a.cnt->work[1], ncand);
+    }
+    R sum = gr.l == 0 ? v.x : (gr.l == 1 ? v.y : v.z);
+    RN ni = RN(0);
+    int cnt5[5] = {0, 0, 0, 0, 0}, have = 0, ncol = 0, nden = 0;
+    while (pend) {
+        const GroupSet t = group_next(pend, me.row, me.c);
+        pend &= ~t.lanes;
+        const bool in = (t.lanes >> gr.lane) & 1u;
+        const SceneDev<R, RN>& ts = group_scene(a, me.sc, t);
+        const R B = MPS_INF_SKIP(a, ts.skip_rc), thr = ts.list_thr, hi = ts.pair_hi;
+        const GroupPts<R, 32 / G> pts(gr, p, s, t.lanes);
+        const bool walls = __any_sync(kFull, in && nearw), mirrors = __any_sync(kFull, in && nearm);
+        // the fluid, the walls (collision only), the mirrors (at rest, kernel.cu:834-836)
+#pragma unroll 1
+        for (int kind = 0; kind < 3; ++kind) {
+            if ((kind == 1 && !walls) || (kind == 2 && !mirrors)) continue;
+            const V4<R>* table = kind == 0 ? a.posf : (kind == 1 ? a.wl.pos : a.m.pos);
+            const R rcol2 = kind == 1 ? ts.rlimw2 : ts.rlim2;
+            int nrow, total;
+            if (kind == 0)
+                group_fluid_rows(m, ts, a.csr, t, B, nrow, total);
+            else
+                group_bucket_rows(m, ts, kind == 1 ? a.wl.cs : a.m.cs, t,
+                                  kind == 1 ? MPS_INF_SKIP(a, ts.skip_rw) : B, nrow, total);
+#pragma unroll 1
+            for (int w0 = 0; w0 < total; w0 += Mem::kWindow) {
+                const int nl = group_list<G>(m, nrow, total, w0);
+                const int n = group_test(m, gr, table, nl, [&](int i, const V4<R>& q) {
+                    const R d2 = pts.d2(i, q);
+                    bool ok = pts.on(i) && (kind == 1 ? d2 < rcol2 : d2 <= thr) &&
+                              (kind != 0 || w_slot(q.w) != pts.s[i]);
+                    if (ok && d2 > hi)
+                        ok = bucket_adjacent(ts, pts.x[i], pts.y[i], pts.z[i], q.x, q.y, q.z);
+                    return ok;
+                });
+                group_col_dens<DIAG>(m, gr, sc, p, v, table, n, rcol2, kind != 1, sum, ni, ncol, nden,
+                                     [&](int h, int k, const V4<R>& q) {
+                                         if (kind == 0 && have + h < a.nbK)
+                                             a.nb[list_at(s, have + h, a.nbK, kListGroup)] = w_slot(q.w);
+                                     },
+                                     [&](int k, const V4<R>& q) {
+                                         V4<R> u{R(0), R(0), R(0), R(0)};
+                                         if (kind == 0) u = ldg4(a.vel + w_slot(q.w));
+                                         else if (kind == 1) u = ldg4(a.wl.vel + k);
+                                         return u;
+                                     });
+                if (kind == 0) have += n;
+            }
+            if (DIAG) {
+                if (kind == 0) { cnt5[0] += ncol; cnt5[3] += nden; }
+                else if (kind == 1) cnt5[1] += ncol;
+                else { cnt5[2] += ncol; cnt5[4] += nden; }
+                ncol = nden = 0;
+            }
+        }
+    }
+    const R wx = gr.from(sum, 0), wy = gr.from(sum, 1), wz = gr.from(sum, 2);
+    ni = gr.from(ni, 3);
+    if (DIAG) {
+        warp_add_u64(&a.cnt->work[2], act && gr.l == 0 ? have : 0);
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+            for (int o = G / 2; o > 0; o >>= 1) cnt5[i] += __shfl_xor_sync(kFull, cnt5[i], o);
+    }
+    if (act && gr.l == 0) {
+        a.nbcnt[s] = have;
+        pass_b_store<R, RN, DIAG>(a, sc, s, me.pid, wx, wy, wz, ni, cnt5);
+    }
+}
+
+// The gradient sums of a group: the plain variant's three as group_sum keeps them, the corrected
+// one's nine moments and three right-hand sides, sum q with lane q % G. A neighbour's term is
+// (dx, dy, dz, w (P_j - P_min)), the corrected one's (dx, dy, dz, w, P_j - P_min).
+template <class R, int G, bool CORR> struct GroupGrad {
+    static constexpr int NT = CORR ? 5 : 4, NQ = CORR ? (12 + G - 1) / G : 1;
+    R s[NQ] = {};
+    template <class M, class F>
+    __device__ __forceinline__ void add(M& m, const Group<G>& gr, int most, F&& f) {
+        for (int h0 = 0; h0 < most; h0 += kGroupChunk) {
+            const int n = min(kGroupChunk, most - h0);
+            for (int u = 0; u < n; u += G) {
+                R d[3] = {R(0), R(0), R(0)}, w = R(0), pd = R(0);
+                f(h0 + u + gr.l, d, w, pd);
+                m.term[0][gr.g][u + gr.l] = d[0];
+                m.term[1][gr.g][u + gr.l] = d[1];
+                m.term[2][gr.g][u + gr.l] = d[2];
+                m.term[3][gr.g][u + gr.l] = CORR ? w : pd * w;
+                if (CORR) m.term[NT - 1][gr.g][u + gr.l] = pd;
+            }
+            __syncwarp();
+            if (!CORR) {
+                if (gr.l < 3)
+                    for (int i = 0; i < n; i += 4)
+                        s[0] = chain4(&m.term[3][gr.g][i], &m.term[gr.l][gr.g][i], s[0]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < NQ; ++k) {
+                    const int q = gr.l + k * G;
+                    if (q < 12) {
+                        const R* x = m.term[q < 9 ? q / 3 : NT - 1][gr.g];
+                        const R* y = m.term[q % 3][gr.g];
+                        for (int i = 0; i < n; ++i) s[k] = fmaR(m.term[3][gr.g][i] * x[i], y[i], s[k]);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+    __device__ __forceinline__ R get(const Group<G>& gr, int q) const {
+        return gr.from(s[CORR ? q / G : 0], q % G);
+    }
+    __device__ __forceinline__ void to(const Group<G>& gr, GradPlain<R>& g) const {
+        g.sx = get(gr, 0); g.sy = get(gr, 1); g.sz = get(gr, 2);
+    }
+    __device__ __forceinline__ void to(const Group<G>& gr, GradCorr<R>& g) const {
+        g.m0 = get(gr, 0); g.m1 = get(gr, 1); g.m2 = get(gr, 2); g.m3 = get(gr, 3); g.m4 = get(gr, 4);
+        g.m5 = get(gr, 5); g.m6 = get(gr, 6); g.m7 = get(gr, 7); g.m8 = get(gr, 8);
+        g.b0 = get(gr, 9); g.b1 = get(gr, 10); g.b2 = get(gr, 11);
+    }
+};
+
+// pass C, G lanes per particle, over the lists that pass B left
+template <class R, class RN, bool DIAG, bool TAPE, bool CORR, int G>
+__global__ void __launch_bounds__(128) k_pass_c_g(const __grid_constant__ PassArgs<R, RN> a) {
+    using GA = typename std::conditional<CORR, GradCorr<R>, GradPlain<R>>::type;
+    using Sums = GroupGrad<R, G, CORR>;
+    using Mem = GroupMem<R, 32 / G, Sums::NT>;
+    __shared__ Mem mem[4];
+    Mem& m = mem[threadIdx.x >> 5];
+    const Group<G> gr;
+    const int s = group_slot<R, RN>(gr);
+    bool act = s < a.nF && s < __ldg(a.cs + a.dead);
+    if (s < a.nF && !act && gr.l == 0) {
+        a.tpos[s] = a.pos[s];
+        a.ttyp[s] = a.typ[s];
+        if (TAPE) a.tape_pre[s] = V4<R>{R(0), R(0), R(0), R(kTapeDead)};
+    }
+    const int n = act ? a.nbcnt[s] : 0;
+    if (act && (n > a.nbK || group_off(a, s))) {  // the walk over the fine rows: any position
+        if (gr.l == 0) pass_c_long<R, RN, DIAG, TAPE, GA>(a, s);
+        act = false;
+    }
+    unsigned pend = __ballot_sync(kFull, act);
+    if (pend == 0u) return;
+    const GroupSlot<R, RN> me = group_load(a, s, act, a.pos);
+    const SceneDev<R, RN>& sc = *me.sc;
+    const V4<R> p = me.p;
+    const R pi = act ? a.tprs[s] : R(0);
+    const int cnt = act ? n : 0, most = __reduce_max_sync(kFull, cnt);
+    const int* __restrict__ nb = a.nb + list_at(s, 0, a.nbK, kListGroup);
+    auto entry = [&](int h) { return __ldg(nb + 4 * (h & ~7) + (h & 7)); };
+    const R rp2 = sc.rp2;
+    // P_min over the fluid neighbours inside rp (order-free), then the gradient in order
+    R pmin = pi;
+    for (int h = gr.l; h < cnt; h += G) {
+        const int j = entry(h);
+        const R pj = __ldg(a.tprs + j);
+        if (pair_d2(ldg4(a.pos + j), p) < rp2 && pj < pmin) pmin = pj;
+    }
+    for (int o = G / 2; o > 0; o >>= 1) {
+        const R x = __shfl_xor_sync(kFull, pmin, o);
+        if (x < pmin) pmin = x;
+    }
+    Sums sums;
+    int cf = 0, cm = 0;
+    sums.add(m, gr, most, [&](int h, R(&d)[3], R& w, R& pd) {
+        if (h >= cnt) return;
+        const int j = entry(h);
+        const V4<R> q = ldg4(a.pos + j);
+        const R pj = __ldg(a.tprs + j);
+        const R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+        const R d2 = dot3(dx, dy, dz, dx, dy, dz);
+        if (d2 < rp2) {
+            d[0] = dx; d[1] = dy; d[2] = dz;
+            w = grad_weight(sc, d2);
+            pd = pj - pmin;
+            if (DIAG) ++cf;
+        }
+    });
+    const bool nearm = act && near_flag(a.near_m, sc, me.c);
+    if (!__any_sync(kFull, nearm)) pend = 0u;
+    const int skip_slot = me.pid - sc.pbase + kNumMRR * sc.pbase;  // kernel.cu:1759
+    while (pend) {
+        const GroupSet t = group_next(pend, me.row, me.c);
+        pend &= ~t.lanes;
+        const bool in = (t.lanes >> gr.lane) & 1u;
+        if (!__any_sync(kFull, in && nearm)) continue;
+        const SceneDev<R, RN>& ts = group_scene(a, me.sc, t);
+        const GroupPts<R, 32 / G> pts(gr, p, s, t.lanes);
+        int nrow, total;
+        group_bucket_rows(m, ts, a.m.cs, t, MPS_INF_SKIP(a, ts.skip_rp), nrow, total);
+        for (int w0 = 0; w0 < total; w0 += Mem::kWindow) {
+            const int nl = group_list<G>(m, nrow, total, w0);
+            const int nm = group_test(m, gr, a.m.pos, nl, [&](int i, const V4<R>& q) {
+                return pts.on(i) && pts.d2(i, q) < ts.rp2;
+            });
+            sums.add(m, gr, __reduce_max_sync(kFull, nm), [&](int h, R(&d)[3], R& w, R& pd) {
+                if (h >= nm) return;
+                const int k = m.kidx[m.hit[gr.g][h]];
+                if (__ldg(a.m.slot + k) == skip_slot) return;
+                const V4<R> q = ldg4(a.m.pos + k);
+                d[0] = q.x - p.x; d[1] = q.y - p.y; d[2] = q.z - p.z;
+                w = grad_weight(sc, dot3(d[0], d[1], d[2], d[0], d[1], d[2]));
+                pd = q.w - pmin;
+                if (DIAG) ++cm;
+            });
+        }
+    }
+    GA g;
+    sums.to(gr, g);
+    if (DIAG)
+        for (int o = G / 2; o > 0; o >>= 1) {
+            cf += __shfl_xor_sync(kFull, cf, o);
+            cm += __shfl_xor_sync(kFull, cm, o);
+        }
+    if (act && gr.l == 0) pass_c_finish<R, RN, DIAG, TAPE>(a, sc, s, me.pid, p, pi, g, cf, cm);
+}
+
+// ---- mirror generation with a group of lanes per particle ---------------------------------
+// scratch: also the distinct normals met, [0] of all walls, [1] of Edge walls, in order of arrival
+template <class R, int P> struct GroupMemG : GroupMem<R, P, 1> {
+    R n[2][P][kNumMRR][3];
+    int id[2][P][kNumMRR];
+};
+
+// One mirror of particle (x, y, z): its reflection through the plane of wall position q with
+// normal n, as emit_mirrors writes it. False when the particle lies behind the plane (a face's
+// plane takes pw = NaN, the corner's does not, as there).
+template <class R>
+__device__ __forceinline__ bool mirror_of(R x, R y, R z, const V4<R>& q, const V4<R>& n, bool corner,
+                                          V4<R>& out, R& nlen) {
+    const R pwx = x - q.x, pwy = y - q.y, pwz = z - q.z;
+    const R pw = dot3(pwx, pwy, pwz, n.x, n.y, n.z);
+    if (corner ? !(pw >= R(0)) : pw < R(0)) return false;
+    nlen = sqrtR(dot3(n.x, n.y, n.z, n.x, n.y, n.z));
+    const R t2 = R(2) * (pw / nlen);
+    out.x = fmaR(-t2, n.x, q.x + pwx);
+    out.y = fmaR(-t2, n.y, q.y + pwy);
+    out.z = fmaR(-t2, n.z, q.z + pwz);
+    return true;
+}
+
+template <class R, class RN, bool TAPE>
+__device__ __noinline__ int gen_single(const PassArgs<R, RN>& a, int s, V4<R> p, R P) {
+    const int pid = a.pid[s];
+    const SceneDev<R, RN>& sc = scene_ref(a, pid);
+    int ix, iy, iz;
+    cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
+    const RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
+    MirrorPlan<R> pl;
+    const int nw = plan_mirrors(sc, c, p.x, p.y, p.z, a.wl, a.skip != 0, pl);
+    const int m = count_mirrors<R, RN>(pl, p.x, p.y, p.z, a.wl, a.cnt);
+    if (m > 0)
+        emit_mirrors<R, RN, TAPE>(pl, p.x, p.y, p.z, P, pid * kNumMRR, a.wl, a.out, a.cnt,
+                                  atomicAdd(&a.cnt->mirror_raw, m));
+    return nw;
+}
+
+// k_gen_cull with G lanes per particle: the walls inside r are found together, the distinct
+// normals registered by ballots (the first lane with a new normal registers it for the group),
+// and one lane per registered normal makes its mirror.
+template <class R, class RN, bool DIAG, bool TAPE, int G>
+__global__ void __launch_bounds__(128) k_gen_cull_g(const __grid_constant__ PassArgs<R, RN> a,
+                                                    const V4<R>* gpos, const R* gprs,
+                                                    const int8_t* gtyp) {
+    using Mem = GroupMemG<R, 32 / G>;
+    __shared__ Mem mem[4];
+    Mem& m = mem[threadIdx.x >> 5];
+    const Group<G> gr;
+    const int s = group_slot<R, RN>(gr);
+    const bool fld = s < a.nF && gtyp[s] == kFLD;
+    const GroupSlot<R, RN> me = group_load(a, s, fld, gpos);
+    const SceneDev<R, RN>& sc = *me.sc;
+    const V4<R> p = me.p;
+    // no wall in the 27 buckets around: no wall within r, no mirror (the common case)
+    bool act = fld && __ldg(a.near_wall + me.row + me.c.ix);
+    const R P = act ? (gprs ? gprs[s] : slot_w(s, R(0))) : R(0);
+    int nwall = 0;
+    if (act && group_off(a, s)) {
+        if (gr.l == 0) nwall = gen_single<R, RN, TAPE>(a, s, p, P);
+        act = false;
+    }
+    unsigned pend = __ballot_sync(kFull, act);
+    int nn[2] = {0, 0}, corner = -1;
+    V4<R> cn{R(0), R(0), R(0), R(0)};  // the corner mirror's plane normal
+    while (pend) {
+        const GroupSet t = group_next(pend, me.row, me.c);
+        pend &= ~t.lanes;
+        const bool in = (t.lanes >> gr.lane) & 1u;
+        const SceneDev<R, RN>& ts = group_scene(a, me.sc, t);
+        const GroupPts<R, 32 / G> pts(gr, p, s, t.lanes);
+        int nrow, total, n = 0;
+        group_bucket_rows(m, ts, a.wl.cs, t, MPS_INF_SKIP(a, ts.skip_r), nrow, total);
+        auto walls = [&](int w0) {
+            const int nl = group_list<G>(m, nrow, total, w0);
+            return group_test(m, gr, a.wl.pos, nl, [&](int i, const V4<R>& q) {
+                const R d2 = pts.d2(i, q);
+                bool ok = pts.on(i) && d2 <= ts.r2;
+                if (ok && d2 > ts.pair_hi)
+                    ok = bucket_adjacent(ts, pts.x[i], pts.y[i], pts.z[i], q.x, q.y, q.z);
+                return ok;
+            });
+        };
+        for (int w0 = 0; w0 < total; w0 += Mem::kWindow) {
+            n = walls(w0);
+            nwall += n;
+            const int most = __reduce_max_sync(kFull, n);
+            for (int h0 = 0; h0 < most; h0 += G) {
+                const int h = h0 + gr.l;
+                const bool on = h < n;
+                const int j = on ? m.kidx[m.hit[gr.g][h]] : 0;
+                const V4<R> nv = ldg4(a.wl.nrm + j);
+                const bool edge = on && __ldg(a.wl.wse + j) == kEDGE;
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    bool fresh = e == 0 ? on : edge;
+                    fresh = fresh && nn[e] < kNumMRR;
+                    for (int k = 0; k < nn[e]; ++k) {
+                        const R* w = m.n[e][gr.g][k];
+                        fresh = fresh && !(w[0] == nv.x && w[1] == nv.y && w[2] == nv.z);
+                    }
+                    unsigned b;
+                    while ((b = __ballot_sync(kFull, fresh)) != 0u) {
+                        const unsigned gb = gr.mine(b);
+                        if (gb) {
+                            if (gr.l == __ffs(gb) - 1) {
+                                m.n[e][gr.g][nn[e]][0] = nv.x;
+                                m.n[e][gr.g][nn[e]][1] = nv.y;
+                                m.n[e][gr.g][nn[e]][2] = nv.z;
+                                m.id[e][gr.g][nn[e]] = j;
+                            }
+                            ++nn[e];
+                        }
+                        __syncwarp();
+                        if (fresh) {
+                            const R* w = m.n[e][gr.g][nn[e] - 1];
+                            fresh = nn[e] < kNumMRR && !(w[0] == nv.x && w[1] == nv.y && w[2] == nv.z);
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+        }
+        // corner mirror (kernel.cu:841-858): see plan_mirrors
+        const bool has = in && nn[0] > 0 && nn[1] >= 2;
+        if (has) {
+            cn = V4<R>{R(0), R(0), R(0), R(0)};
+            for (int k = 0; k < nn[1]; ++k) {
+                cn.x += m.n[1][gr.g][k][0];
+                cn.y += m.n[1][gr.g][k][1];
+                cn.z += m.n[1][gr.g][k][2];
+            }
+            const R as = sqrtR(dot3(cn.x, cn.y, cn.z, cn.x, cn.y, cn.z));
+            cn.x = cn.x / as; cn.y = cn.y / as; cn.z = cn.z / as;
+            corner = m.id[1][gr.g][nn[1] - 1];
+        }
+        const bool two = has && nn[1] == 2;
+        if (__any_sync(kFull, two)) {  // the nearest Edge wall of the last normal, first among equals
+            R best = R(INFINITY);
+            int bj = corner, bh = INT_MAX, seen = 0;
+            const R* ln = m.n[1][gr.g][1];
+            for (int w0 = 0; w0 < total; w0 += Mem::kWindow) {
+                if (total > Mem::kWindow) n = walls(w0);
+                for (int h = gr.l; two && h < n; h += G) {
+                    const int j = m.kidx[m.hit[gr.g][h]];
+                    if (__ldg(a.wl.wse + j) != kEDGE) continue;
+                    const V4<R> nv = ldg4(a.wl.nrm + j);
+                    if (nv.x != ln[0] || nv.y != ln[1] || nv.z != ln[2]) continue;
+                    const R d2 = pair_d2(ldg4(a.wl.pos + j), p);
+                    if (d2 < best) {
+                        best = d2;
+                        bj = j;
+                        bh = seen + h;
+                    }
+                }
+                seen += n;
+                __syncwarp();
+            }
+            for (int o = G / 2; o > 0; o >>= 1) {
+                const R ob = __shfl_xor_sync(kFull, best, o);
+                const int oj = __shfl_xor_sync(kFull, bj, o), oh = __shfl_xor_sync(kFull, bh, o);
+                if (ob < best || (ob == best && oh < bh)) {
+                    best = ob;
+                    bj = oj;
+                    bh = oh;
+                }
+            }
+            if (two) corner = bj;
+        }
+    }
+    if (DIAG && fld && gr.l == 0) a.diag[size_t(me.pid) * kDiagCols + DG_GEN_W] = nwall;
+    // item k < nn[0]: the face mirror of normal k; item nn[0]: the corner mirror
+    auto item = [&](int k, V4<R>& out, V4<R>& nv, R& nlen) {
+        const bool face = k < nn[0];
+        if (!face && corner < 0) return false;
+        const int w = face ? m.id[0][gr.g][k] : corner;
+        nv = face ? ldg4(a.wl.nrm + w) : cn;
+        return mirror_of(p.x, p.y, p.z, ldg4(a.wl.pos + w), nv, !face, out, nlen);
+    };
+    V4<R> out{R(0), R(0), R(0), P}, nv{R(0), R(0), R(0), R(0)};
+    R nlen = R(1);
+    int mine = 0;
+    if (act)
+        for (int k = gr.l; k <= nn[0]; k += G)
+            if (item(k, out, nv, nlen)) {
+                if (k < kNumMRR) ++mine;
+                else atomicAdd(&a.cnt->err_mirror_slot, 1);  // a corner mirror without a slot
+            }
+    int incl = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(kFull, incl, o);
+        if (gr.lane >= o) incl += v;
+    }
+    const int tot = __shfl_sync(kFull, incl, 31);
+    int at = 0;
+    if (gr.lane == 31 && tot > 0) at = atomicAdd(&a.cnt->mirror_raw, tot);
+    at = __shfl_sync(kFull, at, 31) + incl - mine;
+    if (mine > 0)
+        for (int k = gr.l; k <= nn[0] && k < kNumMRR; k += G)
+            if (item(k, out, nv, nlen)) {
+                if (at < a.out.cap) {
+                    a.out.pos[at] = out;
+                    a.out.slot[at] = me.pid * kNumMRR + k;
+                    if (TAPE) {
+                        const R cf = sqrtR(R(2) / nlen);
+                        a.out.nrm[at] = V4<R>{nv.x * cf, nv.y * cf, nv.z * cf, R(0)};
+                    }
+                } else {
+                    atomicAdd(&a.cnt->err_capacity, 1);
+                }
+                ++at;
+            }
 }
 
 // The warp's mirrors take consecutive places in the raw list, reserved with one atomic per
@@ -1724,54 +2425,22 @@ __global__ void __launch_bounds__(128) k_ph_gen(const __grid_constant__ PassArgs
     gen_reserve_emit<R, RN, false>(a, pl, m, p.x, p.y, p.z, P, pid * kNumMRR);
 }
 
-// Nearest wall inside r of a mirror over part of its 27 buckets' rows: row ri = 3 (dz + 1)
-// + (dy + 1) when ri % 4 == part (for_rows's rows and skipping). Keeps the first nearest
-// wall in visiting order: distance, row and wall slot (-1: none).
-template <class R, class RN>
-__device__ __forceinline__ void nearest_wall_part(const SceneDev<R, RN>& sc, const RowCtx<R>& c,
-                                                  R mx, R my, R mz, const WallView<R>& wl, R B,
-                                                  int part, R& wd, int& wrow, int& wj) {
-#pragma unroll 1
-    for (int ri = part; ri < 9; ri += 4) {
-        const int dz = ri / 3 - 1, dy = ri % 3 - 1;
-        const R ddz = dz < 0 ? c.dzl : (dz > 0 ? c.dzh : R(0));
-        const R ddy = dy < 0 ? c.dyl : (dy > 0 ? c.dyh : R(0));
-        const R dyz2 = ddy * ddy + ddz * ddz;
-        if (dyz2 > B) continue;
-        const int jl = (dyz2 + c.dxl * c.dxl <= B) ? c.ix - 1 : c.ix;
-        const int jh = (dyz2 + c.dxh * c.dxh <= B) ? c.ix + 1 : c.ix;
-        const int row = sc.cbase + (c.iz + dz) * sc.nbxy + (c.iy + dy) * sc.nbx;
-        const int lo = __ldg(wl.cs + row + jl), hi = __ldg(wl.cs + row + jh + 1);
-        for (int j = lo; j < hi; ++j) {
-            V4<R> q = ldg4(wl.pos + j);
-            R dx = mx - q.x, dy2 = my - q.y, dz2 = mz - q.z;
-            R d2 = dot3(dx, dy2, dz2, dx, dy2, dz2);
-            if (d2 <= sc.r_le) {  // dist <= r
-                R d = sqrtR(d2);
-                if (d < wd) {
-                    wd = d;
-                    wrow = ri;
-                    wj = j;
-                }
-            }
-        }
-    }
-}
-
 // d_MRRinout (kernel.cu:932-985) over the raw mirrors; a culled mirror's slot becomes
-// negative. Four lanes share a mirror, each walking a quarter of its rows; the group then
-// keeps the smallest distance, on ties the earlier row, which is the wall the sequential
+// negative. Sixteen lanes share a mirror: lane r < 9 finds bucket row r's range of walls
+// (for_rows's rows and skipping), and the lanes stride over each row. The group keeps the
+// smallest distance, on ties the earlier row, then the earlier wall: the wall the sequential
 // walk keeps (the first nearest one found).
+constexpr int kCullLanes = 16;
 template <class R, class RN>
 __global__ void k_ph_cull(const __grid_constant__ PassArgs<R, RN> a) {
     const int n = min(a.cnt->mirror_raw, a.out.cap);
-    const int part = threadIdx.x & 3;
-    const int groups = (gridDim.x * blockDim.x) >> 2;
+    const int part = threadIdx.x & (kCullLanes - 1), first = threadIdx.x & 31 & ~(kCullLanes - 1);
+    const int groups = (gridDim.x * blockDim.x) / kCullLanes;
     const int nround = (n + groups - 1) / groups * groups;  // every lane loops alike
-    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; t < nround; t += groups) {
+    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) / kCullLanes; t < nround; t += groups) {
         const int sl = t < n ? a.out.slot[t] : -1;
         R wd = R(0);
-        int wrow = 9, wj = -1;
+        int wrow = 9, wj = -1, lo = 0, hi = 0;
         V4<R> q{R(0), R(0), R(0), R(0)};
         const SceneDev<R, RN>* scp = a.sc;
         if (sl >= 0) {
@@ -1779,16 +2448,44 @@ __global__ void k_ph_cull(const __grid_constant__ PassArgs<R, RN> a) {
             q = a.out.pos[t];
             int ix, iy, iz;
             if (!cell_of(*scp, q.x, q.y, q.z, ix, iy, iz) && part == 0) atomicAdd(&a.cnt->err_cell, 1);
-            const RowCtx<R> c = row_ctx(*scp, q.x, q.y, q.z, ix, iy, iz);
             wd = scp->wall_dist0;
-            nearest_wall_part(*scp, c, q.x, q.y, q.z, a.wl, a.skip != 0 ? scp->skip_r : R(INFINITY),
-                              part, wd, wrow, wj);
+            if (part < 9) {
+                const RowCtx<R> c = row_ctx(*scp, q.x, q.y, q.z, ix, iy, iz);
+                const R B = a.skip != 0 ? scp->skip_r : R(INFINITY);
+                const int dz = part / 3 - 1, dy = part % 3 - 1;
+                const R ddz = dz < 0 ? c.dzl : (dz > 0 ? c.dzh : R(0));
+                const R ddy = dy < 0 ? c.dyl : (dy > 0 ? c.dyh : R(0));
+                const R dyz2 = ddy * ddy + ddz * ddz;
+                if (!(dyz2 > B)) {
+                    const int jl = (dyz2 + c.dxl * c.dxl <= B) ? c.ix - 1 : c.ix;
+                    const int jh = (dyz2 + c.dxh * c.dxh <= B) ? c.ix + 1 : c.ix;
+                    const int row = scp->cbase + (c.iz + dz) * scp->nbxy + (c.iy + dy) * scp->nbx;
+                    lo = __ldg(a.wl.cs + row + jl);
+                    hi = __ldg(a.wl.cs + row + jh + 1);
+                }
+            }
         }
-        for (int o = 1; o <= 2; o <<= 1) {
-            const R od = __shfl_xor_sync(0xffffffffu, wd, o);
-            const int orow = __shfl_xor_sync(0xffffffffu, wrow, o);
-            const int oj = __shfl_xor_sync(0xffffffffu, wj, o);
-            if (oj >= 0 && (wj < 0 || od < wd || (od == wd && orow < wrow))) {
+        for (int r = 0; r < 9; ++r) {
+            const int l = __shfl_sync(kFull, lo, first + r), h = __shfl_sync(kFull, hi, first + r);
+            for (int j = l + part; j < h; j += kCullLanes) {
+                const V4<R> w = ldg4(a.wl.pos + j);
+                const R dx = q.x - w.x, dy = q.y - w.y, dz = q.z - w.z;
+                const R d2 = dot3(dx, dy, dz, dx, dy, dz);
+                if (d2 <= scp->r_le) {  // dist <= r
+                    const R d = sqrtR(d2);
+                    if (d < wd) {
+                        wd = d;
+                        wrow = r;
+                        wj = j;
+                    }
+                }
+            }
+        }
+        for (int o = kCullLanes / 2; o > 0; o >>= 1) {
+            const R od = __shfl_xor_sync(kFull, wd, o);
+            const int orow = __shfl_xor_sync(kFull, wrow, o), oj = __shfl_xor_sync(kFull, wj, o);
+            const bool tie = od == wd && (orow < wrow || (orow == wrow && oj < wj));
+            if (oj >= 0 && (wj < 0 || od < wd || tie)) {
                 wd = od;
                 wrow = orow;
                 wj = oj;

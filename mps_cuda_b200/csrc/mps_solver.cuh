@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -187,6 +188,17 @@ static void derive_scene(const mps_params& p, int cbase, int fbase, int pbase, i
     s.pmax = RN(R(p.pmax));
     s.rho = RN(rho);
     s.rp_n = RN(rp);
+    s.inv_rp = R(1) / rp;
+    s.inv_rp_n = RN(1) / s.rp_n;
+    // Pairs closer than l0 / 1024 (or coincident) and pairs within the bucket index's rounding
+    // of the bucket width take the general forms: two particles two buckets apart are farther
+    // than the width less twice that rounding. The walk needs the roots and quotients of
+    // every other pair in range and the radii rp and rlim inside that distance.
+    const long long nmax = std::max({nbl[0], nbl[1], nbl[2]});
+    const double slack = 8.0 * double(nmax) * double(std::numeric_limits<R>::epsilon()) + 1e-6;
+    s.pair_lo = R((double(l0) / 1024) * (double(l0) / 1024));
+    s.pair_hi = R(double(r) * double(r) * (1.0 - slack) * (1.0 - slack));
+    s.pairs_ok = double(l0) >= 0x1p-20 && double(l0) <= 0x1p20 && nmax < 4096 ? 1 : 0;
 
     std::memset(&inf, 0, sizeof(inf));
     inf.nbx = s.nbx; inf.nby = s.nby; inf.nbz = s.nbz; inf.nbxyz = s.nbxy * s.nbz;
@@ -693,7 +705,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         io.typ = ar.template get<int8_t>(T);
         io.cell = ar.template get<int>(T);
         d_integ = ar.template get<double>(6 * size_t(nscene));
-        nb = ar.template get<int>(size_t(kListCap) * ((F + 31) / 32 * 32));  // list_at tiles
+        nb = ar.template get<int>(list_size(F, kListCap));
         near_wall = ar.template get<int8_t>(L());
         near_m1 = ar.template get<int8_t>(L());
         near_m2 = ar.template get<int8_t>(L());
@@ -802,6 +814,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         a.out = MirrorSink<R>{U.pos, U.slot, cap, nullptr};
         a.cnt = cnt; a.diag = diag; a.ndens = ndens;
         a.nb = nb; a.nbcnt = nbcnt; a.nbK = nbK;
+        a.lt = list_layout();
         a.near_wall = near_wall;
         a.near_m = mcs == mcs1 ? near_m1 : (mcs == mcs2 ? near_m2 : nullptr);
         a.tape_pre = nullptr;
@@ -810,12 +823,91 @@ template <class R, class RN> class Solver final : public SolverBase {
 
     void reset_raw() { CK(cudaMemsetAsync(&cnt->mirror_raw, 0, sizeof(int), stream)); }
 
-    // MRRinout over the raw mirrors, one thread per mirror (culled slots turn negative)
+    // MRRinout over the raw mirrors (culled slots turn negative)
     void cull_raw() {
-        k_ph_cull<R, RN><<<std::min(blocks(4 * cap, 256), 148 * 32), 256, 0, stream>>>(args(M1, mcs1));
+        const long long lanes = (long long)kCullLanes * cap;
+        const int grid = int(std::min<long long>((lanes + 255) / 256, 148 * 32));
+        k_ph_cull<R, RN><<<grid, 256, 0, stream>>>(args(M1, mcs1));
         KL();
     }
 
+    // Lanes per particle of a pass: a warp while the scene has few particles, 8 up to `most`,
+    // else 0, one thread per particle. A group's lanes shorten a particle's serial chain but
+    // repeat the set-up, and their warp tests the union of its particles' candidates, so the
+    // thread kernels win once they fill the GPU. Measured on dam breaks in FP32, us per launch
+    // (one thread / 8 lanes / a warp):
+    //              3.5k particles    16.8k             48k               93k               192k
+    //   pass A     127 / 35 / 26     145 / 60 / 70     142 / 119 / 175   148 / 208 / 320
+    //   pass B     112 / 31 / 23     126 / 41 / 62     136 / 87 / 144    133 / 140 / 250
+    //   pass C      97 / 19 / 15     104 / 27 / 31     101 / 47 / 66     103 / 75 / 111    120 / 131
+    //   two generations and culls
+    //              167 / 79 / 52     211 / 86 / 95     205 / 119 / 151   203 / 139 / 209   198 / 207
+    // and the FP64 crossings lie at the same sizes.
+    static constexpr int kWarpMost = 5000, kGroupMostA = 65536, kGroupMostBC = 98304,
+                         kGroupMostGen = 180000;
+    int group_lanes(int most) const { return nF <= kWarpMost ? 32 : (nF <= most ? 8 : 0); }
+    int list_layout() const { return group_lanes(kGroupMostBC) ? kListGroup : kListThread; }
+    int group_grid(int g) const { return blocks(nF, 128 / g); }
+
+    // pass A, with the mirror table that `a` names
+    template <bool D, bool TAPE> void run_pass_a(const PassArgs<R, RN>& a, int ba) {
+        const int g = group_lanes(kGroupMostA);
+        if (g == 32)
+            k_pass_a_g<R, RN, D, TAPE, 32><<<group_grid(32), 128, 0, stream>>>(a);
+        else if (g == 8)
+            k_pass_a_g<R, RN, D, TAPE, 8><<<group_grid(8), 128, 0, stream>>>(a);
+        else if (TAPE)
+            k_pass_a<R, RN, D, TAPE><<<blocks(nF, ba), ba, 0, stream>>>(a);
+        else if (reg_bound & 4)
+            launch_pass_a<D, true>(a, ba);
+        else
+            launch_pass_a<D, false>(a, ba);
+        KL();
+    }
+    template <bool D> void run_pass_b(const PassArgs<R, RN>& a, int bb) {
+        const int g = group_lanes(kGroupMostBC);
+        if (g == 32)
+            k_pass_b_g<R, RN, D, 32><<<group_grid(32), 128, 0, stream>>>(a);
+        else if (g == 8)
+            k_pass_b_g<R, RN, D, 8><<<group_grid(8), 128, 0, stream>>>(a);
+        else if (reg_bound & 1)
+            k_pass_b<R, RN, D, true><<<blocks(nF, bb), bb, 0, stream>>>(a);
+        else
+            k_pass_b<R, RN, D><<<blocks(nF, bb), bb, 0, stream>>>(a);
+        KL();
+    }
+    template <bool D, bool TAPE> void run_pass_c(const PassArgs<R, RN>& a, int bc) {
+        const int g = group_lanes(kGroupMostBC);
+        const bool corr = !TAPE && grad_mode == MPS_GRAD_CORRECTED;
+        if (g == 32 && corr)
+            k_pass_c_g<R, RN, D, false, true, 32><<<group_grid(32), 128, 0, stream>>>(a);
+        else if (g == 32)
+            k_pass_c_g<R, RN, D, TAPE, false, 32><<<group_grid(32), 128, 0, stream>>>(a);
+        else if (g == 8 && corr)
+            k_pass_c_g<R, RN, D, false, true, 8><<<group_grid(8), 128, 0, stream>>>(a);
+        else if (g == 8)
+            k_pass_c_g<R, RN, D, TAPE, false, 8><<<group_grid(8), 128, 0, stream>>>(a);
+        else if (corr)
+            k_pass_c<R, RN, D, false, true><<<blocks(nF, bc), bc, 0, stream>>>(a);
+        else if (!TAPE && (reg_bound & 2))
+            k_pass_c<R, RN, D, false, false, true><<<blocks(nF, bc), bc, 0, stream>>>(a);
+        else
+            k_pass_c<R, RN, D, TAPE><<<blocks(nF, bc), bc, 0, stream>>>(a);
+        KL();
+    }
+    // GenMRR_nonslip into the raw list, then the cull
+    template <bool D, bool TAPE>
+    void run_gen(const PassArgs<R, RN>& a, int bg, const V4<R>* pos, const R* prs, const int8_t* typ) {
+        const int g = group_lanes(kGroupMostGen);
+        if (g == 32)
+            k_gen_cull_g<R, RN, D, TAPE, 32><<<group_grid(32), 128, 0, stream>>>(a, pos, prs, typ);
+        else if (g == 8)
+            k_gen_cull_g<R, RN, D, TAPE, 8><<<group_grid(8), 128, 0, stream>>>(a, pos, prs, typ);
+        else
+            k_gen_cull<R, RN, D, TAPE><<<blocks(nF, bg), bg, 0, stream>>>(a, pos, prs, typ);
+        KL();
+        cull_raw();
+    }
 
     // wall bucket build from the load-order copy, then Surface_Edge (kernel.cu:553-668) and
     // the near-wall flags of every bucket
@@ -895,13 +987,13 @@ template <class R, class RN> class Solver final : public SolverBase {
     }
 
     // pass A walking global memory, at the handle's candidate batch
-    template <bool D, bool ALT> void launch_pass_a(int ba) {
+    template <bool D, bool ALT> void launch_pass_a(const PassArgs<R, RN>& a, int ba) {
         if (batch_a == 2)
-            k_pass_a<R, RN, D, false, 2, ALT><<<blocks(nF, ba), ba, 0, stream>>>(args(M1, mcs1));
+            k_pass_a<R, RN, D, false, 2, ALT><<<blocks(nF, ba), ba, 0, stream>>>(a);
         else if (batch_a == 8)
-            k_pass_a<R, RN, D, false, 8, ALT><<<blocks(nF, ba), ba, 0, stream>>>(args(M1, mcs1));
+            k_pass_a<R, RN, D, false, 8, ALT><<<blocks(nF, ba), ba, 0, stream>>>(a);
         else
-            k_pass_a<R, RN, D, false, 4, ALT><<<blocks(nF, ba), ba, 0, stream>>>(args(M1, mcs1));
+            k_pass_a<R, RN, D, false, 4, ALT><<<blocks(nF, ba), ba, 0, stream>>>(a);
     }
 
     template <bool D> void fused_body() {
@@ -910,13 +1002,12 @@ template <class R, class RN> class Solver final : public SolverBase {
         // pass A: VscTrm + UpPcl1
         {
             Scope t(this, MPS_K_PASS_A);
-            if (stage_mode != MPS_STAGE_GLOBAL)
+            if (stage_mode != MPS_STAGE_GLOBAL) {
                 launch_pass_a_staged<D>(ba);
-            else if (reg_bound & 4)
-                launch_pass_a<D, true>(ba);
-            else
-                launch_pass_a<D, false>(ba);
-            KL();
+                KL();
+            } else {
+                run_pass_a<D, false>(args(M1, mcs1), ba);
+            }
         }
         // MkBkt on x* (kernel.cu:1917); the rebuild at kernel.cu:1921 would give the same lists
         bin_fluid(t_pos, t_vel, nullptr, S.prs, S.pav, S.pid, t_typ);
@@ -934,10 +1025,7 @@ template <class R, class RN> class Solver final : public SolverBase {
             reset_raw();
             {
                 Scope t(this, MPS_K_GEN);
-                k_gen_cull<R, RN, D><<<blocks(nF, bg), bg, 0, stream>>>(args(M1, mcs1), S.pos,
-                                                                               nullptr, S.typ);
-                KL();
-                cull_raw();
+                run_gen<D, false>(args(M1, mcs1), bg, S.pos, nullptr, S.typ);
             }
             bin_mirrors(M2, mcs2);
             CK(cudaEventRecord(ev_join, side));
@@ -945,11 +1033,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         // pass B: ChkCol + MkPrs
         {
             Scope t(this, MPS_K_PASS_B);
-            if (reg_bound & 1)
-                k_pass_b<R, RN, D, true><<<blocks(nF, bb), bb, 0, stream>>>(args(M1, mcs1));
-            else
-                k_pass_b<R, RN, D><<<blocks(nF, bb), bb, 0, stream>>>(args(M1, mcs1));
-            KL();
+            run_pass_b<D>(args(M1, mcs1), bb);
         }
         if (fork) {
             CK(cudaStreamWaitEvent(stream, ev_join, 0));
@@ -960,24 +1044,14 @@ template <class R, class RN> class Solver final : public SolverBase {
             reset_raw();
             {
                 Scope t(this, MPS_K_GEN);
-                k_gen_cull<R, RN, D><<<blocks(nF, bg), bg, 0, stream>>>(args(M1, mcs1), S.pos,
-                                                                               t_prs, S.typ);
-                KL();
-                cull_raw();
+                run_gen<D, false>(args(M1, mcs1), bg, S.pos, t_prs, S.typ);
             }
             bin_mirrors(M2, mcs2);
         }
         // pass C: PrsGrdTrm + UpPcl2, then the first mirror generation of the next step
         {
             Scope t(this, MPS_K_PASS_C);
-            if (grad_mode == MPS_GRAD_CORRECTED)
-                k_pass_c<R, RN, D, false, true><<<blocks(nF, bc), bc, 0, stream>>>(args(M2, mcs2));
-            else if (reg_bound & 2)
-                k_pass_c<R, RN, D, false, false, true><<<blocks(nF, bc), bc, 0, stream>>>(
-                    args(M2, mcs2));
-            else
-                k_pass_c<R, RN, D><<<blocks(nF, bc), bc, 0, stream>>>(args(M2, mcs2));
-            KL();
+            run_pass_c<D, false>(args(M2, mcs2), bc);
         }
         // walls that move take their place at the new time before the next step's mirrors
         if (motion_on) move_walls();
@@ -1003,10 +1077,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         }
         {
             Scope t(this, MPS_K_GEN);
-            k_gen_cull<R, RN, false><<<blocks(nF, bg), bg, 0, stream>>>(args(M2, mcs2), t_pos,
-                                                                               t_prs, t_typ);
-            KL();
-            cull_raw();
+            run_gen<false, false>(args(M2, mcs2), bg, t_pos, t_prs, t_typ);
         }
         if (fork) {
             {
@@ -1037,10 +1108,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         }
         if (!m1_valid) {
             reset_raw();
-            k_gen_cull<R, RN, false><<<blocks(nF, block), block, 0, stream>>>(
-                args(M1, mcs1), S.pos, S.prs, S.typ);
-            KL();
-            cull_raw();
+            run_gen<false, false>(args(M1, mcs1), block, S.pos, S.prs, S.typ);
             bin_mirrors(M1, mcs1);
             m1_valid = true;
         }
@@ -1593,7 +1661,6 @@ template <class R, class RN> class Solver final : public SolverBase {
         st->nbK = nbK;
         DevArena& a = st->ar;
         const size_t F = std::max(nF, 1), T = std::max(nT, 1), Cm = size_t(cap), Lc = L() + 1;
-        const size_t F32 = (F + 31) / 32 * 32;  // slots rounded to whole warps (list_at)
         for (int c = 0; c <= nck; ++c)
             st->ck.push_back(Ckpt{a.template get<R>(3 * T), a.template get<R>(3 * T),
                                   a.template get<R>(T), a.template get<R>(T),
@@ -1602,13 +1669,13 @@ template <class R, class RN> class Solver final : public SolverBase {
             TapeStep<R> t;
             t.pid1 = a.template get<int>(F); t.x1 = a.template get<V4<R>>(F);
             t.v1 = a.template get<V4<R>>(F); t.up1 = a.template get<V4<R>>(F);
-            t.nA = a.template get<int>(F); t.nbA = a.template get<int>(size_t(nbK) * F32);
+            t.nA = a.template get<int>(F); t.nbA = a.template get<int>(list_size(F, nbK));
             t.m1pos = a.template get<V4<R>>(Cm); t.m1slot = a.template get<int>(Cm);
             t.m1nrm = a.template get<V4<R>>(Cm); t.mcs1 = a.template get<int>(Lc);
             t.pid2 = a.template get<int>(F); t.x2 = a.template get<V4<R>>(F);
             t.u2 = a.template get<V4<R>>(F); t.vv2 = a.template get<V4<R>>(F);
             t.P2 = a.template get<R>(F); t.vp2 = a.template get<V4<R>>(F);
-            t.nB = a.template get<int>(F); t.nbB = a.template get<int>(size_t(nbK) * F32);
+            t.nB = a.template get<int>(F); t.nbB = a.template get<int>(list_size(F, nbK));
             t.m2pos = a.template get<V4<R>>(Cm); t.m2slot = a.template get<int>(Cm);
             t.m2nrm = a.template get<V4<R>>(Cm); t.mcs2 = a.template get<int>(Lc);
             st->tape.push_back(t);
@@ -1680,10 +1747,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         mkbkt(false);
         reset_raw();
         PassArgs<R, RN> a = tape_args(M1.pos, M1.slot, mcs1, nb, nbcnt, nullptr);
-        k_gen_cull<R, RN, false, true><<<blocks(nF, block), block, 0, stream>>>(
-            a, S.pos, S.prs, S.typ);
-        KL();
-        cull_raw();
+        run_gen<false, true>(a, block, S.pos, S.prs, S.typ);
         bin_mirrors_n(t.m1pos, t.m1slot, t.m1nrm, t.mcs1);
     }
 
@@ -1699,8 +1763,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         cp(t.x1, S.pos, sizeof(V4<R>) * F);
         cp(t.v1, S.vel, sizeof(V4<R>) * F);
         PassArgs<R, RN> a = tape_args(t.m1pos, t.m1slot, t.mcs1, t.nbA, t.nA, t.up1);
-        k_pass_a<R, RN, false, true><<<blocks(nF, ba), ba, 0, stream>>>(a);
-        KL();
+        run_pass_a<false, true>(a, ba);
         bin_fluid(t_pos, t_vel, nullptr, S.prs, S.pav, S.pid, t_typ);
         a = tape_args(t.m1pos, t.m1slot, t.mcs1, t.nbB, t.nB, nullptr);
         // the second mirror generation beside pass B, as in fused_body (overlap bit 1); the
@@ -1711,15 +1774,11 @@ template <class R, class RN> class Solver final : public SolverBase {
             CK(cudaStreamWaitEvent(side, ev_fork, 0));
             OnStream o(this, side);
             reset_raw();
-            k_gen_cull<R, RN, false, true><<<blocks(nF, bg), bg, 0, stream>>>(a, S.pos, nullptr,
-                                                                                    S.typ);
-            KL();
-            cull_raw();
+            run_gen<false, true>(a, bg, S.pos, nullptr, S.typ);
             bin_mirrors_n(t.m2pos, t.m2slot, t.m2nrm, t.mcs2);
             CK(cudaEventRecord(ev_join, side));
         }
-        k_pass_b<R, RN, false><<<blocks(nF, bb), bb, 0, stream>>>(a);
-        KL();
+        run_pass_b<false>(a, bb);
         cp(t.pid2, S.pid, sizeof(int) * F);
         cp(t.x2, S.pos, sizeof(V4<R>) * F);
         cp(t.u2, S.vel, sizeof(V4<R>) * F);
@@ -1732,20 +1791,13 @@ template <class R, class RN> class Solver final : public SolverBase {
             KL();
         } else {
             reset_raw();
-            k_gen_cull<R, RN, false, true><<<blocks(nF, bg), bg, 0, stream>>>(a, S.pos, t_prs,
-                                                                                    S.typ);
-            KL();
-            cull_raw();
+            run_gen<false, true>(a, bg, S.pos, t_prs, S.typ);
             bin_mirrors_n(t.m2pos, t.m2slot, t.m2nrm, t.mcs2);
         }
         a = tape_args(t.m2pos, t.m2slot, t.mcs2, t.nbB, t.nB, t.vp2);
-        k_pass_c<R, RN, false, true><<<blocks(nF, bc), bc, 0, stream>>>(a);
-        KL();
+        run_pass_c<false, true>(a, bc);
         reset_raw();
-        k_gen_cull<R, RN, false, true><<<blocks(nF, bg), bg, 0, stream>>>(a, t_pos, t_prs,
-                                                                                t_typ);
-        KL();
-        cull_raw();
+        run_gen<false, true>(a, bg, t_pos, t_prs, t_typ);
         bin_fluid(t_pos, t_vel, nullptr, t_prs, S.pav, S.pid, t_typ);
         if (next) bin_mirrors_n(next->m1pos, next->m1slot, next->m1nrm, next->mcs1);
         else bin_mirrors(M1, mcs1);
@@ -1754,7 +1806,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     void back_step(const TapeStep<R>& t) {
         AdjState& s = *adj;
         AdjArgs<R, RN> A;
-        A.sc = d_sc; A.nF = nF; A.nbK = nbK; A.t = t; A.wl = wall_view();
+        A.sc = d_sc; A.nF = nF; A.nbK = nbK; A.lt = list_layout(); A.t = t; A.wl = wall_view();
         A.lx = s.lx; A.lv = s.lv; A.lx_acc = s.lx_acc;
         A.lG = s.lG; A.lvv = s.lvv; A.lxs = s.lxs; A.lx_at = s.lx_at;
         A.lP = s.lP; A.lP_at = s.lP_at; A.pmin = s.pmin; A.am = s.am; A.inv2 = s.inv2;

@@ -37,7 +37,9 @@ template <class R, class RN> struct SceneDev {
     // fluid lists use fine cells, a third of a bucket per axis and nested in the buckets,
     // numbered fbase + 27 * bucket + 9 sz + 3 sy + sx (sub-cell s = int(3 t) + 3 - 3 i,
     // t as for the bucket index i)
-    int fbase, pad1, pad2;
+    int fbase;
+    int pairs_ok;     // mps_exact.cuh and the bounds pair_lo, pair_hi hold (derive_scene)
+    int pad2;
     float hf, ihf;    // fine cell width (bucket width / 3) and its inverse
     R r, r2, r_le;    // Laplacian radius; r_le = largest t with sqrt(t) <= r
     R rp, rp2, rp_lt; // gradient radius; rp_lt = largest t with sqrt(t) < rp
@@ -56,6 +58,11 @@ template <class R, class RN> struct SceneDev {
     R skip_r, skip_rp, skip_rl, skip_rw, skip_rc;
     RN n0g, prs_coef, pmax, rho;          // number density / EOS in RN (kernel.cu:1388-1406)
     RN rp_n;
+    // squared distances of pairs whose roots and quotients stay in the range of mps_exact.cuh
+    // and that cannot lie two buckets apart; the rest take the general forms
+    R pair_lo, pair_hi;
+    R inv_rp;         // 1 / rp
+    RN inv_rp_n;
 };
 
 // Prescribed rigid motion of one moving-wall type (OBJ or OBJ2), in double: a wall particle
@@ -84,7 +91,8 @@ struct DevCounters {
     int scan_ticket;      // blocks of the running fine-cell scan that finished (0 between)
     int stage_blocks;     // blocks of a staged pass that walked shared memory (diagnostics)
     int unstaged_blocks;  // ... and those whose neighbourhood did not fit (diagnostics)
-    int pad[5];
+    int off_grid;         // a bucket build met a listed particle outside the grid (sticky)
+    int pad[4];
     // diagnostics: fluid candidates tested by VscTrm's walk and by the list build of
     // ChkCol/MkPrs, and the entries of those lists
     unsigned long long work[3];

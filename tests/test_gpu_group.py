@@ -1,0 +1,111 @@
+"""The neighbour passes with several lanes per particle (mps_group.cuh) against the CPU oracle.
+
+Small scenes run the passes with a warp or eight lanes per particle, larger ones with one thread
+(Solver::group_lanes); every path must give the oracle's state bit for bit. The blocks have odd
+sides, so that a warp's particles span bucket rows and the last warp is ragged; the sizes lie on
+both sides of the line between a warp and eight lanes, and on the line of one thread.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from mps_cuda_b200 import F32, F32_N64, F64, MPS, SceneDesc, dambreak, dambreak_params
+from mps_cuda_b200 import _lib as L
+from oracle.oracle import Oracle, params_from
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("typ", "pos", "vel", "prs", "pav")
+
+
+def _pair(block, tank, prec, l0=0.02, dt=2e-4, **desc):
+    d = SceneDesc(l0, tuple(t * l0 for t in tank), block, seed=5, vel_sigma=0.3, **desc)
+    sc = dambreak(d)
+    p = dambreak_params(d, dt=dt, precision=prec)
+    real = np.float64 if prec == F64 else np.float32
+    args = [sc["typ"], *(sc[k].astype(real) for k in ("pos", "vel", "nrm"))]
+    return MPS(p, *args), Oracle(params_from(p), *args)
+
+
+def _steps(g, o, n, where):
+    g.step(n)
+    o.step(n)
+    a, b = g.state(), o.state()
+    for k in FIELDS:
+        assert np.array_equal(a[k], b[k]), (where, k)
+
+
+@pytest.mark.parametrize("prec", [F32, F64, F32_N64])
+@pytest.mark.parametrize("block,tank", [
+    ((1, 1, 2), (5, 4, 6)),       # two particles, a nearly empty warp
+    ((3, 7, 11), (9, 7, 13)),     # 231
+    ((17, 13, 19), (30, 14, 21)),  # 4199: a warp each
+    ((25, 8, 25), (31, 9, 27)),   # 5000: the last size of a warp each
+    ((23, 17, 13), (40, 17, 15)),  # 5083: eight lanes each
+])
+def test_odd_scenes_equal_the_oracle(block, tank, prec):
+    g, o = _pair(block, tank, prec)
+    try:
+        _steps(g, o, 1, "first")
+        _steps(g, o, 6, "later")
+        a, b = g.mirrors(2), o.mirrors()
+        assert np.array_equal(a["slot"], b["slot"]) and np.array_equal(a["pos"], b["pos"])
+    finally:
+        g.close()
+        o.close()
+
+
+@pytest.mark.parametrize("opts", [
+    {L.OPT_DIAG: 1}, {L.OPT_LIST_CAPACITY: 9}, {L.OPT_GRADIENT: L.GRAD_CORRECTED}, {L.OPT_CELL_SKIP: 0},
+])
+@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13)])
+def test_options_equal_the_oracle(block, opts):
+    tank = tuple(b + 3 for b in block)
+    g, o = _pair(block, tank, F32)
+    try:
+        for k, v in opts.items():
+            g.set_option(k, v)
+        if L.OPT_GRADIENT in opts:
+            o.set_gradient(1)
+        _steps(g, o, 3, opts)
+        if L.OPT_DIAG in opts:
+            a, b, fl = g.diag(), o.diag(), o.state()["typ"] == L.FLD
+            for k in L.DIAG_COLUMNS:
+                assert np.array_equal(a[k][fl], b[k][fl]), k
+    finally:
+        g.close()
+        o.close()
+
+
+@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13)])
+def test_scales_outside_the_fast_arithmetic_equal_the_oracle(block):
+    """A spacing below 2^-20 takes the walk of one lane per particle inside the same kernels."""
+    tank = tuple(b + 3 for b in block)
+    g, o = _pair(block, tank, F32, l0=2e-7, dt=1e-10)
+    try:
+        _steps(g, o, 3, block)
+    finally:
+        g.close()
+        o.close()
+
+
+@pytest.mark.parametrize("shift", [0.0, 1e-6])
+def test_nearly_coincident_particles_equal_the_oracle(shift):
+    """Pairs closer than l0 / 1024 leave the fast arithmetic; coincident ones give infinities."""
+    g, o = _pair((9, 8, 11), (14, 8, 14), F32)
+    try:
+        st = o.state()
+        pos = st["pos"].copy()
+        for i, j in ((100, 101), (400, 470)):
+            pos[:, j] = pos[:, i] + np.float32(shift)
+        g.set_state(pos=pos)
+        o.set_state(pos=pos)
+        g.step(1)
+        o.step(1)
+        a, b = g.state(), o.state()
+        for k in FIELDS:
+            assert np.array_equal(a[k], b[k], equal_nan=k != "typ"), k
+    finally:
+        g.close()
+        o.close()
