@@ -737,6 +737,7 @@ template <class R, class RN> struct PassArgs {
     V4<R>* pos; V4<R>* vel; V4<R>* acc; R* prs; R* pav; const int* pid; int8_t* typ;
     // scratch in the same slot order
     V4<R>* tpos; V4<R>* tvel; R* tprs; int8_t* ttyp;
+    V4<R>* posp;  // pass B's positions with the pressure in w, for pass C's neighbours
     WallView<R> wl;
     MirrorView<R> m;
     MirrorSink<R> out;
@@ -1005,6 +1006,37 @@ __device__ __forceinline__ void staged_range(const StageHdr& h, int fz, int fy, 
     hi = t[xh + 1];
 }
 
+template <class R> __device__ __forceinline__ R pair_d2(const V4<R>& q, const V4<R>& p) {
+    const R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+    return dot3(dx, dy, dz, dx, dy, dz);
+}
+
+// Pair terms by mps_exact.cuh for d2 >= lo (SceneDev::pair_lo, infinite for a scene whose sizes are
+// out of its range), else by the general operations:
+// VscTrm's weight 2 l0 / (d^2 d) (kernel.cu:1062-1064), WEI_grad(d, re) (const.cuh:46)
+template <class R> __device__ __forceinline__ R visc_weight(R two_l0, R d2, R lo) {
+    if (d2 >= lo) return div_in(two_l0, d2 * sqrt_in(d2));
+    return two_l0 / (d2 * sqrtR(d2));
+}
+template <class R> __device__ __forceinline__ R wei_in(R d, R re, R inv_re) {
+    return div_in(re, d) - div_by(d, re, inv_re);
+}
+// MkPrs's term (kernel.cu:1346-1348)
+template <class R, class RN>
+__device__ __forceinline__ RN dens_term(const SceneDev<R, RN>& sc, R d2) {
+    RN t = RN(0);
+    if (!(d2 >= sc.pair_lo)) dens_add(sc, d2, t);
+    else if (sizeof(RN) == sizeof(R)) t = RN(wei_in(sqrt_in(d2), sc.rp, sc.inv_rp));
+    else t = wei_in(sqrt_in(RN(d2)), sc.rp_n, sc.inv_rp_n);
+    return t;
+}
+// PrsGrdTrm's weight WEI_grad(d, rp) / d^2 (kernel.cu:1731-1735)
+template <class R, class RN>
+__device__ __forceinline__ R grad_weight(const SceneDev<R, RN>& sc, R d2) {
+    if (d2 >= sc.pair_lo) return div_in(wei_in(sqrt_in(d2), sc.rp, sc.inv_rp), d2);
+    return wei_grad(sqrtR(d2), sc.rp) / d2;
+}
+
 // state of a slot in a recorded step, kept in the w component of the pre-clamp velocity
 constexpr int kTapeOk = 0, kTapeClamped = 1, kTapeDeleted = 2, kTapeDead = 3;
 
@@ -1032,7 +1064,7 @@ __device__ __forceinline__ void visc_walk(const PassArgs<R, RN>& a, const SceneD
                                           const V4<R>& p, const V4<R>& v, R& sx, R& sy, R& sz,
                                           int& cf, int& ncand, Ranges&& ranges, Cand&& cand,
                                           Velo&& velo) {
-    const R two_l0 = sc.two_l0, r_le = sc.r_le;
+    const R two_l0 = sc.two_l0, r_le = sc.r_le, pair_lo = sc.pair_lo;
     int* __restrict__ nb = a.nb;
     const int nF = a.nF, K = a.nbK;
     auto near = [&](const V4<R>& q, int j, R& d2) {
@@ -1041,8 +1073,7 @@ __device__ __forceinline__ void visc_walk(const PassArgs<R, RN>& a, const SceneD
         return j != s && d2 <= r_le;  // dist <= r
     };
     auto add = [&](R d2, const V4<R>& u, int j) {
-        R d = sqrtR(d2);
-        R w = two_l0 / (d2 * d);
+        const R w = visc_weight(two_l0, d2, pair_lo);
         sx = fmaR(u.x - v.x, w, sx);
         sy = fmaR(u.y - v.y, w, sy);
         sz = fmaR(u.z - v.z, w, sz);
@@ -1227,10 +1258,12 @@ __global__ void __launch_bounds__(128) k_pass_a_st(const __grid_constant__ PassA
 // pass B's stores: velocity after ChkCol, pressure from MkPrs's EOS, diagnostics
 template <class R, class RN, bool DIAG>
 __device__ __forceinline__ void pass_b_store(const PassArgs<R, RN>& a, const SceneDev<R, RN>& sc,
-                                             int s, int pid, R wx, R wy, R wz, RN ni,
-                                             const int* cnt5) {
+                                             int s, int pid, const V4<R>& p, R wx, R wy, R wz,
+                                             RN ni, const int* cnt5) {
+    const R P = eos(sc, ni);
     a.tvel[s] = V4<R>{wx, wy, wz, R(0)};
-    a.tprs[s] = eos(sc, ni);
+    a.tprs[s] = P;
+    a.posp[s] = V4<R>{p.x, p.y, p.z, P};
     if (DIAG) {
         int32_t* d = a.diag + size_t(pid) * kDiagCols;
         d[DG_COL_F] = cnt5[0];
@@ -1259,7 +1292,7 @@ __device__ __noinline__ void pass_b_long(const PassArgs<R, RN>& a, int s) {
     int cnt5[5] = {0, 0, 0, 0, 0};
     col_dens_sum<R, RN, true, true>(sc, c, s, p.x, p.y, p.z, v.x, v.y, v.z, a.csr, a.posf, a.vel,
                                     a.wl, a.m, a.skip != 0, wx, wy, wz, ni, cnt5);
-    pass_b_store<R, RN, DIAG>(a, sc, s, pid, wx, wy, wz, ni, cnt5);
+    pass_b_store<R, RN, DIAG>(a, sc, s, pid, p, wx, wy, wz, ni, cnt5);
 }
 
 // Pass B for one slot with one thread; LT: the lists' layout (list_at)
@@ -1290,8 +1323,7 @@ __device__ __forceinline__ void pass_b_walk(const PassArgs<R, RN>& a, int s) {
     const V4<R>* __restrict__ pos = a.pos;
     const V4<R>* __restrict__ vel = a.vel;
     auto at = [](int k) { return (k >> (5 - LT)) * 32 + (k & ((32 >> LT) - 1)); };
-    const R rlim2 = sc.rlim2, rp_lt = sc.rp_lt, colfac = sc.colfac, rp = sc.rp;
-    const RN rp_n = sc.rp_n;
+    const R rlim2 = sc.rlim2, rp_lt = sc.rp_lt, colfac = sc.colfac;
     auto add = [&](int j, const V4<R>& q) {
         R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
         R d2 = dot3(dx, dy, dz, dx, dy, dz);
@@ -1301,7 +1333,7 @@ __device__ __forceinline__ void pass_b_walk(const PassArgs<R, RN>& a, int s) {
             ++cnt5[0];
         }
         if (d2 <= rp_lt) {
-            dens_add_v(rp, rp_n, d2, ni);
+            ni += dens_term(sc, d2);
             ++cnt5[3];
         }
     };
@@ -1323,7 +1355,7 @@ __device__ __forceinline__ void pass_b_walk(const PassArgs<R, RN>& a, int s) {
                                               a.skip != 0, wx, wy, wz, ni, cnt5,
                                               near_flag(a.near_wall, sc, c),
                                               near_flag(a.near_m, sc, c));
-    pass_b_store<R, RN, DIAG>(a, sc, s, pid, wx, wy, wz, ni, cnt5);
+    pass_b_store<R, RN, DIAG>(a, sc, s, pid, p, wx, wy, wz, ni, cnt5);
 }
 
 // pass B: ChkCol (kernel.cu:1168-1287) + MkPrs (kernel.cu:1306-1411) at x*; leaves the
@@ -1425,58 +1457,52 @@ __global__ void __launch_bounds__(128, pass_c_blocks<R>(ALT, CORR))
     G g;
     int cf = 0, cm = 0;
     const int* __restrict__ nb = a.nb + list_at(s, 0, a.nbK, kListThread);
-    const V4<R>* __restrict__ pos = a.pos;
+    const V4<R>* __restrict__ posp = a.posp;
     const R* __restrict__ prs = a.tprs;
     const int st = 32;
-    const R rp2 = sc.rp2, rp = sc.rp;
-    // P_min over the fluid neighbours inside rp (order-free), then the gradient in order
+    const R rp2 = sc.rp2;
+    // P_min over the fluid neighbours inside rp (order-free), then the gradient in order. The
+    // lists hold no entry beyond rp unless rlim exceeds it, so the first walk reads pressures
+    // alone; the second reads each entry's position and pressure in one load.
     R pmin = pi;
-    // each list entry's position and pressure are loaded together (both depend only on
-    // the index), four entries in flight, before the tests that use them
-    auto mn = [&](const V4<R>& q, R pj) {
-        R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
-        if (dot3(dx, dy, dz, dx, dy, dz) < rp2 && pj < pmin) pmin = pj;
+    const bool inside = sc.list_thr < rp2;
+    auto mn = [&](int j) {
+        const R pj = __ldg(prs + j);
+        return inside || pair_d2(ldg4(posp + j), p) < rp2 ? pj : pi;
     };
     int k = 0;
     for (; k + 4 <= n; k += 4) {
         const int j0 = nb[k * st], j1 = nb[(k + 1) * st], j2 = nb[(k + 2) * st],
                   j3 = nb[(k + 3) * st];
-        V4<R> q0 = ldg4(pos + j0), q1 = ldg4(pos + j1), q2 = ldg4(pos + j2), q3 = ldg4(pos + j3);
-        const R r0 = __ldg(prs + j0), r1 = __ldg(prs + j1), r2 = __ldg(prs + j2),
-                r3 = __ldg(prs + j3);
-        mn(q0, r0);
-        mn(q1, r1);
-        mn(q2, r2);
-        mn(q3, r3);
+        const R r0 = mn(j0), r1 = mn(j1), r2 = mn(j2), r3 = mn(j3);
+        if (r0 < pmin) pmin = r0;
+        if (r1 < pmin) pmin = r1;
+        if (r2 < pmin) pmin = r2;
+        if (r3 < pmin) pmin = r3;
     }
     for (; k < n; ++k) {
-        const int j = nb[k * st];
-        mn(ldg4(pos + j), __ldg(prs + j));
+        const R r = mn(nb[k * st]);
+        if (r < pmin) pmin = r;
     }
-    auto gr = [&](const V4<R>& q, R pj) {
+    auto gr = [&](const V4<R>& q) {
         R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
         R d2 = dot3(dx, dy, dz, dx, dy, dz);
         if (d2 < rp2) {
-            R d = sqrtR(d2);
-            g.add(wei_grad(d, rp) / d2, pj - pmin, dx, dy, dz);
+            g.add(grad_weight(sc, d2), q.w - pmin, dx, dy, dz);
             ++cf;
         }
     };
     for (k = 0; k + 4 <= n; k += 4) {
         const int j0 = nb[k * st], j1 = nb[(k + 1) * st], j2 = nb[(k + 2) * st],
                   j3 = nb[(k + 3) * st];
-        V4<R> q0 = ldg4(pos + j0), q1 = ldg4(pos + j1), q2 = ldg4(pos + j2), q3 = ldg4(pos + j3);
-        const R r0 = __ldg(prs + j0), r1 = __ldg(prs + j1), r2 = __ldg(prs + j2),
-                r3 = __ldg(prs + j3);
-        gr(q0, r0);
-        gr(q1, r1);
-        gr(q2, r2);
-        gr(q3, r3);
+        const V4<R> q0 = ldg4(posp + j0), q1 = ldg4(posp + j1), q2 = ldg4(posp + j2),
+                    q3 = ldg4(posp + j3);
+        gr(q0);
+        gr(q1);
+        gr(q2);
+        gr(q3);
     }
-    for (; k < n; ++k) {
-        const int j = nb[k * st];
-        gr(ldg4(pos + j), __ldg(prs + j));
-    }
+    for (; k < n; ++k) gr(ldg4(posp + nb[k * st]));
     if (near_flag(a.near_m, sc, c))
         grad_sum_mirrors(sc, c, pid - sc.pbase, p.x, p.y, p.z, pmin, a.m, a.skip != 0, g, cm);
     pass_c_finish<R, RN, DIAG, TAPE>(a, sc, s, pid, p, pi, g, cf, cm);
@@ -1485,31 +1511,6 @@ __global__ void __launch_bounds__(128, pass_c_blocks<R>(ALT, CORR))
 // ---------------------------------------------------------------------------------------
 // neighbour passes with a group of G lanes per particle (mps_group.cuh): small scenes
 // ---------------------------------------------------------------------------------------
-// Pair terms inside the common range by mps_exact.cuh (d2 >= lo), else by the general operations:
-// VscTrm's weight 2 l0 / (d^2 d) (kernel.cu:1062-1064), WEI_grad(d, re) (const.cuh:46)
-template <class R> __device__ __forceinline__ R visc_weight(R two_l0, R d2, R lo) {
-    if (d2 >= lo) return div_in(two_l0, d2 * sqrt_in(d2));
-    return two_l0 / (d2 * sqrtR(d2));
-}
-template <class R> __device__ __forceinline__ R wei_in(R d, R re, R inv_re) {
-    return div_in(re, d) - div_by(d, re, inv_re);
-}
-// MkPrs's term (kernel.cu:1346-1348)
-template <class R, class RN>
-__device__ __forceinline__ RN dens_term(const SceneDev<R, RN>& sc, R d2) {
-    RN t = RN(0);
-    if (!(d2 >= sc.pair_lo)) dens_add(sc, d2, t);
-    else if (sizeof(RN) == sizeof(R)) t = RN(wei_in(sqrt_in(d2), sc.rp, sc.inv_rp));
-    else t = wei_in(sqrt_in(RN(d2)), sc.rp_n, sc.inv_rp_n);
-    return t;
-}
-// PrsGrdTrm's weight WEI_grad(d, rp) / d^2 (kernel.cu:1731-1735)
-template <class R, class RN>
-__device__ __forceinline__ R grad_weight(const SceneDev<R, RN>& sc, R d2) {
-    if (d2 >= sc.pair_lo) return div_in(wei_in(sqrt_in(d2), sc.rp, sc.inv_rp), d2);
-    return wei_grad(sqrtR(d2), sc.rp) / d2;
-}
-
 // What a lane knows of its group's particle
 template <class R, class RN> struct GroupSlot {
     const SceneDev<R, RN>* sc;
@@ -1550,10 +1551,6 @@ __device__ __forceinline__ const SceneDev<R, RN>& group_scene(const PassArgs<R, 
                                                               const SceneDev<R, RN>* mine,
                                                               const GroupSet& t) {
     return a.sc[__shfl_sync(kFull, int(mine - a.sc), __ffs(t.lanes) - 1)];
-}
-template <class R> __device__ __forceinline__ R pair_d2(const V4<R>& q, const V4<R>& p) {
-    const R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
-    return dot3(dx, dy, dz, dx, dy, dz);
 }
 
 template <class R, class RN, bool DIAG, bool TAPE>
@@ -1807,7 +1804,7 @@ __global__ void __launch_bounds__(128) k_pass_b_g(const __grid_constant__ PassAr
     }
     if (act && gr.l == 0) {
         a.nbcnt[s] = have;
-        pass_b_store<R, RN, DIAG>(a, sc, s, me.pid, wx, wy, wz, ni, cnt5);
+        pass_b_store<R, RN, DIAG>(a, sc, s, me.pid, p, wx, wy, wz, ni, cnt5);
     }
 }
 
@@ -1893,12 +1890,13 @@ __global__ void __launch_bounds__(128) k_pass_c_g(const __grid_constant__ PassAr
     const int* __restrict__ nb = a.nb + list_at(s, 0, a.nbK, kListGroup);
     auto entry = [&](int h) { return __ldg(nb + 4 * (h & ~7) + (h & 7)); };
     const R rp2 = sc.rp2;
+    const bool inside = sc.list_thr < rp2;
     // P_min over the fluid neighbours inside rp (order-free), then the gradient in order
     R pmin = pi;
     for (int h = gr.l; h < cnt; h += G) {
         const int j = entry(h);
         const R pj = __ldg(a.tprs + j);
-        if (pair_d2(ldg4(a.pos + j), p) < rp2 && pj < pmin) pmin = pj;
+        if ((inside || pair_d2(ldg4(a.posp + j), p) < rp2) && pj < pmin) pmin = pj;
     }
     for (int o = G / 2; o > 0; o >>= 1) {
         const R x = __shfl_xor_sync(kFull, pmin, o);
@@ -1908,15 +1906,13 @@ __global__ void __launch_bounds__(128) k_pass_c_g(const __grid_constant__ PassAr
     int cf = 0, cm = 0;
     sums.add(m, gr, most, [&](int h, R(&d)[3], R& w, R& pd) {
         if (h >= cnt) return;
-        const int j = entry(h);
-        const V4<R> q = ldg4(a.pos + j);
-        const R pj = __ldg(a.tprs + j);
+        const V4<R> q = ldg4(a.posp + entry(h));
         const R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
         const R d2 = dot3(dx, dy, dz, dx, dy, dz);
         if (d2 < rp2) {
             d[0] = dx; d[1] = dy; d[2] = dz;
             w = grad_weight(sc, d2);
-            pd = pj - pmin;
+            pd = q.w - pmin;
             if (DIAG) ++cf;
         }
     });

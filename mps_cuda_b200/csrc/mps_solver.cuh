@@ -199,6 +199,7 @@ static void derive_scene(const mps_params& p, int cbase, int fbase, int pbase, i
     s.pair_lo = R((double(l0) / 1024) * (double(l0) / 1024));
     s.pair_hi = R(double(r) * double(r) * (1.0 - slack) * (1.0 - slack));
     s.pairs_ok = double(l0) >= 0x1p-20 && double(l0) <= 0x1p20 && nmax < 4096 ? 1 : 0;
+    if (!s.pairs_ok) s.pair_lo = R(INFINITY);
 
     std::memset(&inf, 0, sizeof(inf));
     inf.nbx = s.nbx; inf.nby = s.nby; inf.nbz = s.nbz; inf.nbxyz = s.nbxy * s.nbz;
@@ -358,6 +359,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     int* d_nbxyz = nullptr;
     FluidBuf<R> S, S2;
     V4<R>* t_pos; V4<R>* t_vel; R* t_prs; int8_t* t_typ;
+    V4<R>* posp;
     // walls, sorted once
     V4<R>* w_pos; V4<R>* w_nrm; V4<R>* w_vel; int* w_id; int8_t* w_typ; int8_t* w_se;
     int* wcs;
@@ -648,6 +650,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         t_pos = ar.template get<V4<R>>(F);
         t_vel = ar.template get<V4<R>>(F);
         t_prs = ar.template get<R>(F);
+        posp = ar.template get<V4<R>>(F);
         t_typ = ar.template get<int8_t>(F);
         w_pos = ar.template get<V4<R>>(W);
         w_nrm = ar.template get<V4<R>>(W);
@@ -809,6 +812,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         a.pos = S.pos; a.vel = S.vel; a.acc = S.acc; a.prs = S.prs; a.pav = S.pav; a.pid = S.pid;
         a.typ = S.typ;
         a.tpos = t_pos; a.tvel = t_vel; a.tprs = t_prs; a.ttyp = t_typ;
+        a.posp = posp;
         a.wl = wall_view();
         a.m = MirrorView<R>{mcs, m.pos, m.slot};
         a.out = MirrorSink<R>{U.pos, U.slot, cap, nullptr};
