@@ -212,18 +212,55 @@ static void derive_scene(const mps_params& p, int cbase, int fbase, int pbase, i
 }
 
 // ---- device allocation ---------------------------------------------------------------------
+// Device memory of a handle or of a recorded rollout. A set-up that takes many arrays runs its
+// gets twice, inside plan(): once to add up their sizes, then out of one allocation. The tape of
+// 20 recorded steps of 48 000 particles in FP64 is some 370 arrays of 2.8 GB: one by one 106 ms to
+// allocate and 100 ms to free, at once under 1 and 3 ms; a handle of 48 000 particles in FP32 takes
+// 8.2 and 6.4 ms to create and destroy with one allocation an array, 1.1 and 0.5 at once. Small
+// sets stay apart: the driver serves small requests from blocks that it keeps (480 particles:
+// 0.9 ms either way). A get outside plan() is an allocation of its own.
 struct DevArena {
     std::vector<void*> ptrs;
-    template <class T> T* get(size_t n) {
+    bool measuring = false;
+    char *next = nullptr, *end = nullptr;  // what is left of the planned allocation
+    size_t total = 0;
+    static constexpr size_t kAtOnce = size_t(16) << 20;
+    static size_t rounded(size_t bytes) { return (bytes + 255) / 256 * 256; }
+    void* allocate(size_t bytes) {
         void* p = nullptr;
-        size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
         cudaError_t e = cudaMalloc(&p, bytes);
         if (e != cudaSuccess) {
             cudaGetLastError();
             throw ApiError(MPS_ERR_NOMEM, "cudaMalloc of " + std::to_string(bytes) + " bytes failed");
         }
         ptrs.push_back(p);
-        return static_cast<T*>(p);
+        return p;
+    }
+    template <class T> T* get(size_t n) {
+        const size_t bytes = rounded(std::max<size_t>(n, 1) * sizeof(T));
+        if (measuring) {
+            total += bytes;
+            return nullptr;
+        }
+        if (size_t(end - next) >= bytes) {
+            char* p = next;
+            next += bytes;
+            return reinterpret_cast<T*>(p);
+        }
+        return static_cast<T*>(allocate(bytes));
+    }
+    // gets(): assigns every pointer by get() and does nothing else
+    template <class F> void plan(F&& gets) {
+        measuring = true;
+        total = 0;
+        gets();
+        measuring = false;
+        if (total >= kAtOnce) {
+            next = static_cast<char*>(allocate(total));
+            end = next + total;
+        }
+        gets();
+        next = end = nullptr;
     }
     ~DevArena() {
         for (void* p : ptrs) cudaFree(p);
@@ -606,12 +643,6 @@ template <class R, class RN> class Solver final : public SolverBase {
         CK(cudaMemsetAsync(io.pav, 0, sizeof(R) * nT, stream));
         if (nW > 0) {
             // walls: unsorted copy in id order, then one bucket build into w_*
-            V4<R>* sp = ar.template get<V4<R>>(3 * size_t(nW));
-            tw_pos = sp;
-            tw_vel = sp + nW;
-            tw_nrm = sp + 2 * size_t(nW);
-            tw_typ = ar.template get<int8_t>(nW);
-            tw_id = ar.template get<int>(nW);
             k_load_walls<R><<<blocks(nW, 256), 256, 0, stream>>>(nT, io.pos, io.vel, io.acc, io.typ,
                                                                  d_wall_ids, nW, tw_pos, tw_vel,
                                                                  tw_nrm, tw_id, tw_typ);
@@ -634,13 +665,40 @@ template <class R, class RN> class Solver final : public SolverBase {
     }
 
     void allocate() {
+        std::vector<int> rs(nscene + 1, 0);
+        int nbx_max = 0;
+        for (int s = 0; s < nscene; ++s) {
+            rs[s + 1] = rs[s] + hsc[s].nby * hsc[s].nbz;
+            nbx_max = std::max(nbx_max, hsc[s].nbx);
+        }
+        nrows = rs[nscene];
+        row_threads = nbx_max <= 64 ? 64 : (nbx_max <= 128 ? 128 : 256);
+        ar.plan([&] { take_arrays(); });
+        sbuf0 = S.pos;
+        // the fluid's own count table: the start-table pass leaves it zero for the next build
+        CK(cudaMemsetAsync(count_f, 0, sizeof(int) * size_t(LF()), stream));
+        const size_t F = std::max(nF, 1);
+        CK(cudaMemcpyAsync(row_scan, rs.data(), sizeof(int) * rs.size(), cudaMemcpyHostToDevice, stream));
+        CK(cudaMemsetAsync(count, 0, sizeof(int) * L(), stream));
+        CK(cudaMemsetAsync(part, 0, sizeof(int) * ((L() + kScan16Tile - 1) / kScan16Tile + 1), stream));
+        CK(cudaMemsetAsync(S.acc, 0, sizeof(V4<R>) * F, stream));
+        CK(cudaMemsetAsync(S2.acc, 0, sizeof(V4<R>) * F, stream));
+        CK(cudaMemsetAsync(M1.slot, 0, sizeof(int) * cap, stream));
+        CK(cudaMemsetAsync(mcs1, 0, sizeof(int) * (L() + 1), stream));
+        CK(cudaMemsetAsync(mcs2, 0, sizeof(int) * (L() + 1), stream));
+        CK(cudaMemsetAsync(near_m1, 1, L(), stream));  // walk everywhere until a mirror build
+        CK(cudaMemsetAsync(near_m2, 1, L(), stream));
+        CK(cudaStreamSynchronize(stream));  // rs leaves scope
+    }
+
+    // every array of the handle (DevArena::plan runs this twice)
+    void take_arrays() {
         const size_t F = std::max(nF, 1), W = std::max(nW, 1), T = std::max(nT, 1);
         d_sc = ar.template get<SD>(nscene);
         d_nbxyz = ar.template get<int>(nscene);
         for (FluidBuf<R>* b : {&S, &S2}) {
             b->pos = ar.template get<V4<R>>(F);
             b->vel = ar.template get<V4<R>>(F);
-            if (b == &S) sbuf0 = b->pos;
             b->acc = ar.template get<V4<R>>(F);
             b->prs = ar.template get<R>(F);
             b->pav = ar.template get<R>(F);
@@ -652,6 +710,11 @@ template <class R, class RN> class Solver final : public SolverBase {
         t_prs = ar.template get<R>(F);
         posp = ar.template get<V4<R>>(F);
         t_typ = ar.template get<int8_t>(F);
+        tw_pos = ar.template get<V4<R>>(W);
+        tw_vel = ar.template get<V4<R>>(W);
+        tw_nrm = ar.template get<V4<R>>(W);
+        tw_typ = ar.template get<int8_t>(W);
+        tw_id = ar.template get<int>(W);
         w_pos = ar.template get<V4<R>>(W);
         w_nrm = ar.template get<V4<R>>(W);
         w_vel = ar.template get<V4<R>>(W);
@@ -661,23 +724,10 @@ template <class R, class RN> class Solver final : public SolverBase {
         wcs = ar.template get<int>(L() + 1);
         cs = ar.template get<int>(size_t(LF()) + 1);
         csr = ar.template get<int>(size_t(LF()) + 1);
-        // the fluid's own count table: the start-table pass leaves it zero for the next build
         count_f = ar.template get<int>(size_t(LF()));
-        CK(cudaMemsetAsync(count_f, 0, sizeof(int) * size_t(LF()), stream));
-        {
-            std::vector<int> rs(nscene + 1, 0);
-            for (int s = 0; s < nscene; ++s) rs[s + 1] = rs[s] + hsc[s].nby * hsc[s].nbz;
-            nrows = rs[nscene];
-            int nbx_max = 0;
-            for (int s = 0; s < nscene; ++s) nbx_max = std::max(nbx_max, hsc[s].nbx);
-            row_threads = nbx_max <= 64 ? 64 : (nbx_max <= 128 ? 128 : 256);
-            row_scan = ar.template get<int>(rs.size());
-            row_tot = ar.template get<int>(size_t(nrows));
-            frow_tot = ar.template get<int>(9 * size_t(nrows));
-            CK(cudaMemcpyAsync(row_scan, rs.data(), sizeof(int) * rs.size(), cudaMemcpyHostToDevice,
-                               stream));
-            CK(cudaStreamSynchronize(stream));  // rs leaves scope
-        }
+        row_scan = ar.template get<int>(size_t(nscene) + 1);
+        row_tot = ar.template get<int>(size_t(nrows));
+        frow_tot = ar.template get<int>(9 * size_t(nrows));
         posf = ar.template get<V4<R>>(F);
         for (MirrorBuf<R>* b : {&U, &M1, &M2}) {
             b->pos = ar.template get<V4<R>>(cap);
@@ -691,8 +741,6 @@ template <class R, class RN> class Solver final : public SolverBase {
         seg = ar.template get<int>(items);
         count = ar.template get<int>(L());
         part = ar.template get<int>((L() + kScan16Tile - 1) / kScan16Tile + 1);
-        CK(cudaMemsetAsync(count, 0, sizeof(int) * L(), stream));
-        CK(cudaMemsetAsync(part, 0, sizeof(int) * ((L() + kScan16Tile - 1) / kScan16Tile + 1), stream));
         d_fluid_ids = ar.template get<int>(F);
         d_wall_ids = ar.template get<int>(W);
         d_nF = ar.template get<int>(1);
@@ -713,13 +761,6 @@ template <class R, class RN> class Solver final : public SolverBase {
         near_m1 = ar.template get<int8_t>(L());
         near_m2 = ar.template get<int8_t>(L());
         nbcnt = ar.template get<int>(F);
-        CK(cudaMemsetAsync(S.acc, 0, sizeof(V4<R>) * F, stream));
-        CK(cudaMemsetAsync(S2.acc, 0, sizeof(V4<R>) * F, stream));
-        CK(cudaMemsetAsync(M1.slot, 0, sizeof(int) * cap, stream));
-        CK(cudaMemsetAsync(mcs1, 0, sizeof(int) * (L() + 1), stream));
-        CK(cudaMemsetAsync(mcs2, 0, sizeof(int) * (L() + 1), stream));
-        CK(cudaMemsetAsync(near_m1, 1, L(), stream));  // walk everywhere until a mirror build
-        CK(cudaMemsetAsync(near_m2, 1, L(), stream));
     }
 
     // ---- bucket build ------------------------------------------------------------------
@@ -1665,38 +1706,39 @@ template <class R, class RN> class Solver final : public SolverBase {
         st->nbK = nbK;
         DevArena& a = st->ar;
         const size_t F = std::max(nF, 1), T = std::max(nT, 1), Cm = size_t(cap), Lc = L() + 1;
-        for (int c = 0; c <= nck; ++c)
-            st->ck.push_back(Ckpt{a.template get<R>(3 * T), a.template get<R>(3 * T),
-                                  a.template get<R>(T), a.template get<R>(T),
-                                  a.template get<int8_t>(T)});
-        for (int k = 0; k < every; ++k) {
-            TapeStep<R> t;
-            t.pid1 = a.template get<int>(F); t.x1 = a.template get<V4<R>>(F);
-            t.v1 = a.template get<V4<R>>(F); t.up1 = a.template get<V4<R>>(F);
-            t.nA = a.template get<int>(F); t.nbA = a.template get<int>(list_size(F, nbK));
-            t.m1pos = a.template get<V4<R>>(Cm); t.m1slot = a.template get<int>(Cm);
-            t.m1nrm = a.template get<V4<R>>(Cm); t.mcs1 = a.template get<int>(Lc);
-            t.pid2 = a.template get<int>(F); t.x2 = a.template get<V4<R>>(F);
-            t.u2 = a.template get<V4<R>>(F); t.vv2 = a.template get<V4<R>>(F);
-            t.P2 = a.template get<R>(F); t.vp2 = a.template get<V4<R>>(F);
-            t.nB = a.template get<int>(F); t.nbB = a.template get<int>(list_size(F, nbK));
-            t.m2pos = a.template get<V4<R>>(Cm); t.m2slot = a.template get<int>(Cm);
-            t.m2nrm = a.template get<V4<R>>(Cm); t.mcs2 = a.template get<int>(Lc);
-            st->tape.push_back(t);
-        }
-        st->unrm = a.template get<V4<R>>(Cm);
-        for (V4<double>** p : {&st->lx, &st->lv, &st->lx_acc, &st->lxs_pid, &st->lu_pid})
-            *p = a.template get<V4<double>>(T);
-        for (V4<double>** p : {&st->lG, &st->lvv, &st->lxs, &st->lx_at, &st->la, &st->lxa, &st->lva})
-            *p = a.template get<V4<double>>(F);
-        st->lP = a.template get<double>(F);
-        st->lP_at = a.template get<double>(F);
-        st->lkn = a.template get<double>(1);
-        st->stage = a.template get<double>(3 * T);
-        st->pmin = a.template get<R>(F);
-        st->am = a.template get<int>(F);
-        st->inv2 = a.template get<int>(T);
-        st->err = a.template get<int>(1);
+        st->ck.resize(nck + 1);
+        st->tape.resize(every);
+        a.plan([&] {
+            for (Ckpt& c : st->ck)
+                c = Ckpt{a.template get<R>(3 * T), a.template get<R>(3 * T), a.template get<R>(T),
+                         a.template get<R>(T), a.template get<int8_t>(T)};
+            for (TapeStep<R>& t : st->tape) {
+                t.pid1 = a.template get<int>(F); t.x1 = a.template get<V4<R>>(F);
+                t.v1 = a.template get<V4<R>>(F); t.up1 = a.template get<V4<R>>(F);
+                t.nA = a.template get<int>(F); t.nbA = a.template get<int>(list_size(F, nbK));
+                t.m1pos = a.template get<V4<R>>(Cm); t.m1slot = a.template get<int>(Cm);
+                t.m1nrm = a.template get<V4<R>>(Cm); t.mcs1 = a.template get<int>(Lc);
+                t.pid2 = a.template get<int>(F); t.x2 = a.template get<V4<R>>(F);
+                t.u2 = a.template get<V4<R>>(F); t.vv2 = a.template get<V4<R>>(F);
+                t.P2 = a.template get<R>(F); t.vp2 = a.template get<V4<R>>(F);
+                t.nB = a.template get<int>(F); t.nbB = a.template get<int>(list_size(F, nbK));
+                t.m2pos = a.template get<V4<R>>(Cm); t.m2slot = a.template get<int>(Cm);
+                t.m2nrm = a.template get<V4<R>>(Cm); t.mcs2 = a.template get<int>(Lc);
+            }
+            st->unrm = a.template get<V4<R>>(Cm);
+            for (V4<double>** p : {&st->lx, &st->lv, &st->lx_acc, &st->lxs_pid, &st->lu_pid})
+                *p = a.template get<V4<double>>(T);
+            for (V4<double>** p : {&st->lG, &st->lvv, &st->lxs, &st->lx_at, &st->la, &st->lxa, &st->lva})
+                *p = a.template get<V4<double>>(F);
+            st->lP = a.template get<double>(F);
+            st->lP_at = a.template get<double>(F);
+            st->lkn = a.template get<double>(1);
+            st->stage = a.template get<double>(3 * T);
+            st->pmin = a.template get<R>(F);
+            st->am = a.template get<int>(F);
+            st->inv2 = a.template get<int>(T);
+            st->err = a.template get<int>(1);
+        });
         st->nck = nck;
         st->every = every;
         adj = std::move(st);
