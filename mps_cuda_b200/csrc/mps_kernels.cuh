@@ -2422,48 +2422,27 @@ __global__ void __launch_bounds__(128) k_ph_gen(const __grid_constant__ PassArgs
 }
 
 // d_MRRinout (kernel.cu:932-985) over the raw mirrors; a culled mirror's slot becomes
-// negative. Sixteen lanes share a mirror: lane r < 9 finds bucket row r's range of walls
-// (for_rows's rows and skipping), and the lanes stride over each row. The group keeps the
-// smallest distance, on ties the earlier row, then the earlier wall: the wall the sequential
-// walk keeps (the first nearest one found).
-constexpr int kCullLanes = 16;
-template <class R, class RN>
+// negative. LANES lanes share a mirror; lane `part` finds the ranges of walls of the bucket rows r
+// with r % LANES == part (for_rows's rows and skipping). Sixteen lanes stride over each row in
+// turn, which is the shorter chain for the mirrors of a small scene; four walk a row each, which
+// needs fewer lanes where the mirrors fill the GPU (two generations and culls, us: 48 000
+// particles 220 with four lanes, 205 with sixteen; 384 000 in FP64 382 and 343; 6.1M 768 and 796;
+// 64 scenes of 1.1M 819 and 888). The group keeps the smallest distance, on ties the earlier row, then the earlier wall:
+// the wall the sequential walk keeps (the first nearest one found).
+template <class R, class RN, int LANES>
 __global__ void k_ph_cull(const __grid_constant__ PassArgs<R, RN> a) {
     const int n = min(a.cnt->mirror_raw, a.out.cap);
-    const int part = threadIdx.x & (kCullLanes - 1), first = threadIdx.x & 31 & ~(kCullLanes - 1);
-    const int groups = (gridDim.x * blockDim.x) / kCullLanes;
+    const int part = threadIdx.x & (LANES - 1), first = threadIdx.x & 31 & ~(LANES - 1);
+    const int groups = (gridDim.x * blockDim.x) / LANES;
     const int nround = (n + groups - 1) / groups * groups;  // every lane loops alike
-    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) / kCullLanes; t < nround; t += groups) {
+    for (int t = (blockIdx.x * blockDim.x + threadIdx.x) / LANES; t < nround; t += groups) {
         const int sl = t < n ? a.out.slot[t] : -1;
         R wd = R(0);
         int wrow = 9, wj = -1, lo = 0, hi = 0;
         V4<R> q{R(0), R(0), R(0), R(0)};
         const SceneDev<R, RN>* scp = a.sc;
-        if (sl >= 0) {
-            scp = &a.sc[a.nscene > 1 ? scene_of(a.sc, a.nscene, sl / kNumMRR) : 0];
-            q = a.out.pos[t];
-            int ix, iy, iz;
-            if (!cell_of(*scp, q.x, q.y, q.z, ix, iy, iz) && part == 0) atomicAdd(&a.cnt->err_cell, 1);
-            wd = scp->wall_dist0;
-            if (part < 9) {
-                const RowCtx<R> c = row_ctx(*scp, q.x, q.y, q.z, ix, iy, iz);
-                const R B = a.skip != 0 ? scp->skip_r : R(INFINITY);
-                const int dz = part / 3 - 1, dy = part % 3 - 1;
-                const R ddz = dz < 0 ? c.dzl : (dz > 0 ? c.dzh : R(0));
-                const R ddy = dy < 0 ? c.dyl : (dy > 0 ? c.dyh : R(0));
-                const R dyz2 = ddy * ddy + ddz * ddz;
-                if (!(dyz2 > B)) {
-                    const int jl = (dyz2 + c.dxl * c.dxl <= B) ? c.ix - 1 : c.ix;
-                    const int jh = (dyz2 + c.dxh * c.dxh <= B) ? c.ix + 1 : c.ix;
-                    const int row = scp->cbase + (c.iz + dz) * scp->nbxy + (c.iy + dy) * scp->nbx;
-                    lo = __ldg(a.wl.cs + row + jl);
-                    hi = __ldg(a.wl.cs + row + jh + 1);
-                }
-            }
-        }
-        for (int r = 0; r < 9; ++r) {
-            const int l = __shfl_sync(kFull, lo, first + r), h = __shfl_sync(kFull, hi, first + r);
-            for (int j = l + part; j < h; j += kCullLanes) {
+        auto nearest = [&](int r, int j0, int j1, int step) {
+            for (int j = j0; j < j1; j += step) {
                 const V4<R> w = ldg4(a.wl.pos + j);
                 const R dx = q.x - w.x, dy = q.y - w.y, dz = q.z - w.z;
                 const R d2 = dot3(dx, dy, dz, dx, dy, dz);
@@ -2476,8 +2455,37 @@ __global__ void k_ph_cull(const __grid_constant__ PassArgs<R, RN> a) {
                     }
                 }
             }
+        };
+        if (sl >= 0) {
+            scp = &a.sc[a.nscene > 1 ? scene_of(a.sc, a.nscene, sl / kNumMRR) : 0];
+            q = a.out.pos[t];
+            int ix, iy, iz;
+            if (!cell_of(*scp, q.x, q.y, q.z, ix, iy, iz) && part == 0) atomicAdd(&a.cnt->err_cell, 1);
+            wd = scp->wall_dist0;
+            const RowCtx<R> c = row_ctx(*scp, q.x, q.y, q.z, ix, iy, iz);
+            const R B = a.skip != 0 ? scp->skip_r : R(INFINITY);
+#pragma unroll 1
+            for (int r = part; r < 9; r += LANES) {
+                const int dz = r / 3 - 1, dy = r % 3 - 1;
+                const R ddz = dz < 0 ? c.dzl : (dz > 0 ? c.dzh : R(0));
+                const R ddy = dy < 0 ? c.dyl : (dy > 0 ? c.dyh : R(0));
+                const R dyz2 = ddy * ddy + ddz * ddz;
+                if (!(dyz2 > B)) {
+                    const int jl = (dyz2 + c.dxl * c.dxl <= B) ? c.ix - 1 : c.ix;
+                    const int jh = (dyz2 + c.dxh * c.dxh <= B) ? c.ix + 1 : c.ix;
+                    const int row = scp->cbase + (c.iz + dz) * scp->nbxy + (c.iy + dy) * scp->nbx;
+                    lo = __ldg(a.wl.cs + row + jl);
+                    hi = __ldg(a.wl.cs + row + jh + 1);
+                    if (LANES < 9) nearest(r, lo, hi, 1);
+                }
+            }
         }
-        for (int o = kCullLanes / 2; o > 0; o >>= 1) {
+        if (LANES >= 9)
+            for (int r = 0; r < 9; ++r) {
+                const int l = __shfl_sync(kFull, lo, first + r), h = __shfl_sync(kFull, hi, first + r);
+                nearest(r, l + part, h, LANES);
+            }
+        for (int o = LANES / 2; o > 0; o >>= 1) {
             const R od = __shfl_xor_sync(kFull, wd, o);
             const int orow = __shfl_xor_sync(kFull, wrow, o), oj = __shfl_xor_sync(kFull, wj, o);
             const bool tie = od == wd && (orow < wrow || (orow == wrow && oj < wj));

@@ -328,7 +328,7 @@ struct SolverBase {
     long long steps = 0;
     long long launches = 0;       // kernels launched (graph replays included)
     long long head_launches = 0;  // kernels of one captured step up to PrsGrdTrm
-    long long tail_launches = 0;  // kernels of one captured step end (mirrors, bucket builds)
+    long long step_launches = 0;  // ... with the end of the step before it
     bool timing_on = false;
     double t_ms[MPS_K_COUNT] = {};
     long long t_n[MPS_K_COUNT] = {};
@@ -421,7 +421,8 @@ template <class R, class RN> class Solver final : public SolverBase {
     int row_threads = 256;  // threads per bucket row block: the longest row rounded up
     bool posf_stale = false;  // particles moved in place since the copy was made
     // bucket-build scratch
-    int *key, *rnk, *seg, *count, *part;
+    int *key, *rnk, *seg, *count, *part;  // walls and mirrors
+    int *key_f, *rnk_f, *seg_f;           // fluid: its build runs beside a mirror build
     int* d_fluid_ids;
     int* d_wall_ids;
     int* d_nF;
@@ -438,14 +439,14 @@ template <class R, class RN> class Solver final : public SolverBase {
     int nbK = kListCap;                    // list capacity in use (MPS_OPT_LIST_CAPACITY)
     std::vector<int> fluid_ids, wall_ids;
     bool lists_valid = false, sorted = false, m1_valid = false, acc_dirty = false;
-    // Captured graphs of a step's body (passes A to C, moving walls) and of a step's end (the
-    // next step's mirrors and bucket builds), one per buffer the sorted state starts in: each
-    // holds one fluid bucket build, which moves the state from S to S2, so a graph's baked
-    // pointers fit only the buffer it was captured from. A replay swaps S and S2 on the host
+    // Captured graphs of a step's body (passes A to C, moving walls), and of the end of the step
+    // before it (mirrors, bucket builds) with the body, one per buffer the sorted state starts in:
+    // a fluid bucket build moves the state from S to S2, so a graph's baked pointers fit only the
+    // buffer it was captured from. A replay swaps S and S2 on the host
     // as the captured build did.
     cudaGraphExec_t gx_head[2] = {nullptr, nullptr};
-    cudaGraphExec_t gx_tail[2] = {nullptr, nullptr};
-    int swaps_head = 0, swaps_tail = 0;  // fluid bucket builds in each
+    cudaGraphExec_t gx_step[2] = {nullptr, nullptr};
+    int swaps_head = 0, swaps_step = 0;  // fluid bucket builds in each
     const void* sbuf0 = nullptr;          // S.pos at allocation: buffer 0
     int swap_count = 0;                   // fluid bucket builds issued on the host
     bool gexec_diag = false;
@@ -535,7 +536,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     ~Solver() override {
         for (int b = 0; b < 2; ++b) {
             if (gx_head[b]) cudaGraphExecDestroy(gx_head[b]);
-            if (gx_tail[b]) cudaGraphExecDestroy(gx_tail[b]);
+            if (gx_step[b]) cudaGraphExecDestroy(gx_step[b]);
         }
         for (auto& pe : ev_pending) {
             cudaEventDestroy(pe.second.first);
@@ -735,10 +736,13 @@ template <class R, class RN> class Solver final : public SolverBase {
         }
         mcs1 = ar.template get<int>(L() + 1);
         mcs2 = ar.template get<int>(L() + 1);
-        const size_t items = std::max<size_t>({F, W, size_t(cap)});
+        const size_t items = std::max<size_t>(W, size_t(cap));
         key = ar.template get<int>(items);
         rnk = ar.template get<int>(items);
         seg = ar.template get<int>(items);
+        key_f = ar.template get<int>(F);
+        rnk_f = ar.template get<int>(F);
+        seg_f = ar.template get<int>(F);
         count = ar.template get<int>(L());
         part = ar.template get<int>((L() + kScan16Tile - 1) / kScan16Tile + 1);
         d_fluid_ids = ar.template get<int>(F);
@@ -796,10 +800,10 @@ template <class R, class RN> class Solver final : public SolverBase {
         FluidKeySrc<R, RN> ks{d_sc, nscene, deadF(), pos, typ, pid};
         FluidGatherF<R, RN> g{{pos, vel, acc, prs, pav, pid, typ, S2.pos, S2.vel, S2.acc, S2.prs,
                                S2.pav, S2.pid, S2.typ},
-                              d_sc, nscene, key, cs, csr, posf};
+                              d_sc, nscene, key_f, cs, csr, posf};
         const int grid = std::min(blocks(std::max(nF, 1), 256), 148 * 32);
         if (nF > 0) {
-            k_bin_key<FluidKeySrc<R, RN>><<<grid, 256, 0, stream>>>(ks, nullptr, nF, key, rnk,
+            k_bin_key<FluidKeySrc<R, RN>><<<grid, 256, 0, stream>>>(ks, nullptr, nF, key_f, rnk_f,
                                                                     count_f, nullptr, cnt);
             KL();
         }
@@ -808,10 +812,11 @@ template <class R, class RN> class Solver final : public SolverBase {
         else if (row_threads == 128) fine_rows<128>(fr);
         else fine_rows<256>(fr);
         if (nF > 0) {
-            k_bin_seg<FluidKeySrc<R, RN>><<<grid, 256, 0, stream>>>(ks, nullptr, nF, key, rnk, cs, seg);
+            k_bin_seg<FluidKeySrc<R, RN>><<<grid, 256, 0, stream>>>(ks, nullptr, nF, key_f, rnk_f, cs,
+                                                                    seg_f);
             KL();
             k_bin_fin<FluidKeySrc<R, RN>, FluidGatherF<R, RN>><<<grid, 256, 0, stream>>>(
-                ks, g, nullptr, nF, key, rnk, cs, seg, deadF());
+                ks, g, nullptr, nF, key_f, rnk_f, cs, seg_f, deadF());
             KL();
         }
         std::swap(S, S2);
@@ -870,9 +875,11 @@ template <class R, class RN> class Solver final : public SolverBase {
 
     // MRRinout over the raw mirrors (culled slots turn negative)
     void cull_raw() {
-        const long long lanes = (long long)kCullLanes * cap;
+        const bool few = nF <= kCullMost;
+        const long long lanes = (long long)(few ? 16 : 4) * cap;
         const int grid = int(std::min<long long>((lanes + 255) / 256, 148 * 32));
-        k_ph_cull<R, RN><<<grid, 256, 0, stream>>>(args(M1, mcs1));
+        if (few) k_ph_cull<R, RN, 16><<<grid, 256, 0, stream>>>(args(M1, mcs1));
+        else k_ph_cull<R, RN, 4><<<grid, 256, 0, stream>>>(args(M1, mcs1));
         KL();
     }
 
@@ -889,7 +896,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     //              167 / 79 / 52     211 / 86 / 95     205 / 119 / 151   203 / 139 / 209   198 / 207
     // and the FP64 crossings lie at the same sizes.
     static constexpr int kWarpMost = 5000, kGroupMostA = 65536, kGroupMostBC = 98304,
-                         kGroupMostGen = 180000;
+                         kGroupMostGen = 180000, kCullMost = 600000;
     int group_lanes(int most) const { return nF <= kWarpMost ? 32 : (nF <= most ? 8 : 0); }
     int list_layout() const { return group_lanes(kGroupMostBC) ? kListGroup : kListThread; }
     int group_grid(int g) const { return blocks(nF, 128 / g); }
@@ -1107,34 +1114,35 @@ template <class R, class RN> class Solver final : public SolverBase {
     // The generation reads t_pos, t_prs, t_typ, the pre-build S.pid, the walls and the near
     // flags and writes the raw mirrors; the fluid build reads the same t_* and S arrays and
     // writes S2, its start tables, posf and its own key/rank scratch. Neither writes what the
-    // other reads, so with overlap_on the build runs on the second stream beside the
-    // generation and its cull, and the mirror bucket build (which reuses the key/rank
-    // scratch) waits for both. Both launches are issued before the build swaps S and S2 on
-    // the host, so the generation's arguments name the pre-build arrays either way.
+    // other reads, so with bit 0 of overlap the mirrors (generation, cull and bucket build, which
+    // have scratch of their own) run on the second stream beside the fluid build. The generation
+    // is launched before the build swaps S and S2 on the host, so its arguments name the
+    // pre-build arrays.
     void step_tail() {
         const int bg = blk[MPS_K_GEN];
         const bool fork = (overlap & 1) && !timing_on;
-        reset_raw();
+        auto mirrors = [&] {
+            reset_raw();
+            Scope t(this, MPS_K_GEN);
+            run_gen<false, false>(args(M2, mcs2), bg, t_pos, t_prs, t_typ);
+        };
         if (fork) {
             ensure_side();
             CK(cudaEventRecord(ev_fork, stream));
             CK(cudaStreamWaitEvent(side, ev_fork, 0));
-        }
-        {
-            Scope t(this, MPS_K_GEN);
-            run_gen<false, false>(args(M2, mcs2), bg, t_pos, t_prs, t_typ);
-        }
-        if (fork) {
             {
                 OnStream o(this, side);
-                bin_fluid(t_pos, t_vel, nullptr, t_prs, S.pav, S.pid, t_typ);
+                mirrors();
+                bin_mirrors(M1, mcs1);
                 CK(cudaEventRecord(ev_join, side));
             }
+            bin_fluid(t_pos, t_vel, nullptr, t_prs, S.pav, S.pid, t_typ);
             CK(cudaStreamWaitEvent(stream, ev_join, 0));
         } else {
+            mirrors();
             bin_fluid(t_pos, t_vel, nullptr, t_prs, S.pav, S.pid, t_typ);
+            bin_mirrors(M1, mcs1);
         }
-        bin_mirrors(M1, mcs1);
     }
 
     // runs the pending end of the latest step, if any (before reading the sorted state)
@@ -1312,8 +1320,8 @@ template <class R, class RN> class Solver final : public SolverBase {
     void invalidate_graph() override {
         for (int b = 0; b < 2; ++b) {
             if (gx_head[b]) cudaGraphExecDestroy(gx_head[b]);
-            if (gx_tail[b]) cudaGraphExecDestroy(gx_tail[b]);
-            gx_head[b] = gx_tail[b] = nullptr;
+            if (gx_step[b]) cudaGraphExecDestroy(gx_step[b]);
+            gx_head[b] = gx_step[b] = nullptr;
         }
     }
 
@@ -1343,14 +1351,17 @@ template <class R, class RN> class Solver final : public SolverBase {
         gexec_diag = diag_on;
         for (int k = 0; k < n; ++k) {
             if (tail_pending) {
-                if (use_graph) run_graph(gx_tail, tail_launches, swaps_tail, [&] { step_tail(); });
-                else step_tail();
-                tail_pending = false;
-            } else if (!(lists_valid && sorted && m1_valid) || acc_dirty) {
-                prepare_fused();
+                auto whole = [&] {
+                    step_tail();
+                    run_body();
+                };
+                if (use_graph) run_graph(gx_step, step_launches, swaps_step, whole);
+                else whole();
+            } else {
+                if (!(lists_valid && sorted && m1_valid) || acc_dirty) prepare_fused();
+                if (use_graph) run_graph(gx_head, head_launches, swaps_head, [&] { run_body(); });
+                else run_body();
             }
-            if (use_graph) run_graph(gx_head, head_launches, swaps_head, [&] { run_body(); });
-            else run_body();
             tail_pending = true;
             lists_valid = sorted = m1_valid = true;  // as the pending end will leave them
         }
