@@ -590,6 +590,84 @@ template <class R> struct NormalSet {
     }
 };
 
+// A wall's class, kept in its position's w: walls with equal normals share a number, its lowest
+// bit says whether the wall is an Edge wall (k_wall_code). Registration then compares one integer
+// that comes with the position, where it would gather each wall's normal and flag: two generations
+// and culls at 384 000 particles 237 to 192 us (FP64 343 to 307), at 6.1M 768 to 690, for 64 scenes
+// of 1.1M 818 to 710. Walls that have moved carry no classes.
+__device__ __forceinline__ int wall_code(int cls, bool edge) { return 2 * cls + (edge ? 1 : 0); }
+
+// a set of up to kNumMRR classes in arrival order, the first three in registers
+struct ClassSet {
+    int n = 0, a = -1, b = -1, c = -1;
+    int rest[kNumMRR - 3];
+    __device__ __forceinline__ bool has(int k) const {
+        if (a == k || b == k || c == k) return true;
+        for (int i = 3; i < n; ++i)
+            if (rest[i - 3] == k) return true;
+        return false;
+    }
+    __device__ __forceinline__ void add(int k) {
+        if (n == 0) a = k;
+        else if (n == 1) b = k;
+        else if (n == 2) c = k;
+        else rest[n - 3] = k;
+        ++n;
+    }
+};
+
+// plan_mirrors (below) by the walls' classes
+template <class R, class RN>
+__device__ __forceinline__ int plan_mirrors_cls(const SceneDev<R, RN>& sc, const RowCtx<R>& c, R x,
+                                                R y, R z, const WallView<R>& wl, bool skip,
+                                                MirrorPlan<R>& pl) {
+    ClassSet reg, edge;
+    int ew[kNumMRR], last = -1, nwall = 0;  // the registered Edge walls, the last one's class
+    const R B = skip ? sc.skip_r : R(INFINITY);
+    for_rows(sc, wl.cs, c, B, [&](int j) {
+        const V4<R> q = ldg4(wl.pos + j);
+        const R dx = x - q.x, dy = y - q.y, dz = z - q.z;
+        if (!(dot3(dx, dy, dz, dx, dy, dz) <= sc.r2)) return;
+        ++nwall;
+        const int code = w_slot(q.w), k = code >> 1;
+        if (reg.n < kNumMRR && !reg.has(k)) {
+            pl.reg[reg.n] = j;
+            reg.add(k);
+        }
+        if ((code & 1) && edge.n < kNumMRR && !edge.has(k)) {
+            ew[edge.n] = j;
+            last = k;
+            edge.add(k);
+        }
+    });
+    pl.nreg = reg.n;
+    pl.corner = -1;
+    if (reg.n > 0 && edge.n >= 2) {
+        R sx = R(0), sy = R(0), sz = R(0);
+        for (int k = 0; k < edge.n; ++k) {
+            const V4<R> n = ldg4(wl.nrm + ew[k]);
+            sx += n.x; sy += n.y; sz += n.z;
+        }
+        const R as = sqrtR(dot3(sx, sy, sz, sx, sy, sz));
+        pl.sx = sx / as; pl.sy = sy / as; pl.sz = sz / as;
+        pl.corner = ew[edge.n - 1];
+        if (edge.n == 2) {
+            R best = R(INFINITY);
+            for_rows(sc, wl.cs, c, B, [&](int j) {
+                const V4<R> q = ldg4(wl.pos + j);
+                if (w_slot(q.w) != wall_code(last, true)) return;
+                const R dx = x - q.x, dy = y - q.y, dz = z - q.z;
+                const R d2 = dot3(dx, dy, dz, dx, dy, dz);
+                if (d2 <= sc.r2 && d2 < best) {
+                    best = d2;
+                    pl.corner = j;
+                }
+            });
+        }
+    }
+    return nwall;
+}
+
 // registration (kernel.cu:741-800): every distinct normal once, the first wall found wins;
 // Edge walls likewise. Returns the number of walls inside r (diagnostic).
 template <class R, class RN>

@@ -1956,10 +1956,11 @@ __global__ void __launch_bounds__(128) k_pass_c_g(const __grid_constant__ PassAr
 }
 
 // ---- mirror generation with a group of lanes per particle ---------------------------------
-// scratch: also the distinct normals met, [0] of all walls, [1] of Edge walls, in order of arrival
+// scratch: also the distinct normals met, [0] of all walls, [1] of Edge walls, in order of arrival,
+// the wall each comes from and its code (wall_code)
 template <class R, int P> struct GroupMemG : GroupMem<R, P, 1> {
     R n[2][P][kNumMRR][3];
-    int id[2][P][kNumMRR];
+    int id[2][P][kNumMRR], code[2][P][kNumMRR];
 };
 
 // One mirror of particle (x, y, z): its reflection through the plane of wall position q with
@@ -1998,7 +1999,7 @@ __device__ __noinline__ int gen_single(const PassArgs<R, RN>& a, int s, V4<R> p,
 // k_gen_cull with G lanes per particle: the walls inside r are found together, the distinct
 // normals registered by ballots (the first lane with a new normal registers it for the group),
 // and one lane per registered normal makes its mirror.
-template <class R, class RN, bool DIAG, bool TAPE, int G>
+template <class R, class RN, bool DIAG, bool TAPE, bool CLS, int G>
 __global__ void __launch_bounds__(128) k_gen_cull_g(const __grid_constant__ PassArgs<R, RN> a,
                                                     const V4<R>* gpos, const R* gprs,
                                                     const int8_t* gtyp) {
@@ -2048,33 +2049,36 @@ __global__ void __launch_bounds__(128) k_gen_cull_g(const __grid_constant__ Pass
                 const int h = h0 + gr.l;
                 const bool on = h < n;
                 const int j = on ? m.kidx[m.hit[gr.g][h]] : 0;
-                const V4<R> nv = ldg4(a.wl.nrm + j);
-                const bool edge = on && __ldg(a.wl.wse + j) == kEDGE;
+                // by class: the position, just tested, carries the code; else the normal and flag
+                const V4<R> nv = CLS ? ldg4(a.wl.pos + j) : ldg4(a.wl.nrm + j);
+                const int code = CLS ? w_slot(nv.w) : 0;
+                const bool edge = on && (CLS ? (code & 1) != 0 : __ldg(a.wl.wse + j) == kEDGE);
+                auto same = [&](int e, int k) {
+                    if (CLS) return (m.code[e][gr.g][k] >> 1) == (code >> 1);
+                    const R* w = m.n[e][gr.g][k];
+                    return w[0] == nv.x && w[1] == nv.y && w[2] == nv.z;
+                };
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     bool fresh = e == 0 ? on : edge;
                     fresh = fresh && nn[e] < kNumMRR;
-                    for (int k = 0; k < nn[e]; ++k) {
-                        const R* w = m.n[e][gr.g][k];
-                        fresh = fresh && !(w[0] == nv.x && w[1] == nv.y && w[2] == nv.z);
-                    }
+                    for (int k = 0; k < nn[e]; ++k) fresh = fresh && !same(e, k);
                     unsigned b;
                     while ((b = __ballot_sync(kFull, fresh)) != 0u) {
                         const unsigned gb = gr.mine(b);
                         if (gb) {
                             if (gr.l == __ffs(gb) - 1) {
-                                m.n[e][gr.g][nn[e]][0] = nv.x;
-                                m.n[e][gr.g][nn[e]][1] = nv.y;
-                                m.n[e][gr.g][nn[e]][2] = nv.z;
+                                const V4<R> t = CLS ? ldg4(a.wl.nrm + j) : nv;
+                                m.n[e][gr.g][nn[e]][0] = t.x;
+                                m.n[e][gr.g][nn[e]][1] = t.y;
+                                m.n[e][gr.g][nn[e]][2] = t.z;
                                 m.id[e][gr.g][nn[e]] = j;
+                                m.code[e][gr.g][nn[e]] = code;
                             }
                             ++nn[e];
                         }
                         __syncwarp();
-                        if (fresh) {
-                            const R* w = m.n[e][gr.g][nn[e] - 1];
-                            fresh = nn[e] < kNumMRR && !(w[0] == nv.x && w[1] == nv.y && w[2] == nv.z);
-                        }
+                        fresh = fresh && nn[e] < kNumMRR && !same(e, nn[e] - 1);
                         __syncwarp();
                     }
                 }
@@ -2102,10 +2106,15 @@ __global__ void __launch_bounds__(128) k_gen_cull_g(const __grid_constant__ Pass
                 if (total > Mem::kWindow) n = walls(w0);
                 for (int h = gr.l; two && h < n; h += G) {
                     const int j = m.kidx[m.hit[gr.g][h]];
-                    if (__ldg(a.wl.wse + j) != kEDGE) continue;
-                    const V4<R> nv = ldg4(a.wl.nrm + j);
-                    if (nv.x != ln[0] || nv.y != ln[1] || nv.z != ln[2]) continue;
-                    const R d2 = pair_d2(ldg4(a.wl.pos + j), p);
+                    const V4<R> q = ldg4(a.wl.pos + j);
+                    if (CLS) {
+                        if (w_slot(q.w) != m.code[1][gr.g][1]) continue;
+                    } else {
+                        if (__ldg(a.wl.wse + j) != kEDGE) continue;
+                        const V4<R> nv = ldg4(a.wl.nrm + j);
+                        if (nv.x != ln[0] || nv.y != ln[1] || nv.z != ln[2]) continue;
+                    }
+                    const R d2 = pair_d2(q, p);
                     if (d2 < best) {
                         best = d2;
                         bj = j;
@@ -2196,7 +2205,8 @@ __device__ __forceinline__ void gen_reserve_emit(const PassArgs<R, RN>& a, const
 // instead of stretching the neighbour passes. With gprs null a mirror's pressure field holds
 // its owner's slot instead, for k_mirror_prs to replace once the pressures exist: the
 // positions of the second generation need only x*, so they are made beside pass B.
-template <class R, class RN, bool DIAG, bool TAPE = false>
+// CLS: the walls carry their classes.
+template <class R, class RN, bool DIAG, bool TAPE, bool CLS>
 __global__ void __launch_bounds__(128, min_blocks<R>(10)) k_gen_cull(const __grid_constant__ PassArgs<R, RN> a, const V4<R>* gpos,
                                                   const R* gprs, const int8_t* gtyp) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2216,7 +2226,8 @@ __global__ void __launch_bounds__(128, min_blocks<R>(10)) k_gen_cull(const __gri
         // no wall in the 27 buckets around: no wall within r, no mirror (the common case)
         if (__ldg(a.near_wall + sc.cbase + iz * sc.nbxy + iy * sc.nbx + ix)) {
             RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
-            nw = plan_mirrors(sc, c, p.x, p.y, p.z, a.wl, a.skip != 0, pl);
+            if constexpr (CLS) nw = plan_mirrors_cls(sc, c, p.x, p.y, p.z, a.wl, a.skip != 0, pl);
+            else nw = plan_mirrors(sc, c, p.x, p.y, p.z, a.wl, a.skip != 0, pl);
             m = count_mirrors<R, RN>(pl, p.x, p.y, p.z, a.wl, a.cnt);
             P = gprs ? gprs[s] : slot_w(s, R(0));
         }
@@ -2586,6 +2597,17 @@ __global__ void k_surface_edge(const SceneDev<R, RN>* scs, int nscene, int nW, W
         }
     });
     wse[t] = edge ? int8_t(kEDGE) : int8_t(0);
+}
+
+// the sorted walls' codes: the class that came in w with each position, and the Edge flag
+template <class R> __global__ void k_wall_code(int nW, V4<R>* pos, const int8_t* wse) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < nW) pos[t].w = slot_w(wall_code(w_slot(pos[t].w), wse[t] == kEDGE), R(0));
+}
+// the load-order walls' classes
+template <class R> __global__ void k_wall_class(int nW, V4<R>* pos, const int* cls) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < nW) pos[t].w = slot_w(cls[t], R(0));
 }
 
 // ---------------------------------------------------------------------------------------

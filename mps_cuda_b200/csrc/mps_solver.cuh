@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -406,7 +407,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     double *mx0 = nullptr, *mn0 = nullptr;  // reference state of the moving walls
     WallMotion* d_motion = nullptr;
     WallMotion hmot[2] = {};
-    bool motion_on = false;
+    bool motion_on = false, walls_moved = false;
     // mirrors: raw list U and two sorted generations
     MirrorBuf<R> U, M1, M2;
     int *mcs1, *mcs2;
@@ -648,6 +649,11 @@ template <class R, class RN> class Solver final : public SolverBase {
                                                                  d_wall_ids, nW, tw_pos, tw_vel,
                                                                  tw_nrm, tw_id, tw_typ);
             KL();
+            const std::vector<int> cls = wall_classes(nrm);
+            CK(cudaMemcpyAsync(key, cls.data(), sizeof(int) * nW, cudaMemcpyHostToDevice, stream));
+            k_wall_class<R><<<blocks(nW, 256), 256, 0, stream>>>(nW, tw_pos, key);
+            KL();
+            CK(cudaStreamSynchronize(stream));  // cls leaves scope
             bin_walls();
         } else {
             CK(cudaMemsetAsync(wcs, 0, sizeof(int) * (L() + 1), stream));
@@ -765,6 +771,32 @@ template <class R, class RN> class Solver final : public SolverBase {
         near_m1 = ar.template get<int8_t>(L());
         near_m2 = ar.template get<int8_t>(L());
         nbcnt = ar.template get<int>(F);
+    }
+
+    // A number per wall (load order), the same for walls whose normals compare equal. Walls come
+    // face by face, so most have the number of the wall before them.
+    std::vector<int> wall_classes(const R* nrm) const {
+        std::vector<int> cls(wall_ids.size());
+        std::map<std::array<R, 3>, int> known;
+        std::array<R, 3> last{};
+        int next = 0, last_cls = -1;
+        for (size_t w = 0; w < wall_ids.size(); ++w) {
+            const size_t id = wall_ids[w];
+            // + 0: a negative zero equals a positive one
+            const std::array<R, 3> n{nrm[id] + R(0), nrm[nT + id] + R(0), nrm[2 * size_t(nT) + id] + R(0)};
+            if (!(n[0] == n[0] && n[1] == n[1] && n[2] == n[2])) {
+                cls[w] = next++;  // a NaN equals nothing
+                continue;
+            }
+            if (last_cls < 0 || n != last) {
+                const auto at = known.insert({n, next});
+                if (at.second) ++next;
+                last = n;
+                last_cls = at.first->second;
+            }
+            cls[w] = last_cls;
+        }
+        return cls;
     }
 
     // ---- bucket build ------------------------------------------------------------------
@@ -947,16 +979,22 @@ template <class R, class RN> class Solver final : public SolverBase {
             k_pass_c<R, RN, D, TAPE><<<blocks(nF, bc), bc, 0, stream>>>(a);
         KL();
     }
-    // GenMRR_nonslip into the raw list, then the cull
-    template <bool D, bool TAPE>
-    void run_gen(const PassArgs<R, RN>& a, int bg, const V4<R>* pos, const R* prs, const int8_t* typ) {
+    template <bool D, bool TAPE, bool CLS>
+    void launch_gen(const PassArgs<R, RN>& a, int bg, const V4<R>* pos, const R* prs, const int8_t* typ) {
         const int g = group_lanes(kGroupMostGen);
         if (g == 32)
-            k_gen_cull_g<R, RN, D, TAPE, 32><<<group_grid(32), 128, 0, stream>>>(a, pos, prs, typ);
+            k_gen_cull_g<R, RN, D, TAPE, CLS, 32><<<group_grid(32), 128, 0, stream>>>(a, pos, prs, typ);
         else if (g == 8)
-            k_gen_cull_g<R, RN, D, TAPE, 8><<<group_grid(8), 128, 0, stream>>>(a, pos, prs, typ);
+            k_gen_cull_g<R, RN, D, TAPE, CLS, 8><<<group_grid(8), 128, 0, stream>>>(a, pos, prs, typ);
         else
-            k_gen_cull<R, RN, D, TAPE><<<blocks(nF, bg), bg, 0, stream>>>(a, pos, prs, typ);
+            k_gen_cull<R, RN, D, TAPE, CLS><<<blocks(nF, bg), bg, 0, stream>>>(a, pos, prs, typ);
+    }
+    // GenMRR_nonslip into the raw list, then the cull. Once walls have moved they carry no classes:
+    // their normals are compared.
+    template <bool D, bool TAPE>
+    void run_gen(const PassArgs<R, RN>& a, int bg, const V4<R>* pos, const R* prs, const int8_t* typ) {
+        if (walls_moved) launch_gen<D, TAPE, false>(a, bg, pos, prs, typ);
+        else launch_gen<D, TAPE, true>(a, bg, pos, prs, typ);
         KL();
         cull_raw();
     }
@@ -969,6 +1007,8 @@ template <class R, class RN> class Solver final : public SolverBase {
         bin(ks, g, nullptr, nW, wcs, L());
         k_surface_edge<R, RN><<<blocks(nW, 128), 128, 0, stream>>>(d_sc, nscene, nW, wall_view(),
                                                                    w_id, w_se);
+        KL();
+        k_wall_code<R><<<blocks(nW, 256), 256, 0, stream>>>(nW, w_pos, w_se);
         KL();
         near_wall_flags();
     }
@@ -1016,6 +1056,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         CK(cudaMemcpyAsync(d_motion, hmot, sizeof(hmot), cudaMemcpyHostToDevice, stream));
         CK(cudaStreamSynchronize(stream));
         motion_on = nW > 0 && (hmot[0].type != 0 || hmot[1].type != 0);
+        walls_moved = walls_moved || motion_on;
         invalidate_graph();
     }
 

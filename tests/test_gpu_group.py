@@ -109,3 +109,58 @@ def test_nearly_coincident_particles_equal_the_oracle(shift):
     finally:
         g.close()
         o.close()
+
+
+@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13)])
+def test_walls_that_moved_and_stopped_equal_the_oracle(block):
+    """Walls at rest are told apart by class; a wall that has moved is not, nor once it stops."""
+    l0 = 0.02
+    tank = tuple(b + 4 for b in block)
+    d = SceneDesc(l0, tuple(t * l0 for t in tank), block, seed=5, vel_sigma=0.3)
+    sc = dambreak(d)
+    yy, zz = np.meshgrid((np.arange(tank[1]) + 0.5) * l0, (np.arange(block[2]) + 0.5) * l0)
+    plate = np.stack([np.full(yy.size, (block[0] + 0.7) * l0), yy.ravel(), zz.ravel()])
+    side = np.tile([[-1.0], [0.0], [0.0]], (1, yy.size))
+    typ = np.concatenate([sc["typ"], np.full(yy.size, L.OBJ, np.int8)])
+    args = [typ, *(np.concatenate(v, 1).astype(np.float32) for v in (
+        (sc["pos"], plate), (sc["vel"], np.zeros_like(plate)), (sc["nrm"], side)))]
+    p = dambreak_params(d, dt=2e-4, precision=F32)
+    g, o = MPS(p, *args), Oracle(params_from(p), *args)
+    try:
+        _steps(g, o, 2, "before")
+        for omega, vx in ((3.0, -0.5), (0.0, 0.0)):
+            for h in (g, o):
+                h.set_wall_motion(L.OBJ, ((block[0] + 0.7) * l0, 0.1, 0.1), (0.0, 0.0, 1.0), omega,
+                                  (vx, 0.0, 0.0))
+            _steps(g, o, 4, (omega, vx))
+    finally:
+        g.close()
+        o.close()
+
+
+@pytest.mark.parametrize("prec", [F32, F64])
+@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13)])
+def test_many_wall_normals_equal_the_oracle(block, prec):
+    """A rough plate: 14 normals within reach of a particle, more than a particle registers."""
+    l0 = 0.02
+    tank = tuple(b + 4 for b in block)
+    d = SceneDesc(l0, tuple(t * l0 for t in tank), block, seed=5, vel_sigma=0.3)
+    sc = dambreak(d)
+    yy, zz = np.meshgrid((np.arange(tank[1]) + 0.5) * l0, (np.arange(block[2]) + 0.5) * l0)
+    plate = np.stack([np.full(yy.size, (block[0] + 0.7) * l0), yy.ravel(), zz.ravel()])
+    tilt = np.random.default_rng(2).uniform(-0.2, 0.2, (14, 2))
+    side = np.stack([-np.ones(14), tilt[:, 0], tilt[:, 1]])
+    side = (side / np.linalg.norm(side, axis=0))[:, np.arange(yy.size) % 14]
+    real = np.float64 if prec == F64 else np.float32
+    typ = np.concatenate([sc["typ"], np.full(yy.size, L.OBJ, np.int8)])
+    args = [typ, *(np.concatenate(v, 1).astype(real) for v in (
+        (sc["pos"], plate), (sc["vel"], np.zeros_like(plate)), (sc["nrm"], side)))]
+    p = dambreak_params(d, dt=2e-4, precision=prec)
+    g, o = MPS(p, *args), Oracle(params_from(p), *args)
+    try:
+        _steps(g, o, 3, block)
+        a, b = g.mirrors(2), o.mirrors()
+        assert np.array_equal(a["slot"], b["slot"]) and np.array_equal(a["pos"], b["pos"])
+    finally:
+        g.close()
+        o.close()
