@@ -324,7 +324,7 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const int* _
 // loads, and the counts cleared as they are read, so that the next bucket build starts from
 // zeros without a memset.
 
-__device__ __forceinline__ void load16(const int* __restrict__ in, int base, int L, int v[16]) {
+__device__ __forceinline__ void load16(const int* in, int base, int L, int v[16]) {
     if (base + 16 <= L) {
         const int4* p = reinterpret_cast<const int4*>(in + base);
 #pragma unroll
@@ -685,6 +685,169 @@ __global__ void __launch_bounds__(T) k_fine_rows_write(FineRows f,
 }
 
 // ---------------------------------------------------------------------------------------
+// whole bucket builds in one launch, for small scenes
+// ---------------------------------------------------------------------------------------
+// A build of a few thousand items is five or six launches of a few microseconds each, most of it
+// launch and drain. One cluster of eight blocks runs all of its phases instead, with cluster
+// barriers between them. What one block writes and another reads goes through global memory with
+// plain loads: __ldg may not see writes of the running kernel. The figures stand with the rule
+// (Solver::small_fluid).
+constexpr int kSmallBlocks = 8, kSmallThreads = 512, kSmallAll = kSmallBlocks * kSmallThreads;
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// exclusive scan of count[0, L) into out[0, L], the counts left zero, by the whole cluster; block
+// b's part of the table follows those of the blocks before it, sixteen counts a thread at a time.
+// part: kSmallBlocks ints of global memory.
+__device__ __forceinline__ void small_scan(int* count, int* out, int L, int* part) {
+    __shared__ int sh[32];
+    const int b = blockIdx.x, per = ((L + kSmallBlocks - 1) / kSmallBlocks + 15) / 16 * 16;
+    const int lo = min(L, b * per), hi = min(L, lo + per);
+    int sum = 0;
+    for (int i = lo + 16 * threadIdx.x; i < hi; i += 16 * kSmallThreads) {
+        int v[16];
+        load16(count, i, hi, v);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) sum += v[k];
+    }
+    sum = block_sum(sum, sh);
+    if (threadIdx.x == 0) part[b] = sum;
+    cluster_sync();
+    int run = 0;
+    for (int k = 0; k < b; ++k) run += part[k];
+    for (int i0 = lo; i0 < hi; i0 += 16 * kSmallThreads) {
+        const int i = i0 + 16 * int(threadIdx.x);
+        int v[16], mine[1] = {0}, tot[1];
+        if (i < hi) {
+            load16(count, i, hi, v);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) mine[0] += v[k];
+        }
+        block_exscan<1>(mine, tot, sh);
+        if (i < hi) {
+            int e = run + mine[0];
+            if (i + 16 <= hi) {
+                int4* o4 = reinterpret_cast<int4*>(out + i);
+                int4* c4 = reinterpret_cast<int4*>(count + i);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    int4 x;
+                    x.x = e; x.y = x.x + v[4 * k]; x.z = x.y + v[4 * k + 1]; x.w = x.z + v[4 * k + 2];
+                    e = x.w + v[4 * k + 3];
+                    o4[k] = x;
+                    c4[k] = make_int4(0, 0, 0, 0);
+                }
+            } else {
+                for (int k = 0; i + k < hi; ++k) {
+                    out[i + k] = e;
+                    e += v[k];
+                    count[i + k] = 0;
+                }
+            }
+        }
+        run += tot[0];
+    }
+    if (hi == L && lo < L && threadIdx.x == 0) out[L] = run;
+}
+
+// near flag of bucket b of a scene from the bucket table cs
+template <class R, class RN>
+__device__ __forceinline__ int8_t near_bucket(const SceneDev<R, RN>& sc, const int* cs, int b) {
+    const int iz = b / sc.nbxy, iy = (b % sc.nbxy) / sc.nbx, ix = b % sc.nbx;
+    // buckets on the grid border hold no particle: keep them conservative
+    if (ix < 1 || ix > sc.nbx - 2 || iy < 1 || iy > sc.nby - 2 || iz < 1 || iz > sc.nbz - 2) return 1;
+    int8_t f = 0;
+    for (int dz = -1; dz <= 1; ++dz)
+        for (int dy = -1; dy <= 1; ++dy) {
+            const int row = sc.cbase + (iz + dz) * sc.nbxy + (iy + dy) * sc.nbx;
+            if (cs[row + ix + 2] > cs[row + ix - 1]) f = 1;
+        }
+    return f;
+}
+
+// near flags (k_near_wall) by the whole cluster, from a table of this launch
+template <class R, class RN>
+__device__ __forceinline__ void small_near(const SceneDev<R, RN>* scs, int nscene, const int* cs,
+                                           int8_t* near) {
+    for (int s = 0; s < nscene; ++s) {
+        const SceneDev<R, RN>& sc = scs[s];
+        const int nb = sc.nbxy * sc.nbz;
+        for (int b = blockIdx.x * kSmallThreads + threadIdx.x; b < nb; b += kSmallAll)
+            near[sc.cbase + b] = near_bucket(sc, cs, b);
+    }
+}
+
+// mirror (or wall) build: bucket starts cs, items gathered by g, near flags
+template <class R, class RN, class Src, class G>
+__global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThreads)
+    k_bin_small(Src src, G g, const int* n_ptr, int n_fixed, int* key, int* rnk, int* seg, int* count,
+                int* cs, int L, int* part, const SceneDev<R, RN>* scs, int nscene, int8_t* near,
+                DevCounters* cnt) {
+    const int n = item_count(n_ptr, n_fixed), t0 = blockIdx.x * kSmallThreads + threadIdx.x;
+    for (int t = t0; t < n; t += kSmallAll) {
+        const int c = src.key(t, cnt);
+        key[t] = c;
+        rnk[t] = atomicAdd(&count[c], 1);
+    }
+    cluster_sync();
+    small_scan(count, cs, L, part);
+    cluster_sync();
+    for (int t = t0; t < n; t += kSmallAll) seg[cs[key[t]] + rnk[t]] = src.id(t);
+    if (near) small_near(scs, nscene, cs, near);
+    cluster_sync();
+    for (int t = t0; t < n; t += kSmallAll) {
+        const int c = key[t], lo = cs[c];
+        int d = rnk[t];  // order of unlisted items is irrelevant
+        if (c != L - 1) {
+            const int hi = cs[c + 1], my = src.id(t);
+            d = 0;
+            for (int k = lo; k < hi; ++k) d += seg[k] < my;
+        }
+        g(t, lo + d);
+    }
+}
+
+// fluid build: both start tables (cs bucket-major, csr row-major, each from its own counts), the
+// state gathered and the row-ordered copy written
+template <class R, class RN>
+__global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThreads)
+    k_fluid_small(FluidKeySrc<R, RN> src, FluidGather<R> g, int n, int* key, int* rnk, int* seg,
+                  int* count, int* count_r, int* cs, int* csr, int L, int* part, V4<R>* posf,
+                  DevCounters* cnt) {
+    const int t0 = blockIdx.x * kSmallThreads + threadIdx.x, dead = L - 1;
+    auto row = [&](int t, int c) {
+        if (c == dead) return dead;
+        return fine_rowmajor(src.sc[src.nscene > 1 ? scene_of(src.sc, src.nscene, src.pid[t]) : 0], c);
+    };
+    for (int t = t0; t < n; t += kSmallAll) {
+        const int c = src.key(t, cnt);
+        key[t] = c;
+        rnk[t] = atomicAdd(&count[c], 1);
+        atomicAdd(&count_r[row(t, c)], 1);
+    }
+    cluster_sync();
+    small_scan(count, cs, L, part);
+    small_scan(count_r, csr, L, part + kSmallBlocks);
+    cluster_sync();
+    for (int t = t0; t < n; t += kSmallAll) seg[cs[key[t]] + rnk[t]] = src.id(t);
+    cluster_sync();
+    for (int t = t0; t < n; t += kSmallAll) {
+        const int c = key[t], lo = cs[c];
+        int d = rnk[t];
+        if (c != dead) {
+            const int hi = cs[c + 1], my = src.id(t);
+            d = 0;
+            for (int k = lo; k < hi; ++k) d += seg[k] < my;
+            const V4<R> p = g.pos[t];
+            posf[csr[row(t, c)] + d] = V4<R>{p.x, p.y, p.z, slot_w(lo + d, R(0))};
+        }
+        g(t, lo + d);
+    }
+}
+
+// ---------------------------------------------------------------------------------------
 // neighbour passes
 // ---------------------------------------------------------------------------------------
 // Entry k of slot s's neighbour list, T slots sharing runs of 32-entry lines with E = 32 / T
@@ -768,23 +931,10 @@ template <class R, class RN> struct PassArgs {
 template <class R, class RN>
 __global__ void k_near_wall(const SceneDev<R, RN>* scs, int nscene, const int* __restrict__ wcs,
                             int8_t* near_wall) {
-    const int sidx = blockIdx.y;
-    const SceneDev<R, RN>& sc = scs[sidx];
+    const SceneDev<R, RN>& sc = scs[blockIdx.y];
     const int nb = sc.nbxy * sc.nbz;
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
-        const int iz = b / sc.nbxy, iy = (b % sc.nbxy) / sc.nbx, ix = b % sc.nbx;
-        int8_t f = 1;  // buckets on the grid border hold no particle: keep them conservative
-        if (ix >= 1 && ix <= sc.nbx - 2 && iy >= 1 && iy <= sc.nby - 2 && iz >= 1 &&
-            iz <= sc.nbz - 2) {
-            f = 0;
-            for (int dz = -1; dz <= 1; ++dz)
-                for (int dy = -1; dy <= 1; ++dy) {
-                    const int row = sc.cbase + (iz + dz) * sc.nbxy + (iy + dy) * sc.nbx;
-                    if (wcs[row + ix + 2] > wcs[row + ix - 1]) f = 1;
-                }
-        }
-        near_wall[sc.cbase + b] = f;
-    }
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x)
+        near_wall[sc.cbase + b] = near_bucket(sc, wcs, b);
 }
 
 template <class R, class RN>

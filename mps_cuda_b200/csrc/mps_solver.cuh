@@ -415,6 +415,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     // fluid positions in row-major fine-cell order (slot in w) and that order's cell starts
     V4<R>* posf;
     int *csr, *count_f;
+    int *count_r = nullptr, *small_part;  // small_fluid's row-major counts; block totals of both
     // the fluid build's start tables by bucket rows (k_fine_rows_*): per bucket row and per
     // fine row totals, then starts; per scene the bucket rows before it
     int *row_tot, *frow_tot, *row_scan;
@@ -684,6 +685,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         sbuf0 = S.pos;
         // the fluid's own count table: the start-table pass leaves it zero for the next build
         CK(cudaMemsetAsync(count_f, 0, sizeof(int) * size_t(LF()), stream));
+        CK(cudaMemsetAsync(count_r, 0, sizeof(int) * (small_fluid() ? size_t(LF()) : 1), stream));
         const size_t F = std::max(nF, 1);
         CK(cudaMemcpyAsync(row_scan, rs.data(), sizeof(int) * rs.size(), cudaMemcpyHostToDevice, stream));
         CK(cudaMemsetAsync(count, 0, sizeof(int) * L(), stream));
@@ -732,6 +734,8 @@ template <class R, class RN> class Solver final : public SolverBase {
         cs = ar.template get<int>(size_t(LF()) + 1);
         csr = ar.template get<int>(size_t(LF()) + 1);
         count_f = ar.template get<int>(size_t(LF()));
+        count_r = ar.template get<int>(small_fluid() ? size_t(LF()) : 1);
+        small_part = ar.template get<int>(4 * kSmallBlocks);
         row_scan = ar.template get<int>(size_t(nscene) + 1);
         row_tot = ar.template get<int>(size_t(nrows));
         frow_tot = ar.template get<int>(9 * size_t(nrows));
@@ -823,6 +827,15 @@ template <class R, class RN> class Solver final : public SolverBase {
         }
     }
 
+    // Builds in one launch (k_bin_small, k_fluid_small) for scenes of few particles and cells. us
+    // for a step's two fluid and two mirror builds, by launches / in one: 480 particles 61 + 53 /
+    // 42 + 31, 3 500 63 + 56 / 46 + 34, 8 200 68 + 56 / 64 + 42, mirrors of 48 000 61 / 70. A step of 480
+    // launched kernel by kernel 147 to 117 us, replayed 112 to 107; of 3 500 149 to 138, of 6 000 in
+    // FP64 200 to 206: beside other kernels a cluster waits for its eight blocks' places.
+    static constexpr int kSmallItems = 5000, kSmallCells = 131072;
+    bool small_fluid() const { return nF <= kSmallItems && LF() <= kSmallCells; }
+    bool small_mirrors() const { return nF <= kSmallItems && L() <= kSmallCells; }
+
     // fluid bucket build from (pos, vel, typ) sources into S2, then S <-> S2
     // The sorted state S2 is bucket-major in fine cells (start table cs); the same build
     // also writes the row-major copy posf (start table csr) that the neighbour walks read.
@@ -833,6 +846,16 @@ template <class R, class RN> class Solver final : public SolverBase {
         FluidGatherF<R, RN> g{{pos, vel, acc, prs, pav, pid, typ, S2.pos, S2.vel, S2.acc, S2.prs,
                                S2.pav, S2.pid, S2.typ},
                               d_sc, nscene, key_f, cs, csr, posf};
+        if (small_fluid()) {
+            k_fluid_small<R, RN><<<kSmallBlocks, kSmallThreads, 0, stream>>>(
+                ks, g.g, nF, key_f, rnk_f, seg_f, count_f, count_r, cs, csr, LF(),
+                small_part + 2 * kSmallBlocks, posf, cnt);
+            KL();
+            std::swap(S, S2);
+            ++swap_count;
+            posf_stale = false;
+            return;
+        }
         const int grid = std::min(blocks(std::max(nF, 1), 256), 148 * 32);
         if (nF > 0) {
             k_bin_key<FluidKeySrc<R, RN>><<<grid, 256, 0, stream>>>(ks, nullptr, nF, key_f, rnk_f,
@@ -874,8 +897,16 @@ template <class R, class RN> class Solver final : public SolverBase {
         Scope sc_(this, MPS_K_BIN_MIRROR);
         MirrorKeySrc<R, RN> ks{d_sc, nscene, dead(), U.pos, U.slot};
         MirrorGather<R> g{U.pos, U.slot, dst.pos, dst.slot};
+        int8_t* near = dcs == mcs1 ? near_m1 : (dcs == mcs2 ? near_m2 : nullptr);
+        if (small_mirrors()) {
+            k_bin_small<R, RN><<<kSmallBlocks, kSmallThreads, 0, stream>>>(
+                ks, g, &cnt->mirror_raw, cap, key, rnk, seg, count, dcs, L(), small_part, d_sc, nscene,
+                near, cnt);
+            KL();
+            return;
+        }
         bin(ks, g, &cnt->mirror_raw, cap, dcs, L());
-        if (dcs == mcs1 || dcs == mcs2) near_flags(dcs, dcs == mcs1 ? near_m1 : near_m2);
+        if (near) near_flags(dcs, near);
     }
 
     WallView<R> wall_view() const { return WallView<R>{wcs, w_pos, w_nrm, w_vel, w_se, w_typ}; }
