@@ -30,7 +30,7 @@ constexpr unsigned kFull = 0xffffffffu;
 
 // one warp's scratch
 template <class T, int P, int NT> struct GroupMem {
-    static constexpr int kWindow = sizeof(T) == 8 ? 384 : 512;  // candidates listed at a time
+    static constexpr int kWindow = 384;  // candidates listed at a time
     alignas(16) T term[NT][P][kGroupPitch];
     alignas(16) int kidx[kWindow];   // table index of each listed candidate, then zeros
     unsigned short hit[P][kWindow];  // accepted candidates' places in kidx

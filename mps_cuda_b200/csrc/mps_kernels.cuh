@@ -1658,6 +1658,94 @@ __global__ void __launch_bounds__(128, pass_c_blocks<R>(ALT, CORR))
     pass_c_finish<R, RN, DIAG, TAPE>(a, sc, s, pid, p, pi, g, cf, cm);
 }
 
+// one method of the reference for one FLD slot (mps_phase), one thread
+template <class R, class RN, bool DIAG>
+__device__ __forceinline__ void ph_vsc_one(const PassArgs<R, RN>& a, int s) {
+    const int pid = a.pid[s];
+    const SceneDev<R, RN>& sc = scene_ref(a, pid);
+    V4<R> p = ldg4(a.pos + s), v = ldg4(a.vel + s);
+    int ix, iy, iz;
+    cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
+    RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
+    R sx = 0, sy = 0, sz = 0;
+    int cf = 0, cm = 0;
+    visc_sum(sc, c, s, p.x, p.y, p.z, v.x, v.y, v.z, a.csr, a.posf, a.vel, a.m,
+             MPS_INF_SKIP(a, sc.skip_r), sx, sy, sz, cf, cm);
+    a.acc[s] = V4<R>{fmaR(sc.kn, sx, sc.g[0]), fmaR(sc.kn, sy, sc.g[1]), fmaR(sc.kn, sz, sc.g[2]),
+                     R(0)};
+    if (DIAG) {
+        int32_t* d = a.diag + size_t(pid) * kDiagCols;
+        d[DG_VSC_F] = cf;
+        d[DG_VSC_M] = cm;
+    }
+}
+
+template <class R, class RN, bool DIAG>
+__device__ __forceinline__ void ph_col_one(const PassArgs<R, RN>& a, int s) {
+    const int pid = a.pid[s];
+    const SceneDev<R, RN>& sc = scene_ref(a, pid);
+    V4<R> p = ldg4(a.pos + s), v = ldg4(a.vel + s);
+    int ix, iy, iz;
+    cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
+    RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
+    R wx = v.x, wy = v.y, wz = v.z;
+    RN ni = 0;
+    int cnt5[5] = {0, 0, 0, 0, 0};
+    col_dens_sum<R, RN, true, false>(sc, c, s, p.x, p.y, p.z, v.x, v.y, v.z, a.csr, a.posf, a.vel,
+                                     a.wl, a.m, a.skip != 0, wx, wy, wz, ni, cnt5);
+    a.tvel[s] = V4<R>{wx, wy, wz, R(0)};
+    if (DIAG) {
+        int32_t* d = a.diag + size_t(pid) * kDiagCols;
+        d[DG_COL_F] = cnt5[0];
+        d[DG_COL_W] = cnt5[1];
+        d[DG_COL_M] = cnt5[2];
+    }
+}
+
+template <class R, class RN, bool DIAG>
+__device__ __forceinline__ void ph_prs_one(const PassArgs<R, RN>& a, int s) {
+    const int pid = a.pid[s];
+    const SceneDev<R, RN>& sc = scene_ref(a, pid);
+    V4<R> p = ldg4(a.pos + s);
+    int ix, iy, iz;
+    cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
+    RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
+    R wx = 0, wy = 0, wz = 0;
+    RN ni = 0;
+    int cnt5[5] = {0, 0, 0, 0, 0};
+    col_dens_sum<R, RN, false, true>(sc, c, s, p.x, p.y, p.z, R(0), R(0), R(0), a.csr, a.posf,
+                                     a.vel, a.wl, a.m, a.skip != 0, wx, wy, wz, ni, cnt5);
+    a.prs[s] = eos(sc, ni);
+    if (DIAG) {
+        int32_t* d = a.diag + size_t(pid) * kDiagCols;
+        d[DG_PRS_F] = cnt5[3];
+        d[DG_PRS_M] = cnt5[4];
+        a.ndens[pid] = ni;
+    }
+}
+
+template <class R, class RN, bool DIAG, bool CORR>
+__device__ __forceinline__ void ph_grd_one(const PassArgs<R, RN>& a, int s) {
+    using G = typename std::conditional<CORR, GradCorr<R>, GradPlain<R>>::type;
+    const int pid = a.pid[s];
+    const SceneDev<R, RN>& sc = scene_ref(a, pid);
+    V4<R> p = ldg4(a.pos + s);
+    int ix, iy, iz;
+    cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
+    RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
+    G g;
+    int cf = 0, cm = 0;
+    grad_sum(sc, c, s, pid - sc.pbase, p.x, p.y, p.z, a.prs[s], a.csr, a.posf, a.prs, a.m,
+             a.skip != 0, g, cf, cm);
+    R ax, ay, az;
+    if (grad_acc(sc, g, ax, ay, az)) a.acc[s] = V4<R>{ax, ay, az, R(0)};  // else d_Acc stays
+    if (DIAG) {
+        int32_t* d = a.diag + size_t(pid) * kDiagCols;
+        d[DG_GRD_F] = cf;
+        d[DG_GRD_M] = cm;
+    }
+}
+
 // ---------------------------------------------------------------------------------------
 // neighbour passes with a group of G lanes per particle (mps_group.cuh): small scenes
 // ---------------------------------------------------------------------------------------
@@ -1703,23 +1791,31 @@ __device__ __forceinline__ const SceneDev<R, RN>& group_scene(const PassArgs<R, 
     return a.sc[__shfl_sync(kFull, int(mine - a.sc), __ffs(t.lanes) - 1)];
 }
 
-template <class R, class RN, bool DIAG, bool TAPE>
+template <class R, class RN, bool DIAG, bool TAPE, bool PHASE>
 __device__ __noinline__ void pass_a_single(const PassArgs<R, RN>& a, int s) {
-    pass_a_walk<R, RN, DIAG, TAPE, 2>(a, s);
+    if constexpr (PHASE) ph_vsc_one<R, RN, false>(a, s);
+    else pass_a_walk<R, RN, DIAG, TAPE, 2>(a, s);
 }
 
-// pass A, G lanes per particle
-template <class R, class RN, bool DIAG, bool TAPE, int G>
+// whether slot s takes part: FLD in a method of its own, listed in a pass
+template <bool PHASE, class R, class RN>
+__device__ __forceinline__ bool group_act(const PassArgs<R, RN>& a, int s) {
+    if (s >= a.nF) return false;
+    return PHASE ? a.typ[s] == kFLD : s < __ldg(a.cs + a.dead);
+}
+
+// pass A, G lanes per particle; PHASE: VscTrm alone, its acceleration
+template <class R, class RN, bool DIAG, bool TAPE, int G, bool PHASE = false>
 __global__ void __launch_bounds__(128) k_pass_a_g(const __grid_constant__ PassArgs<R, RN> a) {
     using Mem = GroupMem<R, 32 / G, 4>;
     __shared__ Mem mem[4];
     Mem& m = mem[threadIdx.x >> 5];
     const Group<G> gr;
     const int s = group_slot<R, RN>(gr);
-    bool act = s < a.nF && s < __ldg(a.cs + a.dead);
-    if (s < a.nF && !act && gr.l == 0) pass_a_unlisted(a, s, TAPE);
+    bool act = group_act<PHASE>(a, s);
+    if (!PHASE && s < a.nF && !act && gr.l == 0) pass_a_unlisted(a, s, TAPE);
     if (act && group_off(a, s)) {
-        if (gr.l == 0) pass_a_single<R, RN, DIAG, TAPE>(a, s);
+        if (gr.l == 0) pass_a_single<R, RN, DIAG, TAPE, PHASE>(a, s);
         act = false;
     }
     unsigned pend = __ballot_sync(kFull, act);
@@ -1783,7 +1879,11 @@ __global__ void __launch_bounds__(128) k_pass_a_g(const __grid_constant__ PassAr
         }
     }
     const R sx = gr.from(sum, 0), sy = gr.from(sum, 1), sz = gr.from(sum, 2);
-    if (act && gr.l == 0) pass_a_finish<R, RN, DIAG, TAPE>(a, sc, s, me.pid, p, v, sx, sy, sz, cf, cm);
+    if (!act || gr.l != 0) return;
+    if (PHASE)
+        a.acc[s] = V4<R>{fmaR(sc.kn, sx, sc.g[0]), fmaR(sc.kn, sy, sc.g[1]), fmaR(sc.kn, sz, sc.g[2]), R(0)};
+    else
+        pass_a_finish<R, RN, DIAG, TAPE>(a, sc, s, me.pid, p, v, sx, sy, sz, cf, cm);
 }
 
 // scratch of pass B: also MkPrs's terms, in its own arithmetic
@@ -1853,26 +1953,30 @@ __device__ __forceinline__ void group_col_dens(GroupMemB<R, RN, 32 / G>& m, cons
     }
 }
 
-template <class R, class RN, bool DIAG>
+// pass B whole, or one of its methods
+enum { PASS_B = 0, PASS_COL = 1, PASS_PRS = 2 };
+template <class R, class RN, bool DIAG, int MODE>
 __device__ __noinline__ void pass_b_single(const PassArgs<R, RN>& a, int s) {
-    pass_b_walk<R, RN, DIAG, kListGroup>(a, s);
+    if constexpr (MODE == PASS_COL) ph_col_one<R, RN, false>(a, s);
+    else if constexpr (MODE == PASS_PRS) ph_prs_one<R, RN, false>(a, s);
+    else pass_b_walk<R, RN, DIAG, kListGroup>(a, s);
 }
 
-// pass B, G lanes per particle
-template <class R, class RN, bool DIAG, int G>
+// pass B, G lanes per particle; MODE PASS_COL: ChkCol alone, PASS_PRS: MkPrs alone
+template <class R, class RN, bool DIAG, int G, int MODE = PASS_B>
 __global__ void __launch_bounds__(128) k_pass_b_g(const __grid_constant__ PassArgs<R, RN> a) {
     using Mem = GroupMemB<R, RN, 32 / G>;
     __shared__ Mem mem[4];
     Mem& m = mem[threadIdx.x >> 5];
     const Group<G> gr;
     const int s = group_slot<R, RN>(gr);
-    bool act = s < a.nF && s < __ldg(a.cs + a.dead);
-    if (s < a.nF && !act && gr.l == 0) {
+    bool act = group_act<MODE != PASS_B>(a, s);
+    if (MODE == PASS_B && s < a.nF && !act && gr.l == 0) {
         a.tvel[s] = a.vel[s];
         a.tprs[s] = R(0);
     }
     if (act && group_off(a, s)) {
-        if (gr.l == 0) pass_b_single<R, RN, DIAG>(a, s);
+        if (gr.l == 0) pass_b_single<R, RN, DIAG, MODE>(a, s);
         act = false;
     }
     unsigned pend = __ballot_sync(kFull, act);
@@ -1881,7 +1985,7 @@ __global__ void __launch_bounds__(128) k_pass_b_g(const __grid_constant__ PassAr
     const SceneDev<R, RN>& sc = *me.sc;
     const V4<R> p = me.p, v = act ? ldg4(a.vel + s) : p;
     const bool nearm = act && near_flag(a.near_m, sc, me.c),
-               nearw = act && near_flag(a.near_wall, sc, me.c);
+               nearw = MODE != PASS_PRS && act && near_flag(a.near_wall, sc, me.c);
     if (DIAG) {
         int ncand = 0;
         if (act && gr.l == 0)
@@ -1897,7 +2001,8 @@ __global__ void __launch_bounds__(128) k_pass_b_g(const __grid_constant__ PassAr
         pend &= ~t.lanes;
         const bool in = (t.lanes >> gr.lane) & 1u;
         const SceneDev<R, RN>& ts = group_scene(a, me.sc, t);
-        const R B = MPS_INF_SKIP(a, ts.skip_rc), thr = ts.list_thr, hi = ts.pair_hi;
+        const R B = MPS_INF_SKIP(a, MODE == PASS_COL ? ts.skip_rl : (MODE == PASS_PRS ? ts.skip_rp : ts.skip_rc));
+        const R thr = MODE == PASS_PRS ? ts.rp_lt : ts.list_thr, hi = ts.pair_hi;
         const GroupPts<R, 32 / G> pts(gr, p, s, t.lanes);
         const bool walls = __any_sync(kFull, in && nearw), mirrors = __any_sync(kFull, in && nearm);
         // the fluid, the walls (collision only), the mirrors (at rest, kernel.cu:834-836)
@@ -1905,7 +2010,7 @@ __global__ void __launch_bounds__(128) k_pass_b_g(const __grid_constant__ PassAr
         for (int kind = 0; kind < 3; ++kind) {
             if ((kind == 1 && !walls) || (kind == 2 && !mirrors)) continue;
             const V4<R>* table = kind == 0 ? a.posf : (kind == 1 ? a.wl.pos : a.m.pos);
-            const R rcol2 = kind == 1 ? ts.rlimw2 : ts.rlim2;
+            const R rcol2 = kind == 1 ? ts.rlimw2 : (MODE == PASS_PRS ? R(-1) : ts.rlim2);
             int nrow, total;
             if (kind == 0)
                 group_fluid_rows(m, ts, a.csr, t, B, nrow, total);
@@ -1917,15 +2022,15 @@ __global__ void __launch_bounds__(128) k_pass_b_g(const __grid_constant__ PassAr
                 const int nl = group_list<G>(m, nrow, total, w0);
                 const int n = group_test(m, gr, table, nl, [&](int i, const V4<R>& q) {
                     const R d2 = pts.d2(i, q);
-                    bool ok = pts.on(i) && (kind == 1 ? d2 < rcol2 : d2 <= thr) &&
+                    bool ok = pts.on(i) && (kind == 1 || MODE == PASS_COL ? d2 < rcol2 : d2 <= thr) &&
                               (kind != 0 || w_slot(q.w) != pts.s[i]);
                     if (ok && d2 > hi)
                         ok = bucket_adjacent(ts, pts.x[i], pts.y[i], pts.z[i], q.x, q.y, q.z);
                     return ok;
                 });
-                group_col_dens<DIAG>(m, gr, sc, p, v, table, n, rcol2, kind != 1, sum, ni, ncol, nden,
+                group_col_dens<DIAG>(m, gr, sc, p, v, table, n, rcol2, MODE != PASS_COL && kind != 1, sum, ni, ncol, nden,
                                      [&](int h, int k, const V4<R>& q) {
-                                         if (kind == 0 && have + h < a.nbK)
+                                         if (MODE == PASS_B && kind == 0 && have + h < a.nbK)
                                              a.nb[list_at(s, have + h, a.nbK, kListGroup)] = w_slot(q.w);
                                      },
                                      [&](int k, const V4<R>& q) {
@@ -1952,7 +2057,12 @@ __global__ void __launch_bounds__(128) k_pass_b_g(const __grid_constant__ PassAr
         for (int i = 0; i < 5; ++i)
             for (int o = G / 2; o > 0; o >>= 1) cnt5[i] += __shfl_xor_sync(kFull, cnt5[i], o);
     }
-    if (act && gr.l == 0) {
+    if (!act || gr.l != 0) return;
+    if (MODE == PASS_COL) {
+        a.tvel[s] = V4<R>{wx, wy, wz, R(0)};
+    } else if (MODE == PASS_PRS) {
+        a.prs[s] = eos(sc, ni);
+    } else {
         a.nbcnt[s] = have;
         pass_b_store<R, RN, DIAG>(a, sc, s, me.pid, p, wx, wy, wz, ni, cnt5);
     }
@@ -2009,8 +2119,15 @@ template <class R, int G, bool CORR> struct GroupGrad {
     }
 };
 
-// pass C, G lanes per particle, over the lists that pass B left
-template <class R, class RN, bool DIAG, bool TAPE, bool CORR, int G>
+template <class R, class RN, bool DIAG, bool TAPE, bool CORR, bool PHASE, class GA>
+__device__ __noinline__ void pass_c_single(const PassArgs<R, RN>& a, int s) {
+    if constexpr (PHASE) ph_grd_one<R, RN, false, CORR>(a, s);
+    else pass_c_long<R, RN, DIAG, TAPE, GA>(a, s);
+}
+
+// pass C, G lanes per particle, over the lists that pass B left; PHASE: PrsGrdTrm alone, its
+// acceleration, over a walk of its own
+template <class R, class RN, bool DIAG, bool TAPE, bool CORR, int G, bool PHASE = false>
 __global__ void __launch_bounds__(128) k_pass_c_g(const __grid_constant__ PassArgs<R, RN> a) {
     using GA = typename std::conditional<CORR, GradCorr<R>, GradPlain<R>>::type;
     using Sums = GroupGrad<R, G, CORR>;
@@ -2019,15 +2136,15 @@ __global__ void __launch_bounds__(128) k_pass_c_g(const __grid_constant__ PassAr
     Mem& m = mem[threadIdx.x >> 5];
     const Group<G> gr;
     const int s = group_slot<R, RN>(gr);
-    bool act = s < a.nF && s < __ldg(a.cs + a.dead);
-    if (s < a.nF && !act && gr.l == 0) {
+    bool act = group_act<PHASE>(a, s);
+    if (!PHASE && s < a.nF && !act && gr.l == 0) {
         a.tpos[s] = a.pos[s];
         a.ttyp[s] = a.typ[s];
         if (TAPE) a.tape_pre[s] = V4<R>{R(0), R(0), R(0), R(kTapeDead)};
     }
-    const int n = act ? a.nbcnt[s] : 0;
+    const int n = !PHASE && act ? a.nbcnt[s] : 0;
     if (act && (n > a.nbK || group_off(a, s))) {  // the walk over the fine rows: any position
-        if (gr.l == 0) pass_c_long<R, RN, DIAG, TAPE, GA>(a, s);
+        if (gr.l == 0) pass_c_single<R, RN, DIAG, TAPE, CORR, PHASE, GA>(a, s);
         act = false;
     }
     unsigned pend = __ballot_sync(kFull, act);
@@ -2035,7 +2152,8 @@ __global__ void __launch_bounds__(128) k_pass_c_g(const __grid_constant__ PassAr
     const GroupSlot<R, RN> me = group_load(a, s, act, a.pos);
     const SceneDev<R, RN>& sc = *me.sc;
     const V4<R> p = me.p;
-    const R pi = act ? a.tprs[s] : R(0);
+    const R* __restrict__ prs = PHASE ? a.prs : a.tprs;
+    const R pi = act ? prs[s] : R(0);
     const int cnt = act ? n : 0, most = __reduce_max_sync(kFull, cnt);
     const int* __restrict__ nb = a.nb + list_at(s, 0, a.nbK, kListGroup);
     auto entry = [&](int h) { return __ldg(nb + 4 * (h & ~7) + (h & 7)); };
@@ -2043,29 +2161,70 @@ __global__ void __launch_bounds__(128) k_pass_c_g(const __grid_constant__ PassAr
     const bool inside = sc.list_thr < rp2;
     // P_min over the fluid neighbours inside rp (order-free), then the gradient in order
     R pmin = pi;
-    for (int h = gr.l; h < cnt; h += G) {
-        const int j = entry(h);
-        const R pj = __ldg(a.tprs + j);
-        if ((inside || pair_d2(ldg4(a.posp + j), p) < rp2) && pj < pmin) pmin = pj;
-    }
-    for (int o = G / 2; o > 0; o >>= 1) {
-        const R x = __shfl_xor_sync(kFull, pmin, o);
-        if (x < pmin) pmin = x;
-    }
     Sums sums;
     int cf = 0, cm = 0;
-    sums.add(m, gr, most, [&](int h, R(&d)[3], R& w, R& pd) {
-        if (h >= cnt) return;
-        const V4<R> q = ldg4(a.posp + entry(h));
-        const R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
-        const R d2 = dot3(dx, dy, dz, dx, dy, dz);
-        if (d2 < rp2) {
-            d[0] = dx; d[1] = dy; d[2] = dz;
-            w = grad_weight(sc, d2);
-            pd = q.w - pmin;
-            if (DIAG) ++cf;
+    auto least = [&] {  // over the group
+        for (int o = G / 2; o > 0; o >>= 1) {
+            const R x = __shfl_xor_sync(kFull, pmin, o);
+            if (x < pmin) pmin = x;
         }
-    });
+    };
+    if constexpr (!PHASE) {
+        for (int h = gr.l; h < cnt; h += G) {
+            const int j = entry(h);
+            const R pj = __ldg(prs + j);
+            if ((inside || pair_d2(ldg4(a.posp + j), p) < rp2) && pj < pmin) pmin = pj;
+        }
+        least();
+        sums.add(m, gr, most, [&](int h, R(&d)[3], R& w, R& pd) {
+            if (h >= cnt) return;
+            const V4<R> q = ldg4(a.posp + entry(h));
+            const R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+            const R d2 = dot3(dx, dy, dz, dx, dy, dz);
+            if (d2 < rp2) {
+                d[0] = dx; d[1] = dy; d[2] = dz;
+                w = grad_weight(sc, d2);
+                pd = q.w - pmin;
+                if (DIAG) ++cf;
+            }
+        });
+    } else {
+        for (unsigned rest = pend; rest;) {
+            const GroupSet t = group_next(rest, me.row, me.c);
+            rest &= ~t.lanes;
+            const SceneDev<R, RN>& ts = group_scene(a, me.sc, t);
+            const GroupPts<R, 32 / G> pts(gr, p, s, t.lanes);
+            int nrow, total, nf = 0;
+            group_fluid_rows(m, ts, a.csr, t, MPS_INF_SKIP(a, ts.skip_rp), nrow, total);
+            // all windows for P_min, then all of them for the gradient
+            for (int walk = 0; walk < 2; ++walk) {
+                for (int w0 = 0; w0 < total; w0 += Mem::kWindow) {
+                    if (walk == 0 || total > Mem::kWindow) {
+                        const int nl = group_list<G>(m, nrow, total, w0);
+                        nf = group_test(m, gr, a.posf, nl, [&](int i, const V4<R>& q) {
+                            return pts.on(i) && w_slot(q.w) != pts.s[i] && pts.d2(i, q) < ts.rp2;
+                        });
+                    }
+                    if (walk == 0) {
+                        for (int h = gr.l; h < nf; h += G) {
+                            const R pj = __ldg(prs + w_slot(ldg4(a.posf + m.kidx[m.hit[gr.g][h]]).w));
+                            if (pj < pmin) pmin = pj;
+                        }
+                        __syncwarp();
+                    } else {
+                        sums.add(m, gr, __reduce_max_sync(kFull, nf), [&](int h, R(&d)[3], R& w, R& pd) {
+                            if (h >= nf) return;
+                            const V4<R> q = ldg4(a.posf + m.kidx[m.hit[gr.g][h]]);
+                            d[0] = q.x - p.x; d[1] = q.y - p.y; d[2] = q.z - p.z;
+                            w = grad_weight(sc, dot3(d[0], d[1], d[2], d[0], d[1], d[2]));
+                            pd = __ldg(prs + w_slot(q.w)) - pmin;
+                        });
+                    }
+                }
+                if (walk == 0) least();
+            }
+        }
+    }
     const bool nearm = act && near_flag(a.near_m, sc, me.c);
     if (!__any_sync(kFull, nearm)) pend = 0u;
     const int skip_slot = me.pid - sc.pbase + kNumMRR * sc.pbase;  // kernel.cu:1759
@@ -2102,7 +2261,13 @@ __global__ void __launch_bounds__(128) k_pass_c_g(const __grid_constant__ PassAr
             cf += __shfl_xor_sync(kFull, cf, o);
             cm += __shfl_xor_sync(kFull, cm, o);
         }
-    if (act && gr.l == 0) pass_c_finish<R, RN, DIAG, TAPE>(a, sc, s, me.pid, p, pi, g, cf, cm);
+    if (!act || gr.l != 0) return;
+    if constexpr (PHASE) {
+        R ax, ay, az;
+        if (grad_acc(sc, g, ax, ay, az)) a.acc[s] = V4<R>{ax, ay, az, R(0)};  // else d_Acc stays
+    } else {
+        pass_c_finish<R, RN, DIAG, TAPE>(a, sc, s, me.pid, p, pi, g, cf, cm);
+    }
 }
 
 // ---- mirror generation with a group of lanes per particle ---------------------------------
@@ -2407,24 +2572,7 @@ __global__ void k_mirror_prs(const int* __restrict__ mcs, int dead, V4<R>* __res
 template <class R, class RN, bool DIAG>
 __global__ void __launch_bounds__(128) k_ph_vsc(const __grid_constant__ PassArgs<R, RN> a) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.nF || a.typ[s] != kFLD) return;
-    const int pid = a.pid[s];
-    const SceneDev<R, RN>& sc = scene_ref(a, pid);
-    V4<R> p = ldg4(a.pos + s), v = ldg4(a.vel + s);
-    int ix, iy, iz;
-    cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
-    RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
-    R sx = 0, sy = 0, sz = 0;
-    int cf = 0, cm = 0;
-    visc_sum(sc, c, s, p.x, p.y, p.z, v.x, v.y, v.z, a.csr, a.posf, a.vel, a.m,
-             MPS_INF_SKIP(a, sc.skip_r), sx, sy, sz, cf, cm);
-    a.acc[s] = V4<R>{fmaR(sc.kn, sx, sc.g[0]), fmaR(sc.kn, sy, sc.g[1]), fmaR(sc.kn, sz, sc.g[2]),
-                     R(0)};
-    if (DIAG) {
-        int32_t* d = a.diag + size_t(pid) * kDiagCols;
-        d[DG_VSC_F] = cf;
-        d[DG_VSC_M] = cm;
-    }
+    if (s < a.nF && a.typ[s] == kFLD) ph_vsc_one<R, RN, DIAG>(a, s);
 }
 
 template <class R, class RN>
@@ -2451,25 +2599,7 @@ __global__ void k_ph_uppcl1(const __grid_constant__ PassArgs<R, RN> a) {
 template <class R, class RN, bool DIAG>
 __global__ void __launch_bounds__(128) k_ph_col(const __grid_constant__ PassArgs<R, RN> a) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.nF || a.typ[s] != kFLD) return;
-    const int pid = a.pid[s];
-    const SceneDev<R, RN>& sc = scene_ref(a, pid);
-    V4<R> p = ldg4(a.pos + s), v = ldg4(a.vel + s);
-    int ix, iy, iz;
-    cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
-    RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
-    R wx = v.x, wy = v.y, wz = v.z;
-    RN ni = 0;
-    int cnt5[5] = {0, 0, 0, 0, 0};
-    col_dens_sum<R, RN, true, false>(sc, c, s, p.x, p.y, p.z, v.x, v.y, v.z, a.csr, a.posf, a.vel,
-                                     a.wl, a.m, a.skip != 0, wx, wy, wz, ni, cnt5);
-    a.tvel[s] = V4<R>{wx, wy, wz, R(0)};
-    if (DIAG) {
-        int32_t* d = a.diag + size_t(pid) * kDiagCols;
-        d[DG_COL_F] = cnt5[0];
-        d[DG_COL_W] = cnt5[1];
-        d[DG_COL_M] = cnt5[2];
-    }
+    if (s < a.nF && a.typ[s] == kFLD) ph_col_one<R, RN, DIAG>(a, s);
 }
 
 // d_UpChkCol (kernel.cu:1281-1287): Acc holds the corrected velocity, Vel = Acc
@@ -2485,49 +2615,13 @@ __global__ void k_ph_upchkcol(const __grid_constant__ PassArgs<R, RN> a) {
 template <class R, class RN, bool DIAG>
 __global__ void __launch_bounds__(128) k_ph_prs(const __grid_constant__ PassArgs<R, RN> a) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.nF || a.typ[s] != kFLD) return;
-    const int pid = a.pid[s];
-    const SceneDev<R, RN>& sc = scene_ref(a, pid);
-    V4<R> p = ldg4(a.pos + s);
-    int ix, iy, iz;
-    cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
-    RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
-    R wx = 0, wy = 0, wz = 0;
-    RN ni = 0;
-    int cnt5[5] = {0, 0, 0, 0, 0};
-    col_dens_sum<R, RN, false, true>(sc, c, s, p.x, p.y, p.z, R(0), R(0), R(0), a.csr, a.posf,
-                                     a.vel, a.wl, a.m, a.skip != 0, wx, wy, wz, ni, cnt5);
-    a.prs[s] = eos(sc, ni);
-    if (DIAG) {
-        int32_t* d = a.diag + size_t(pid) * kDiagCols;
-        d[DG_PRS_F] = cnt5[3];
-        d[DG_PRS_M] = cnt5[4];
-        a.ndens[pid] = ni;
-    }
+    if (s < a.nF && a.typ[s] == kFLD) ph_prs_one<R, RN, DIAG>(a, s);
 }
 
 template <class R, class RN, bool DIAG, bool CORR = false>
 __global__ void __launch_bounds__(128) k_ph_grd(const __grid_constant__ PassArgs<R, RN> a) {
-    using G = typename std::conditional<CORR, GradCorr<R>, GradPlain<R>>::type;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= a.nF || a.typ[s] != kFLD) return;
-    const int pid = a.pid[s];
-    const SceneDev<R, RN>& sc = scene_ref(a, pid);
-    V4<R> p = ldg4(a.pos + s);
-    int ix, iy, iz;
-    cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
-    RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
-    G g;
-    int cf = 0, cm = 0;
-    grad_sum(sc, c, s, pid - sc.pbase, p.x, p.y, p.z, a.prs[s], a.csr, a.posf, a.prs, a.m,
-             a.skip != 0, g, cf, cm);
-    R ax, ay, az;
-    if (grad_acc(sc, g, ax, ay, az)) a.acc[s] = V4<R>{ax, ay, az, R(0)};  // else d_Acc stays
-    if (DIAG) {
-        int32_t* d = a.diag + size_t(pid) * kDiagCols;
-        d[DG_GRD_F] = cf;
-        d[DG_GRD_M] = cm;
-    }
+    if (s < a.nF && a.typ[s] == kFLD) ph_grd_one<R, RN, DIAG, CORR>(a, s);
 }
 
 template <class R, class RN>
@@ -2555,31 +2649,6 @@ __global__ void k_ph_uppcl2(const __grid_constant__ PassArgs<R, RN> a) {
     } else {
         a.pav[s] = a.pav[s] + a.prs[s];
     }
-}
-
-// GenMRR_nonslip without the cull (the cull is MkBkt_MRR's d_MRRinout)
-template <class R, class RN, bool DIAG>
-__global__ void __launch_bounds__(128) k_ph_gen(const __grid_constant__ PassArgs<R, RN> a) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    MirrorPlan<R> pl;
-    pl.nreg = 0;
-    pl.corner = -1;
-    int m = 0, pid = 0;
-    V4<R> p{R(0), R(0), R(0), R(0)};
-    R P = R(0);
-    if (s < a.nF && a.typ[s] == kFLD) {  // every lane stays for the warp's reservation
-        pid = a.pid[s];
-        const SceneDev<R, RN>& sc = scene_ref(a, pid);
-        p = ldg4(a.pos + s);
-        int ix, iy, iz;
-        cell_of(sc, p.x, p.y, p.z, ix, iy, iz);
-        RowCtx<R> c = row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
-        const int nw = plan_mirrors(sc, c, p.x, p.y, p.z, a.wl, a.skip != 0, pl);
-        m = count_mirrors<R, RN>(pl, p.x, p.y, p.z, a.wl, a.cnt);
-        P = a.prs[s];
-        if (DIAG) a.diag[size_t(pid) * kDiagCols + DG_GEN_W] = nw;
-    }
-    gen_reserve_emit<R, RN, false>(a, pl, m, p.x, p.y, p.z, P, pid * kNumMRR);
 }
 
 // d_MRRinout (kernel.cu:932-985) over the raw mirrors; a culled mirror's slot becomes

@@ -1011,7 +1011,8 @@ template <class R, class RN> class Solver final : public SolverBase {
         KL();
     }
     template <bool D, bool TAPE, bool CLS>
-    void launch_gen(const PassArgs<R, RN>& a, int bg, const V4<R>* pos, const R* prs, const int8_t* typ) {
+    void launch_gen_cls(const PassArgs<R, RN>& a, int bg, const V4<R>* pos, const R* prs,
+                        const int8_t* typ) {
         const int g = group_lanes(kGroupMostGen);
         if (g == 32)
             k_gen_cull_g<R, RN, D, TAPE, CLS, 32><<<group_grid(32), 128, 0, stream>>>(a, pos, prs, typ);
@@ -1020,12 +1021,17 @@ template <class R, class RN> class Solver final : public SolverBase {
         else
             k_gen_cull<R, RN, D, TAPE, CLS><<<blocks(nF, bg), bg, 0, stream>>>(a, pos, prs, typ);
     }
-    // GenMRR_nonslip into the raw list, then the cull. Once walls have moved they carry no classes:
-    // their normals are compared.
+    // GenMRR_nonslip into the raw list. Once walls have moved they carry no classes: their normals
+    // are compared.
+    template <bool D, bool TAPE>
+    void launch_gen(const PassArgs<R, RN>& a, int bg, const V4<R>* pos, const R* prs, const int8_t* typ) {
+        if (walls_moved) launch_gen_cls<D, TAPE, false>(a, bg, pos, prs, typ);
+        else launch_gen_cls<D, TAPE, true>(a, bg, pos, prs, typ);
+    }
+    // ... then the cull
     template <bool D, bool TAPE>
     void run_gen(const PassArgs<R, RN>& a, int bg, const V4<R>* pos, const R* prs, const int8_t* typ) {
-        if (walls_moved) launch_gen<D, TAPE, false>(a, bg, pos, prs, typ);
-        else launch_gen<D, TAPE, true>(a, bg, pos, prs, typ);
+        launch_gen<D, TAPE>(a, bg, pos, prs, typ);
         KL();
         cull_raw();
     }
@@ -1440,10 +1446,22 @@ template <class R, class RN> class Solver final : public SolverBase {
         steps += n;
     }
 
+    template <bool CORR> void run_ph_grd(const PassArgs<R, RN>& a, int gb, int g) {
+        if (diag_on) k_ph_grd<R, RN, true, CORR><<<gb, block, 0, stream>>>(a);
+        else if (g == 32)
+            k_pass_c_g<R, RN, false, false, CORR, 32, true><<<group_grid(32), 128, 0, stream>>>(a);
+        else if (g == 8)
+            k_pass_c_g<R, RN, false, false, CORR, 8, true><<<group_grid(8), 128, 0, stream>>>(a);
+        else k_ph_grd<R, RN, false, CORR><<<gb, block, 0, stream>>>(a);
+    }
+
+    // One method. The group kernels find a particle's candidates in the rows of its current
+    // position, so they serve the methods while no particle has moved since the bucket build.
     void phase(int ph) override {
         finish_tail();
         PassArgs<R, RN> a = args(M1, mcs1);
         const int gb = blocks(nF, block);
+        auto lanes = [&](int most) { return sorted ? group_lanes(most) : 0; };
         auto need_lists = [&]() {
             if (!lists_valid)
                 throw ApiError(MPS_ERR_STATE, "bucket lists are not built: run MPS_PHASE_MKBKT first");
@@ -1470,8 +1488,8 @@ template <class R, class RN> class Solver final : public SolverBase {
                 reset_raw();
                 break;
             case MPS_PHASE_GENMRR_NONSLIP:
-                if (diag_on) k_ph_gen<R, RN, true><<<gb, block, 0, stream>>>(a);
-                else k_ph_gen<R, RN, false><<<gb, block, 0, stream>>>(a);
+                if (diag_on) launch_gen<true, false>(a, block, S.pos, S.prs, S.typ);
+                else launch_gen<false, false>(a, block, S.pos, S.prs, S.typ);
                 KL();
                 break;
             case MPS_PHASE_MKBKT_MRR:
@@ -1481,6 +1499,10 @@ template <class R, class RN> class Solver final : public SolverBase {
             case MPS_PHASE_VSCTRM:
                 need_lists();
                 if (diag_on) k_ph_vsc<R, RN, true><<<gb, block, 0, stream>>>(a);
+                else if (lanes(kGroupMostA) == 32)
+                    k_pass_a_g<R, RN, false, false, 32, true><<<group_grid(32), 128, 0, stream>>>(a);
+                else if (lanes(kGroupMostA) == 8)
+                    k_pass_a_g<R, RN, false, false, 8, true><<<group_grid(8), 128, 0, stream>>>(a);
                 else k_ph_vsc<R, RN, false><<<gb, block, 0, stream>>>(a);
                 KL();
                 acc_dirty = true;
@@ -1495,6 +1517,10 @@ template <class R, class RN> class Solver final : public SolverBase {
             case MPS_PHASE_CHKCOL:
                 need_lists();
                 if (diag_on) k_ph_col<R, RN, true><<<gb, block, 0, stream>>>(a);
+                else if (lanes(kGroupMostBC) == 32)
+                    k_pass_b_g<R, RN, false, 32, PASS_COL><<<group_grid(32), 128, 0, stream>>>(a);
+                else if (lanes(kGroupMostBC) == 8)
+                    k_pass_b_g<R, RN, false, 8, PASS_COL><<<group_grid(8), 128, 0, stream>>>(a);
                 else k_ph_col<R, RN, false><<<gb, block, 0, stream>>>(a);
                 KL();
                 k_ph_upchkcol<R, RN><<<gb, block, 0, stream>>>(a);
@@ -1504,18 +1530,17 @@ template <class R, class RN> class Solver final : public SolverBase {
             case MPS_PHASE_MKPRS:
                 need_lists();
                 if (diag_on) k_ph_prs<R, RN, true><<<gb, block, 0, stream>>>(a);
+                else if (lanes(kGroupMostBC) == 32)
+                    k_pass_b_g<R, RN, false, 32, PASS_PRS><<<group_grid(32), 128, 0, stream>>>(a);
+                else if (lanes(kGroupMostBC) == 8)
+                    k_pass_b_g<R, RN, false, 8, PASS_PRS><<<group_grid(8), 128, 0, stream>>>(a);
                 else k_ph_prs<R, RN, false><<<gb, block, 0, stream>>>(a);
                 KL();
                 break;
             case MPS_PHASE_PRSGRDTRM:
                 need_lists();
-                if (grad_mode == MPS_GRAD_CORRECTED) {
-                    if (diag_on) k_ph_grd<R, RN, true, true><<<gb, block, 0, stream>>>(a);
-                    else k_ph_grd<R, RN, false, true><<<gb, block, 0, stream>>>(a);
-                } else {
-                    if (diag_on) k_ph_grd<R, RN, true><<<gb, block, 0, stream>>>(a);
-                    else k_ph_grd<R, RN, false><<<gb, block, 0, stream>>>(a);
-                }
+                if (grad_mode == MPS_GRAD_CORRECTED) run_ph_grd<true>(a, gb, lanes(kGroupMostBC));
+                else run_ph_grd<false>(a, gb, lanes(kGroupMostBC));
                 KL();
                 acc_dirty = true;
                 break;

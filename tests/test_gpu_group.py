@@ -164,3 +164,29 @@ def test_many_wall_normals_equal_the_oracle(block, prec):
     finally:
         g.close()
         o.close()
+
+
+@pytest.mark.parametrize("corrected", [0, 1])
+@pytest.mark.parametrize("prec", [F32, F64, F32_N64])
+@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13)])
+def test_methods_one_by_one_equal_the_oracle(block, prec, corrected):
+    """Every method on its own, in the reference's order and then without the bucket builds that
+    follow a move: the lists are then older than the positions, and one thread walks them."""
+    tank = tuple(b + 3 for b in block)
+    g, o = _pair(block, tank, prec)
+    step = [0, 2, 3, 4, 5, 6, 0, 7, 0, 8, 2, 3, 4, 9, 10]
+    stale = [2, 3, 4, 5, 6, 7, 8, 2, 3, 4, 9, 10]
+    try:
+        if corrected:
+            g.set_option(L.OPT_GRADIENT, L.GRAD_CORRECTED)
+            o.set_gradient(1)
+        for phases in (step, step, [0] + stale):
+            for ph in phases:
+                g.phase(ph)
+                o.phase(ph)
+                a, b = g.state(), o.state()
+                for k in FIELDS + ("acc",):
+                    assert np.array_equal(a[k], b[k], equal_nan=k != "typ"), (ph, k)
+    finally:
+        g.close()
+        o.close()
