@@ -33,7 +33,13 @@ template <class R> __device__ __forceinline__ D3 d3v(const V4<R>& a) {
 __device__ __forceinline__ D3 operator+(D3 a, D3 b) { return D3{a.x + b.x, a.y + b.y, a.z + b.z}; }
 __device__ __forceinline__ D3 operator-(D3 a, D3 b) { return D3{a.x - b.x, a.y - b.y, a.z - b.z}; }
 __device__ __forceinline__ D3 operator*(double s, D3 a) { return D3{s * a.x, s * a.y, s * a.z}; }
-__device__ __forceinline__ double dot(D3 a, D3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+__device__ __forceinline__ double dot(D3 a, D3 b) {
+    return __fma_rn(a.z, b.z, __fma_rn(a.y, b.y, a.x * b.x));
+}
+// s a + b
+__device__ __forceinline__ D3 fma3(double s, D3 a, D3 b) {
+    return D3{__fma_rn(s, a.x, b.x), __fma_rn(s, a.y, b.y), __fma_rn(s, a.z, b.z)};
+}
 __device__ __forceinline__ V4<double> v4(D3 a) { return V4<double>{a.x, a.y, a.z, 0.0}; }
 __device__ __forceinline__ D3 d3d(const V4<double>& a) { return D3{a.x, a.y, a.z}; }
 __device__ __forceinline__ void atomic_add3(V4<double>* p, D3 a) {
@@ -90,38 +96,85 @@ __device__ __forceinline__ RowCtx<R> adj_row(const SceneDev<R, RN>& sc, const V4
     return row_ctx(sc, p.x, p.y, p.z, ix, iy, iz);
 }
 
+// The gathering kernels below (C1, C2, B2, A2) give a slot's list entries, walls and mirrors to
+// LANES neighbouring lanes (entry k to lane k mod LANES) and add up what the lanes hold. With one
+// thread per slot they were bound by latency: 3 of 16 warps per scheduler, each waiting for its
+// own chain of loads and FP64 arithmetic. The lanes put more entries in flight, the shared
+// reciprocals below shorten the chain, and six blocks per SM (80 registers) hide what is left. One
+// step's replay and adjoint, us (one thread before / 4 / 8 / 16 / 32 lanes):
+//     3.5k particles   844  / 530  / 427  / 353  / 293
+//     48k              1362 / 1086 / 1073 / 1016 / 1086
+//     192k             3074 / 2710 / 2818 / 2904 / 3475
+//     384k             6039 / 5471 / 5682 / 6057 / 7107
+constexpr int kAdjBlocks = 6;
+template <int LANES> struct AdjLanes {
+    int s, lane;
+    unsigned mask;
+    __device__ __forceinline__ AdjLanes() {
+        const int t = blockIdx.x * blockDim.x + threadIdx.x;
+        s = t / LANES;
+        lane = t % LANES;
+        mask = LANES == 32 ? 0xffffffffu : ((1u << LANES) - 1u) << (threadIdx.x & 31 & ~(LANES - 1));
+    }
+    __device__ __forceinline__ double sum(double v) const {
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+        return v;
+    }
+    __device__ __forceinline__ D3 sum(D3 v) const { return D3{sum(v.x), sum(v.y), sum(v.z)}; }
+    // f(j) for the rows' buckets around a particle (for_rows), dealt to the lanes row by row
+    template <class R, class RN, class F>
+    __device__ __forceinline__ void rows(const SceneDev<R, RN>& sc, const int* __restrict__ cs,
+                                         const RowCtx<R>& c, R B, F&& f) const {
+        for_rows_ranges(sc, cs, c, B, [&](int lo, int hi) {
+            for (int j = lo + lane; j < hi; j += LANES) f(j);
+        });
+    }
+};
+
 // C1: adjoint of UpPcl2 + ChkPcl for every slot; Pmin and its argmin over the list
-template <class R, class RN> __global__ void __launch_bounds__(128) k_adj_c1(AdjArgs<R, RN> a) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+template <class R, class RN, int LANES>
+__global__ void __launch_bounds__(128) k_adj_c1(AdjArgs<R, RN> a) {
+    const AdjLanes<LANES> ln;
+    const int s = ln.s;
     if (s >= a.nF) return;
     const SceneDev<R, RN>& sc = a.sc[0];
-    a.lP_at[s] = 0.0;
-    a.lx_at[s] = V4<double>{0, 0, 0, 0};
     const V4<R> pre = a.t.vp2[s];
     const int st = int(pre.w);
-    const int pid = a.t.pid2[s];
-    a.inv2[pid] = s;
-    const V4<double> zero{0, 0, 0, 0};
     R pm = R(0);
     int am = -1;
     if (st != kTapeDead) {
         const int n = a.t.nB[s];
         if (n > a.nbK) {
-            atomicAdd(a.err, 1);
+            if (ln.lane == 0) atomicAdd(a.err, 1);
         } else {
             const V4<R> p = a.t.x2[s];
             pm = a.t.P2[s];
-            for (int k = 0; k < n; ++k) {
+            int at = n;
+            for (int k = ln.lane; k < n; k += LANES) {
                 const int j = a.t.nbB[list_at(s, k, a.nbK, a.lt)];
                 const V4<R> q = ldg4(a.t.x2 + j);
                 R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
                 if (dot3(dx, dy, dz, dx, dy, dz) < sc.rp2) {
                     R pj = __ldg(a.t.P2 + j);
-                    if (pj < pm) { pm = pj; am = j; }
+                    if (pj < pm) { pm = pj; am = j; at = k; }
                 }
+            }
+            // the lowest pressure, of equal ones the first of the list
+#pragma unroll
+            for (int o = LANES / 2; o > 0; o >>= 1) {
+                const R po = __shfl_xor_sync(ln.mask, pm, o);
+                const int jo = __shfl_xor_sync(ln.mask, am, o), ko = __shfl_xor_sync(ln.mask, at, o);
+                if (po < pm || (po == pm && ko < at)) { pm = po; am = jo; at = ko; }
             }
         }
     }
+    if (ln.lane) return;
+    const int pid = a.t.pid2[s];
+    const V4<double> zero{0, 0, 0, 0};
+    a.lP_at[s] = 0.0;
+    a.lx_at[s] = zero;
+    a.inv2[pid] = s;
     a.pmin[s] = pm;
     a.am[s] = am;
     if (st == kTapeDead || st == kTapeDeleted) {
@@ -137,49 +190,82 @@ template <class R, class RN> __global__ void __launch_bounds__(128) k_adj_c1(Adj
     a.lxs[s] = v4(lxo);
 }
 
-// pressure-gradient pair factor f(d) = (rp/d - d/rp) / d^2 and (df/dd) / d
-__device__ __forceinline__ void grad_f(double d2, double rp, double& f, double& fp) {
-    double d = sqrt(d2);
-    f = (rp / d - d / rp) / d2;
-    fp = (-3.0 * rp / (d2 * d2) + 1.0 / (rp * d2)) / d;
+// Pair factors in double. From lo = SceneDev::pair_lo on, the quotients are mps_exact.cuh's: a
+// pair's five divisions share the reciprocals of d and d^2, and none branches.
+// 1 / b from y, which is a few last places off
+__device__ __forceinline__ double rcp_near(double b, double y) {
+    return __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+}
+// viscosity: w = 2 l0 / d^3 and 3 w / d^2
+__device__ __forceinline__ void visc_f(double d2, double two_l0, double lo, double& w, double& g) {
+    if (d2 >= lo) {
+        const double d = sqrt_in(d2), i2 = rcp_in(d2);
+        w = div_in(two_l0, d2 * d);
+        g = div_by(3.0 * w, d2, i2);
+    } else {
+        const double d = sqrt(d2);
+        w = two_l0 / (d2 * d);
+        g = 3.0 * w / d2;
+    }
+}
+// density: W'(d) / d of W = rp/d - d/rp (irp = 1 / rp)
+__device__ __forceinline__ double dens_f(double d2, double rp, double irp, double lo) {
+    if (d2 >= lo) return div_in(div_in(-rp, d2) - irp, sqrt_in(d2));
+    return (-rp / d2 - 1.0 / rp) / sqrt(d2);
+}
+// pressure gradient: f(d) = (rp/d - d/rp) / d^2 and (df/dd) / d
+__device__ __forceinline__ void grad_f(double d2, double rp, double irp, double lo, double& f,
+                                       double& fp) {
+    if (d2 >= lo) {
+        const double d = sqrt_in(d2), i1 = rcp_in(d), i2 = rcp_in(d2), d4 = d2 * d2, rd = rp * d2;
+        f = div_by(div_by(rp, d, i1) - div_by(d, rp, irp), d2, i2);
+        fp = div_by(div_by(-3.0 * rp, d4, rcp_near(d4, i2 * i2)) + rcp_near(rd, irp * i2), d, i1);
+    } else {
+        const double d = sqrt(d2);
+        f = (rp / d - d / rp) / d2;
+        fp = (-3.0 * rp / (d2 * d2) + 1.0 / (rp * d2)) / d;
+    }
 }
 
 // C2: adjoint of PrsGrdTrm, gathered per slot
-template <class R, class RN> __global__ void __launch_bounds__(128) k_adj_c2(AdjArgs<R, RN> a) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+template <class R, class RN, int LANES>
+__global__ void __launch_bounds__(128, kAdjBlocks) k_adj_c2(AdjArgs<R, RN> a) {
+    const AdjLanes<LANES> ln;
+    const int s = ln.s;
     if (s >= a.nF) return;
     const SceneDev<R, RN>& sc = a.sc[0];
     const int st = int(a.t.vp2[s].w);
     const int n = a.t.nB[s];
     if (st == kTapeDead || n > a.nbK) {
-        a.lP[s] = 0.0;
+        if (ln.lane == 0) a.lP[s] = 0.0;
         return;
     }
     const V4<R> p = a.t.x2[s];
     const D3 x = d3v(p);
-    const double Ps = double(a.t.P2[s]), pms = double(a.pmin[s]), rp = double(sc.rp);
+    const double Ps = double(a.t.P2[s]), pms = double(a.pmin[s]);
+    const double rp = double(sc.rp), irp = 1.0 / rp, lo = double(sc.pair_lo);
     const D3 lGs = d3d(a.lG[s]);
-    D3 accx = d3d(a.lxs[s]), sphi = d3(0, 0, 0);
+    D3 accx = d3(0, 0, 0), sphi = d3(0, 0, 0);
     double accP = 0.0;
-    for (int k = 0; k < n; ++k) {
+    for (int k = ln.lane; k < n; k += LANES) {
         const int i = a.t.nbB[list_at(s, k, a.nbK, a.lt)];
         const V4<R> q = ldg4(a.t.x2 + i);
         R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
         if (!(dot3(dx, dy, dz, dx, dy, dz) < sc.rp2)) continue;
         const D3 r = d3v(q) - x;
         double f, fp;
-        grad_f(dot(r, r), rp, f, fp);
-        const D3 lGi = d3d(a.lG[i]);
+        grad_f(dot(r, r), rp, irp, lo, f, fp);
+        const D3 lGi = d3d(ldg4(a.lG + i));
         // G_i holds (P_s - Pmin_i) phi(x_s - x_i), G_s holds (P_i - Pmin_s) phi(r)
-        const D3 y = (Ps - double(a.pmin[i])) * lGi - (double(a.t.P2[i]) - pms) * lGs;
-        accx = accx + f * y + (fp * dot(r, y)) * r;
-        accP -= f * dot(r, lGi);
-        sphi = sphi + f * r;
+        const D3 y = fma3(pms - double(__ldg(a.t.P2 + i)), lGs, (Ps - double(__ldg(a.pmin + i))) * lGi);
+        accx = fma3(fp * dot(r, y), r, fma3(f, y, accx));
+        accP = __fma_rn(-f, dot(r, lGi), accP);
+        sphi = fma3(f, r, sphi);
     }
     // mirrors of the second generation (the reference skips the slot equal to i, :1759)
     const RowCtx<R> c = adj_row(sc, p);
     const int skip_slot = (a.t.pid2[s] - sc.pbase) + kNumMRR * sc.pbase;
-    for_rows(sc, a.t.mcs2, c, sc.skip_rp, [&](int k) {
+    ln.rows(sc, a.t.mcs2, c, sc.skip_rp, [&](int k) {
         const int slot = __ldg(a.t.m2slot + k);
         if (slot == skip_slot) return;
         const V4<R> q = ldg4(a.t.m2pos + k);
@@ -187,18 +273,22 @@ template <class R, class RN> __global__ void __launch_bounds__(128) k_adj_c2(Adj
         if (!(dot3(dx, dy, dz, dx, dy, dz) < sc.rp2)) return;
         const D3 r = d3v(q) - x;
         double f, fp;
-        grad_f(dot(r, r), rp, f, fp);
-        sphi = sphi + f * r;
+        grad_f(dot(r, r), rp, irp, lo, f, fp);
+        sphi = fma3(f, r, sphi);
         const int os = a.inv2[slot / kNumMRR];
         atomicAdd(a.lP_at + os, f * dot(r, lGs));
         const D3 lm = (double(q.w) - pms) * (f * lGs + (fp * dot(r, lGs)) * r);
         accx = accx - lm;
         atomic_add3(a.lx_at + os, reflect_t(a.t.m2nrm[k], lm));
     });
+    accx = ln.sum(accx);
+    accP = ln.sum(accP);
+    sphi = ln.sum(sphi);
+    if (ln.lane) return;
     const double lpmin = -dot(sphi, lGs);
     if (a.am[s] < 0) accP += lpmin;
     else atomicAdd(a.lP_at + a.am[s], lpmin);
-    a.lxs[s] = v4(accx);
+    a.lxs[s] = v4(d3d(a.lxs[s]) + accx);
     a.lP[s] = accP;
 }
 
@@ -218,20 +308,23 @@ __device__ __forceinline__ D3 col_adj(double colfac, D3 r, double d2, D3 du, D3 
     const double f = dot(du, r);
     if (!(f > 0.0)) return d3(0, 0, 0);
     const double al = colfac / d2, ry = dot(r, y);
-    accu = accu + (al * ry) * r;
-    return (-al * f) * y + (-al * ry) * du + (2.0 * al * f * ry / d2) * r;
+    accu = fma3(al * ry, r, accu);
+    return fma3(-al * f, y, fma3(-al * ry, du, (2.0 * al * f * ry / d2) * r));
 }
 
 // B2: adjoint of ChkCol + MkPrs, gathered per slot; writes the adjoints of x* and u in
 // particle-id order
-template <class R, class RN> __global__ void __launch_bounds__(128) k_adj_b2(AdjArgs<R, RN> a) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+template <class R, class RN, int LANES>
+__global__ void __launch_bounds__(128, kAdjBlocks) k_adj_b2(AdjArgs<R, RN> a) {
+    const AdjLanes<LANES> ln;
+    const int s = ln.s;
     if (s >= a.nF) return;
     const SceneDev<R, RN>& sc = a.sc[0];
     const int st = int(a.t.vp2[s].w);
     const int pid = a.t.pid2[s];
     const int n = a.t.nB[s];
     if (st == kTapeDead || n > a.nbK) {
+        if (ln.lane) return;
         a.lxs_pid[pid] = V4<double>{0, 0, 0, 0};
         a.lu_pid[pid] = V4<double>{0, 0, 0, 0};
         return;
@@ -239,26 +332,24 @@ template <class R, class RN> __global__ void __launch_bounds__(128) k_adj_b2(Adj
     const V4<R> p = a.t.x2[s];
     const D3 x = d3v(p), u = d3v(a.t.u2[s]);
     const D3 lvs = d3d(a.lvv[s]);
-    const double lns = adj_ln(a, sc, s), rp = double(sc.rp), colfac = double(sc.colfac);
-    D3 accx = d3d(a.lxs[s]) + d3d(a.lx_at[s]), accu = lvs;
-    for (int k = 0; k < n; ++k) {
+    const double lns = adj_ln(a, sc, s), colfac = double(sc.colfac);
+    const double rp = double(sc.rp), irp = 1.0 / rp, lo = double(sc.pair_lo);
+    D3 accx = d3(0, 0, 0), accu = d3(0, 0, 0);
+    for (int k = ln.lane; k < n; k += LANES) {
         const int i = a.t.nbB[list_at(s, k, a.nbK, a.lt)];
         const V4<R> q = ldg4(a.t.x2 + i);
         R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
         const R d2r = dot3(dx, dy, dz, dx, dy, dz);
         const D3 r = d3v(q) - x;
         const double d2 = dot(r, r);
-        if (d2r <= sc.rp_lt) {  // both densities: n_s and n_i hold W(|r|)
-            const double d = sqrt(d2);
-            const double wp = (-rp / d2 - 1.0 / rp) / d;  // W'(d) / d
-            accx = accx - (wp * (lns + adj_ln(a, sc, i))) * r;
-        }
+        if (d2r <= sc.rp_lt)   // both densities: n_s and n_i hold W(|r|)
+            accx = fma3(-dens_f(d2, rp, irp, lo) * (lns + adj_ln(a, sc, i)), r, accx);
         if (d2r < sc.rlim2)
-            accx = accx + col_adj(colfac, r, d2, u - d3v(a.t.u2[i]), d3d(a.lvv[i]) - lvs, accu);
+            accx = accx + col_adj(colfac, r, d2, u - d3v(ldg4(a.t.u2 + i)), d3d(ldg4(a.lvv + i)) - lvs, accu);
     }
     const RowCtx<R> c = adj_row(sc, p);
     const D3 mlvs = d3(-lvs.x, -lvs.y, -lvs.z);
-    for_rows(sc, a.wl.cs, c, sc.skip_rw, [&](int j) {
+    ln.rows(sc, a.wl.cs, c, sc.skip_rw, [&](int j) {
         const V4<R> q = ldg4(a.wl.pos + j);
         R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
         if (!(dot3(dx, dy, dz, dx, dy, dz) < sc.rlimw2)) return;
@@ -266,7 +357,7 @@ template <class R, class RN> __global__ void __launch_bounds__(128) k_adj_b2(Adj
         accx = accx + col_adj(colfac, r, dot(r, r), u - d3v(ldg4(a.wl.vel + j)), mlvs, accu);
     });
     // the step's first mirror generation (built from x, not x*: kernel.cu:1904-1921)
-    for_rows(sc, a.t.mcs1, c, sc.skip_rc, [&](int k) {
+    ln.rows(sc, a.t.mcs1, c, sc.skip_rc, [&](int k) {
         const V4<R> q = ldg4(a.t.m1pos + k);
         R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
         const R d2r = dot3(dx, dy, dz, dx, dy, dz);
@@ -277,19 +368,18 @@ template <class R, class RN> __global__ void __launch_bounds__(128) k_adj_b2(Adj
         // every term depends on r = m - x*: x* receives gx, the mirror's owner -H gx
         D3 gx = d3(0, 0, 0);
         if (col) gx = col_adj(colfac, r, d2, u, mlvs, accu);
-        if (dens && lns != 0.0) {
-            const double d = sqrt(d2);
-            const double wp = (-rp / d2 - 1.0 / rp) / d;
-            gx = gx - (wp * lns) * r;
-        }
+        if (dens && lns != 0.0) gx = fma3(-dens_f(d2, rp, irp, lo) * lns, r, gx);
         if (gx.x != 0.0 || gx.y != 0.0 || gx.z != 0.0) {
             accx = accx + gx;
             atomic_add3(a.lx_acc + __ldg(a.t.m1slot + k) / kNumMRR,
                         reflect_t(a.t.m1nrm[k], d3(-gx.x, -gx.y, -gx.z)));
         }
     });
-    a.lxs_pid[pid] = v4(accx);
-    a.lu_pid[pid] = v4(accu);
+    accx = ln.sum(accx);
+    accu = ln.sum(accu);
+    if (ln.lane) return;
+    a.lxs_pid[pid] = v4(d3d(a.lxs[s]) + d3d(a.lx_at[s]) + accx);
+    a.lu_pid[pid] = v4(lvs + accu);
 }
 
 // A1: adjoint of UpPcl1 + ChkPcl for every slot of pass A
@@ -317,8 +407,10 @@ template <class R, class RN> __global__ void __launch_bounds__(128) k_adj_a1(Adj
 
 // A2: adjoint of VscTrm, gathered per slot; writes the adjoints of the step's input in
 // particle-id order and accumulates sum S . lambda_a for the viscosity
-template <class R, class RN> __global__ void __launch_bounds__(128) k_adj_a2(AdjArgs<R, RN> a) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+template <class R, class RN, int LANES>
+__global__ void __launch_bounds__(128, kAdjBlocks) k_adj_a2(AdjArgs<R, RN> a) {
+    const AdjLanes<LANES> ln;
+    const int s = ln.s;
     double part = 0.0;
     if (s < a.nF) {
         const SceneDev<R, RN>& sc = a.sc[0];
@@ -326,44 +418,53 @@ template <class R, class RN> __global__ void __launch_bounds__(128) k_adj_a2(Adj
         const int pid = a.t.pid1[s];
         const int n = a.t.nA[s];
         if (st == kTapeDead || n > a.nbK) {
-            if (n > a.nbK && st != kTapeDead) atomicAdd(a.err, 1);
-            a.lx[pid] = V4<double>{0, 0, 0, 0};
-            a.lv[pid] = V4<double>{0, 0, 0, 0};
+            if (ln.lane == 0) {
+                if (n > a.nbK && st != kTapeDead) atomicAdd(a.err, 1);
+                a.lx[pid] = V4<double>{0, 0, 0, 0};
+                a.lv[pid] = V4<double>{0, 0, 0, 0};
+            }
         } else {
             const V4<R> p = a.t.x1[s];
             const D3 x = d3v(p), v = d3v(a.t.v1[s]);
             const double kn = double(sc.kn), two_l0 = double(sc.two_l0);
+            const double lo = double(sc.pair_lo);
             const D3 las = d3d(a.la[s]);
             const D3 lSs = kn * las;
-            D3 accx = d3d(a.lxa[s]), accv = d3d(a.lva[s]), S = d3(0, 0, 0);
-            for (int k = 0; k < n; ++k) {
+            D3 accx = d3(0, 0, 0), accv = d3(0, 0, 0), S = d3(0, 0, 0);
+            for (int k = ln.lane; k < n; k += LANES) {
                 const int i = a.t.nbA[list_at(s, k, a.nbK, a.lt)];
                 const D3 r = d3v(ldg4(a.t.x1 + i)) - x;
                 const D3 vi = d3v(ldg4(a.t.v1 + i));
-                const double d2 = dot(r, r), d = sqrt(d2), w = two_l0 / (d2 * d);
-                S = S + w * (vi - v);
+                double w, g;
+                visc_f(dot(r, r), two_l0, lo, w, g);
+                S = fma3(w, vi - v, S);
                 // S_i holds (v_s - v_i) w, S_s holds (v_i - v_s) w; grad w(x_s - x_i) = 3 w r / d^2
-                const D3 y = kn * d3d(a.la[i]) - lSs;
-                accv = accv + w * y;
-                accx = accx + ((3.0 * w / d2) * dot(v - vi, y)) * r;
+                const D3 y = kn * d3d(ldg4(a.la + i)) - lSs;
+                accv = fma3(w, y, accv);
+                accx = fma3(g * dot(v - vi, y), r, accx);
             }
             const RowCtx<R> c = adj_row(sc, p);
             const double vl = dot(v, lSs);
-            for_rows(sc, a.t.mcs1, c, sc.skip_r, [&](int k) {
+            ln.rows(sc, a.t.mcs1, c, sc.skip_r, [&](int k) {
                 const V4<R> q = ldg4(a.t.m1pos + k);
                 R dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
                 if (!(dot3(dx, dy, dz, dx, dy, dz) <= sc.r_le)) return;
                 const D3 r = d3v(q) - x;
-                const double d2 = dot(r, r), d = sqrt(d2), w = two_l0 / (d2 * d);
-                S = S - w * v;
-                accv = accv - w * lSs;
-                const D3 gm = ((3.0 * w / d2) * vl) * r;  // d/dm of -(v . lambda_S) w(|m - x|)
+                double w, g;
+                visc_f(dot(r, r), two_l0, lo, w, g);
+                S = fma3(-w, v, S);
+                accv = fma3(-w, lSs, accv);
+                const D3 gm = (g * vl) * r;  // d/dm of -(v . lambda_S) w(|m - x|)
                 accx = accx - gm;
                 atomic_add3(a.lx_acc + __ldg(a.t.m1slot + k) / kNumMRR, reflect_t(a.t.m1nrm[k], gm));
             });
-            part = dot(S, las);
-            a.lx[pid] = v4(accx);
-            a.lv[pid] = v4(accv);
+            part = dot(S, las);  // of this lane's entries: the block's sum adds them up
+            accx = ln.sum(accx);
+            accv = ln.sum(accv);
+            if (ln.lane == 0) {
+                a.lx[pid] = v4(d3d(a.lxa[s]) + accx);
+                a.lv[pid] = v4(d3d(a.lva[s]) + accv);
+            }
         }
     }
     // block sum of S . lambda_a, one atomic per block

@@ -1957,7 +1957,15 @@ template <class R, class RN> class Solver final : public SolverBase {
         else bin_mirrors(M1, mcs1);
     }
 
+    // lanes per slot: where the pass kernels go from a warp to a group and to one thread per
+    // particle (k_adj_*: times at all sizes)
     void back_step(const TapeStep<R>& t) {
+        const int g = group_lanes(kGroupMostBC);
+        if (g == 32) back_step_lanes<32>(t);
+        else if (g == 8) back_step_lanes<16>(t);
+        else back_step_lanes<4>(t);
+    }
+    template <int G> void back_step_lanes(const TapeStep<R>& t) {
         AdjState& s = *adj;
         AdjArgs<R, RN> A;
         A.sc = d_sc; A.nF = nF; A.nbK = nbK; A.lt = list_layout(); A.t = t; A.wl = wall_view();
@@ -1967,16 +1975,16 @@ template <class R, class RN> class Solver final : public SolverBase {
         A.lxs_pid = s.lxs_pid; A.lu_pid = s.lu_pid;
         A.la = s.la; A.lxa = s.lxa; A.lva = s.lva;
         A.lkn = s.lkn; A.err = s.err;
-        const int g = blocks(nF, 128);
-        k_adj_c1<R, RN><<<g, 128, 0, stream>>>(A);
+        const int g = blocks(nF, 128), gl = blocks(nF, 128 / G);
+        k_adj_c1<R, RN, G><<<gl, 128, 0, stream>>>(A);
         KL();
-        k_adj_c2<R, RN><<<g, 128, 0, stream>>>(A);
+        k_adj_c2<R, RN, G><<<gl, 128, 0, stream>>>(A);
         KL();
-        k_adj_b2<R, RN><<<g, 128, 0, stream>>>(A);
+        k_adj_b2<R, RN, G><<<gl, 128, 0, stream>>>(A);
         KL();
         k_adj_a1<R, RN><<<g, 128, 0, stream>>>(A);
         KL();
-        k_adj_a2<R, RN><<<g, 128, 0, stream>>>(A);
+        k_adj_a2<R, RN, G><<<gl, 128, 0, stream>>>(A);
         KL();
         k_adj_fin<<<g, 128, 0, stream>>>(d_fluid_ids, nF, s.lx, s.lx_acc);
         KL();

@@ -1,0 +1,65 @@
+"""The step adjoint at the sizes where its kernels change their lanes per slot (a warp, 16, 4).
+
+Reverse-mode gradients of a random linear functional of the final state against central
+differences of the FP64 forward on the same GPU, to the adjoint tests' 1e-3. Three steps of 0.05
+m/s move a particle by 2e-3 of the spacing, and the jitter leaves neighbours 0.98 spacings apart,
+so no pair comes under the collision distance of 0.9: the rollout is smooth in the velocities and
+a relative step of 1e-6 puts truncation and rounding of the differences under 1e-6.
+"""
+from __future__ import annotations
+
+import math
+
+import numpy as np
+import pytest
+
+from mps_cuda_b200 import SceneDesc, configs
+from mps_cuda_b200.adjoint import RolloutProblem
+
+pytestmark = pytest.mark.gpu
+
+
+def _dot(a, b):
+    return math.fsum((np.asarray(a) * np.asarray(b)).ravel())
+
+
+@pytest.mark.parametrize("block,tank,steps,every", [
+    ((1, 1, 2), (5, 4, 6), 3, 3),
+    ((3, 7, 11), (9, 7, 13), 5, 2),       # three segments, the last one short
+    ((25, 8, 25), (31, 9, 27), 3, 3),     # 5000: the last size of a warp each
+    ((23, 17, 13), (40, 17, 15), 3, 3),   # 5083: 16 lanes each
+    ((46, 46, 47), (60, 46, 50), 2, 2),   # 99 452: 4 lanes each
+])
+def test_gradient_at_the_lines_of_the_lane_rule(block, tank, steps, every):
+    l0 = 0.02
+    pr = RolloutProblem(SceneDesc(l0, tuple(t * l0 for t in tank), block, seed=5, vel_sigma=0.05,
+                                  vel_seed=2), dt=2e-4, steps=steps, every=every)
+    n, f = pr.typ.shape[0], pr.fluid
+    rng = np.random.default_rng(7)
+    a, b, d = (rng.standard_normal((3, f.size)) for _ in range(3))
+    lam_pos, lam_vel = np.zeros((3, n)), np.zeros((3, n))
+    lam_pos[:, f], lam_vel[:, f] = a, b
+    v0 = pr.vel[:, f].copy()
+    h = pr.solver(configs.NU, v0)
+    try:
+        h.adjoint_record(steps, every)
+        end = h.state()
+        _, gv, gnu = h.adjoint_backward(lam_pos, lam_vel)
+        _, gv2, gnu2 = h.adjoint_backward(lam_pos, lam_vel)
+        again = h.state()
+    finally:
+        h.close()
+    assert all(np.array_equal(end[k], again[k]) for k in ("typ", "pos", "vel", "prs"))
+    # the same up to the order of the double atomic adds
+    assert np.max(np.abs(gv - gv2)) <= 1e-8 * np.max(np.abs(gv)) and abs(gnu - gnu2) <= 1e-8 * abs(gnu)
+
+    def value(nu, v):
+        st = pr.run(nu, v)
+        return _dot(a, st["pos"][:, f]) + _dot(b, st["vel"][:, f])
+
+    eps = 1e-6 * float(np.sqrt(np.mean(v0 ** 2)))
+    fd = (value(configs.NU, v0 + eps * d) - value(configs.NU, v0 - eps * d)) / (2 * eps)
+    assert abs(fd - _dot(gv[:, f], d)) <= 1e-3 * abs(fd), (fd, _dot(gv[:, f], d))
+    hn = 1e-4 * configs.NU
+    fd = (value(configs.NU + hn, v0) - value(configs.NU - hn, v0)) / (2 * hn)
+    assert abs(fd - gnu) <= 1e-3 * abs(fd), (fd, gnu)
