@@ -1094,6 +1094,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         CK(cudaStreamSynchronize(stream));
         motion_on = nW > 0 && (hmot[0].type != 0 || hmot[1].type != 0);
         walls_moved = walls_moved || motion_on;
+        if (adj) adj->taped = -1;
         invalidate_graph();
     }
 
@@ -1230,13 +1231,15 @@ template <class R, class RN> class Solver final : public SolverBase {
         tail_pending = false;
     }
 
+    void clear_acc() {
+        CK(cudaMemsetAsync(S.acc, 0, sizeof(V4<R>) * std::max(nF, 1), stream));
+        CK(cudaMemsetAsync(S2.acc, 0, sizeof(V4<R>) * std::max(nF, 1), stream));
+        acc_dirty = false;
+    }
+
     void prepare_fused() {
         if (!lists_valid || !sorted) mkbkt(acc_dirty);
-        if (acc_dirty) {
-            CK(cudaMemsetAsync(S.acc, 0, sizeof(V4<R>) * std::max(nF, 1), stream));
-            CK(cudaMemsetAsync(S2.acc, 0, sizeof(V4<R>) * std::max(nF, 1), stream));
-            acc_dirty = false;
-        }
+        if (acc_dirty) clear_acc();
         if (!m1_valid) {
             reset_raw();
             run_gen<false, false>(args(M1, mcs1), block, S.pos, S.prs, S.typ);
@@ -1770,6 +1773,10 @@ template <class R, class RN> class Solver final : public SolverBase {
     // keep the neighbour lists, mirror generations and pre-clamp velocities of each step)
     // and runs the step adjoints in reverse over what they kept. The replay repeats the
     // original steps exactly: the bucket order and every sum depend on the state only.
+    // The sweep starts with the last segment, so the recording runs that one with the recording
+    // kernels in the first place and the sweep does not replay it: a rollout of one segment (20
+    // steps of 48 000 particles in FP64) is recorded in 13.6 instead of 11.6 ms and swept in 8.6
+    // instead of 21.0.
     struct Ckpt {
         R* pos; R* vel; R* prs; R* pav; int8_t* typ;
     };
@@ -1778,6 +1785,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         int nsteps = 0, every = 0, nck = 0;
         int nbK = 0;  // list capacity the tape was allocated and recorded with
         long long steps_end = 0;
+        int taped = -1;  // the segment the tape holds, if the handle's walls are still its walls
         std::vector<Ckpt> ck;  // nck segment starts + the final state
         std::vector<TapeStep<R>> tape;
         V4<R>* unrm = nullptr;
@@ -1867,13 +1875,24 @@ template <class R, class RN> class Solver final : public SolverBase {
         const int nck = (nsteps + every - 1) / every;
         if (!adj || adj->nck != nck || adj->every != every) adj_alloc(nck, every);
         adj->nsteps = 0;
+        adj->taped = -1;
+        // diagnostics, the kernels' times and staged walks belong to the ordinary step
+        const bool tape_last = nF > 0 && !diag_on && !timing_on && stage_mode == MPS_STAGE_GLOBAL;
         for (int c = 0; c < nck; ++c) {
             snapshot(adj->ck[c]);
-            step(std::min(every, nsteps - c * every));
+            const int ns = std::min(every, nsteps - c * every);
+            if (c + 1 < nck || !tape_last) {
+                step(ns);
+                continue;
+            }
+            finish_tail();
+            tape_steps(ns, TAPE_PENDING);
+            steps += ns;
         }
         snapshot(adj->ck[nck]);
         adj->nsteps = nsteps;
         adj->steps_end = steps;
+        if (tape_last) adj->taped = nck - 1;
         CK(cudaStreamSynchronize(stream));
     }
 
@@ -1896,17 +1915,34 @@ template <class R, class RN> class Solver final : public SolverBase {
         return a;
     }
 
-    // the first mirror generation of a replayed segment, as prepare_fused makes it
+    // the first mirror generation of a taped segment, as prepare_fused makes it
     void tape_prepare(const TapeStep<R>& t) {
-        mkbkt(false);
+        if (!lists_valid || !sorted) mkbkt(acc_dirty);
+        if (acc_dirty) clear_acc();
         reset_raw();
         PassArgs<R, RN> a = tape_args(M1.pos, M1.slot, mcs1, nb, nbcnt, nullptr);
         run_gen<false, true>(a, block, S.pos, S.prs, S.typ);
         bin_mirrors_n(t.m1pos, t.m1slot, t.m1nrm, t.mcs1);
     }
 
+    // What follows a taped segment: its end with the mirrors in M1, nothing (another segment is
+    // taped over it), or a pending end, with the mirror tables as a step leaves them
+    enum TapeEnd { TAPE_ENDED, TAPE_DROPPED, TAPE_PENDING };
+    void tape_steps(int ns, TapeEnd end) {
+        tape_prepare(adj->tape[0]);
+        for (int k = 0; k < ns; ++k)
+            tape_body(adj->tape[k], k + 1 < ns ? &adj->tape[k + 1] : nullptr, end);
+    }
+    void tape_mirrors(const MirrorBuf<R>& m, int* mcs, int8_t* near, const V4<R>* pos, const int* slot,
+                      const int* cs_) {
+        CK(cudaMemcpyAsync(m.pos, pos, sizeof(V4<R>) * size_t(cap), cudaMemcpyDeviceToDevice, stream));
+        CK(cudaMemcpyAsync(m.slot, slot, sizeof(int) * size_t(cap), cudaMemcpyDeviceToDevice, stream));
+        CK(cudaMemcpyAsync(mcs, cs_, sizeof(int) * (size_t(L()) + 1), cudaMemcpyDeviceToDevice, stream));
+        near_flags(mcs, near);
+    }
+
     // fused_body with the recording kernels; `next` receives the next step's mirrors
-    void tape_body(const TapeStep<R>& t, const TapeStep<R>* next) {
+    void tape_body(const TapeStep<R>& t, const TapeStep<R>* next, TapeEnd end) {
         const int ba = blk[MPS_K_PASS_A], bb = blk[MPS_K_PASS_B], bc = blk[MPS_K_PASS_C],
                   bg = blk[MPS_K_GEN];
         const size_t F = size_t(nF);
@@ -1950,6 +1986,13 @@ template <class R, class RN> class Solver final : public SolverBase {
         }
         a = tape_args(t.m2pos, t.m2slot, t.mcs2, t.nbB, t.nB, t.vp2);
         run_pass_c<false, true>(a, bc);
+        if (!next && end == TAPE_DROPPED) return;
+        if (!next && end == TAPE_PENDING) {
+            tape_mirrors(M1, mcs1, near_m1, t.m1pos, t.m1slot, t.mcs1);
+            tape_mirrors(M2, mcs2, near_m2, t.m2pos, t.m2slot, t.mcs2);
+            tail_pending = lists_valid = sorted = m1_valid = true;
+            return;
+        }
         reset_raw();
         run_gen<false, true>(a, bg, t_pos, t_prs, t_typ);
         bin_fluid(t_pos, t_vel, nullptr, t_prs, S.pav, S.pid, t_typ);
@@ -2018,10 +2061,15 @@ template <class R, class RN> class Solver final : public SolverBase {
         CK(cudaMemsetAsync(s.err, 0, sizeof(int), stream));
         invalidate_graph();
         for (int c = s.nck - 1; c >= 0; --c) {
-            restore(s.ck[c]);
             const int ns = std::min(s.every, s.nsteps - c * s.every);
-            tape_prepare(s.tape[0]);
-            for (int k = 0; k < ns; ++k) tape_body(s.tape[k], k + 1 < ns ? &s.tape[k + 1] : nullptr);
+            if (s.taped != c) {
+                s.taped = -1;
+                restore(s.ck[c]);
+                tape_steps(ns, c > 0 ? TAPE_DROPPED : TAPE_ENDED);
+                s.taped = c;
+            } else if (c == 0) {
+                finish_tail();  // M1 as the replay would leave it
+            }
             for (int k = ns - 1; k >= 0; --k) back_step(s.tape[k]);
         }
         auto out = [&](const V4<double>* src, double* dst) {

@@ -14,6 +14,7 @@ import numpy as np
 import pytest
 
 from mps_cuda_b200 import SceneDesc, configs
+from mps_cuda_b200 import _lib as L
 from mps_cuda_b200.adjoint import RolloutProblem
 
 pytestmark = pytest.mark.gpu
@@ -63,3 +64,52 @@ def test_gradient_at_the_lines_of_the_lane_rule(block, tank, steps, every):
     hn = 1e-4 * configs.NU
     fd = (value(configs.NU + hn, v0) - value(configs.NU - hn, v0)) / (2 * hn)
     assert abs(fd - gnu) <= 1e-3 * abs(fd), (fd, gnu)
+
+
+@pytest.mark.parametrize("block,tank,every", [
+    ((8, 6, 10), (20, 10, 20), 6),      # one segment
+    ((8, 6, 10), (20, 10, 20), 4),      # the last one short
+    ((23, 17, 13), (40, 17, 15), 3),
+])
+def test_recording_leaves_the_handle_as_the_same_steps_do(block, tank, every):
+    """The last segment runs with the recording kernels: state, mirrors and counters, the steps
+    that follow, and the gradient are those of ordinary steps and a replay (diagnostics on)."""
+    l0, n = 0.02, 6
+    pr = RolloutProblem(SceneDesc(l0, tuple(t * l0 for t in tank), block, seed=6, vel_sigma=0.2,
+                                  vel_seed=3), dt=2e-4, steps=n, every=every)
+    v0 = pr.vel[:, pr.fluid].copy()
+    hs = [pr.solver(configs.NU, v0) for _ in range(3)]
+    lam = np.zeros((3, pr.typ.shape[0]))
+    lam[:, pr.fluid] = np.random.default_rng(8).standard_normal((3, pr.fluid.size))
+
+    def same(a, b):
+        x, y = a.state(), b.state()
+        for k in ("typ", "pos", "vel", "acc", "prs", "pav"):
+            assert np.array_equal(x[k], y[k]), k
+        for k in ("steps", "n_fluid_alive", "n_mirror_1", "n_mirror_2"):
+            assert a.counters()[k] == b.counters()[k], k
+        for w in (2, 1, 0):
+            p, q = a.mirrors(w), b.mirrors(w)
+            assert all(np.array_equal(p[k], q[k]) for k in ("slot", "pos")), w
+
+    try:
+        stepped, taped, replayed = hs
+        replayed.set_option(L.OPT_DIAG, 1)
+        for h in hs:
+            h.step(2)   # a pending step end before the recording
+        stepped.step(n)
+        grads = []
+        for h in (taped, replayed):
+            h.adjoint_record(n, every)
+            grads.append(h.adjoint_backward(lam, lam) if h is replayed else None)
+        same(stepped, taped)
+        grads[0] = taped.adjoint_backward(lam, lam)
+        for a, b in zip(*grads):
+            assert np.max(np.abs(np.subtract(a, b))) <= 1e-8 * np.max(np.abs(a))
+        for h in hs:
+            h.step(3)
+        same(stepped, taped)
+        same(stepped, replayed)
+    finally:
+        for h in hs:
+            h.close()
