@@ -1199,29 +1199,32 @@ template <class R, class RN> class Solver final : public SolverBase {
     // pre-build arrays.
     void step_tail() {
         const int bg = blk[MPS_K_GEN];
-        const bool fork = (overlap & 1) && !timing_on;
         auto mirrors = [&] {
             reset_raw();
-            Scope t(this, MPS_K_GEN);
-            run_gen<false, false>(args(M2, mcs2), bg, t_pos, t_prs, t_typ);
+            {
+                Scope t(this, MPS_K_GEN);
+                run_gen<false, false>(args(M2, mcs2), bg, t_pos, t_prs, t_typ);
+            }
+            bin_mirrors(M1, mcs1);
         };
+        beside(mirrors, [&] { bin_fluid(t_pos, t_vel, nullptr, t_prs, S.pav, S.pid, t_typ); });
+    }
+
+    // a step's end: the mirrors on the second stream beside the fluid's bucket build
+    template <class M, class F> void beside(M&& mirrors, F&& fluid) {
+        const bool fork = (overlap & 1) && !timing_on;
         if (fork) {
             ensure_side();
             CK(cudaEventRecord(ev_fork, stream));
             CK(cudaStreamWaitEvent(side, ev_fork, 0));
-            {
-                OnStream o(this, side);
-                mirrors();
-                bin_mirrors(M1, mcs1);
-                CK(cudaEventRecord(ev_join, side));
-            }
-            bin_fluid(t_pos, t_vel, nullptr, t_prs, S.pav, S.pid, t_typ);
-            CK(cudaStreamWaitEvent(stream, ev_join, 0));
+            OnStream o(this, side);
+            mirrors();
+            CK(cudaEventRecord(ev_join, side));
         } else {
             mirrors();
-            bin_fluid(t_pos, t_vel, nullptr, t_prs, S.pav, S.pid, t_typ);
-            bin_mirrors(M1, mcs1);
         }
+        fluid();
+        if (fork) CK(cudaStreamWaitEvent(stream, ev_join, 0));
     }
 
     // runs the pending end of the latest step, if any (before reading the sorted state)
@@ -1993,11 +1996,13 @@ template <class R, class RN> class Solver final : public SolverBase {
             tail_pending = lists_valid = sorted = m1_valid = true;
             return;
         }
-        reset_raw();
-        run_gen<false, true>(a, bg, t_pos, t_prs, t_typ);
-        bin_fluid(t_pos, t_vel, nullptr, t_prs, S.pav, S.pid, t_typ);
-        if (next) bin_mirrors_n(next->m1pos, next->m1slot, next->m1nrm, next->mcs1);
-        else bin_mirrors(M1, mcs1);
+        auto mirrors = [&] {
+            reset_raw();
+            run_gen<false, true>(a, bg, t_pos, t_prs, t_typ);
+            if (next) bin_mirrors_n(next->m1pos, next->m1slot, next->m1nrm, next->mcs1);
+            else bin_mirrors(M1, mcs1);
+        };
+        beside(mirrors, [&] { bin_fluid(t_pos, t_vel, nullptr, t_prs, S.pav, S.pid, t_typ); });
     }
 
     // lanes per slot: where the pass kernels go from a warp to a group and to one thread per
