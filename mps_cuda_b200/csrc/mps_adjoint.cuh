@@ -122,13 +122,38 @@ template <int LANES> struct AdjLanes {
         return v;
     }
     __device__ __forceinline__ D3 sum(D3 v) const { return D3{sum(v.x), sum(v.y), sum(v.z)}; }
-    // f(j) for the rows' buckets around a particle (for_rows), dealt to the lanes row by row
+    // f(j) for the buckets around a particle (for_rows). Each lane reads a row's range, so that the
+    // nine rows' loads, most of them of empty rows, run side by side; a row's items are dealt to
+    // the lanes. Row after row an adjoint step took 74 / 394 / 1610 us at 3.5k / 48k / 192k
+    // particles, so 67 / 382 / 1468.
     template <class R, class RN, class F>
     __device__ __forceinline__ void rows(const SceneDev<R, RN>& sc, const int* __restrict__ cs,
                                          const RowCtx<R>& c, R B, F&& f) const {
-        for_rows_ranges(sc, cs, c, B, [&](int lo, int hi) {
-            for (int j = lo + lane; j < hi; j += LANES) f(j);
-        });
+#pragma unroll 1
+        for (int r0 = 0; r0 < 9; r0 += LANES) {
+            int lo = 0, hi = 0;
+            const int r = r0 + lane;
+            if (r < 9) {
+                const int dz = r / 3 - 1, dy = r % 3 - 1;
+                const R ddz = dz < 0 ? c.dzl : (dz > 0 ? c.dzh : R(0));
+                const R ddy = dy < 0 ? c.dyl : (dy > 0 ? c.dyh : R(0));
+                const R dyz2 = ddy * ddy + ddz * ddz;
+                if (!(dyz2 > B)) {
+                    const int jl = (dyz2 + c.dxl * c.dxl <= B) ? c.ix - 1 : c.ix;
+                    const int jh = (dyz2 + c.dxh * c.dxh <= B) ? c.ix + 1 : c.ix;
+                    const int row = sc.cbase + (c.iz + dz) * sc.nbxy + (c.iy + dy) * sc.nbx;
+                    lo = __ldg(cs + row + jl);
+                    hi = __ldg(cs + row + jh + 1);
+                }
+            }
+            unsigned full = (__ballot_sync(mask, hi > lo) & mask) >> (threadIdx.x & 31 & ~(LANES - 1));
+            while (full) {
+                const int q = __ffs(full) - 1;
+                full &= full - 1;
+                const int l = __shfl_sync(mask, lo, q, LANES), h = __shfl_sync(mask, hi, q, LANES);
+                for (int j = l + lane; j < h; j += LANES) f(j);
+            }
+        }
     }
 };
 
