@@ -149,7 +149,10 @@ enum {
 enum {
     MPS_OPT_DIAG = 0,        /* 1: record per-particle neighbour counts (slower)        */
     MPS_OPT_GRAPH = 1,       /* 1: replay mps_step through a captured CUDA graph        */
-    MPS_OPT_BLOCK = 2,       /* threads per block of the neighbour passes (0 = tuned)   */
+    MPS_OPT_BLOCK = 2,       /* threads per block of the neighbour passes (0 = tuned). This,
+                                MPS_OPT_CANDIDATE_BATCH and MPS_OPT_REGISTER_BOUND shape the
+                                kernels with one thread per particle; scenes small enough for
+                                several lanes per particle run without them.             */
     MPS_OPT_CELL_SKIP = 3,   /* 1: skip bucket rows outside the radius (default 1)      */
     MPS_OPT_TIMING = 4,      /* 1: time every kernel group of mps_step with CUDA events
                                 on the handle's stream (steps then run without a graph) */
@@ -171,7 +174,7 @@ enum {
                                 at the default). Results never depend on it.              */
     MPS_OPT_OVERLAP = 11     /* work on a second stream of the handle, bit 0: at the end
                                 of a step the fluid bucket build beside the next step's
-                                mirror generation; bit 1: the step's second mirror
+                                mirror generation and mirror bucket build; bit 1: the step's second mirror
                                 generation (positions, cull, buckets) beside ChkCol/MkPrs,
                                 its pressures filled in after them. 3 (both) is the
                                 default, 0 one stream. Steps timed with MPS_OPT_TIMING
@@ -355,7 +358,8 @@ int mps_get_option(mps_handle* h, int32_t opt, int32_t* value);
  * one behind the same state layout.
  *
  * mps_adjoint_record advances the handle `nsteps` steps (as mps_step) and keeps the state
- * every `checkpoint_every` steps on the device. Single-scene handles only.
+ * every `checkpoint_every` steps on the device, and of the last of these segments all that its
+ * adjoint needs. Single-scene handles only.
  *
  * mps_adjoint_backward takes the adjoint of a scalar loss with respect to the final
  * positions and velocities (SoA x[n], y[n], z[n], doubles, particle-id order; NULL = zero)
