@@ -957,10 +957,17 @@ template <class R, class RN> class Solver final : public SolverBase {
     //   pass C      97 / 19 / 15     104 / 27 / 31     101 / 47 / 66     103 / 75 / 111    120 / 131
     //   two generations and culls
     //              167 / 79 / 52     211 / 86 / 95     205 / 119 / 151   203 / 139 / 209   198 / 207
-    // and the FP64 crossings lie at the same sizes.
-    static constexpr int kWarpMost = 5000, kGroupMostA = 65536, kGroupMostBC = 98304,
-                         kGroupMostGen = 180000, kCullMost = 600000;
-    int group_lanes(int most) const { return nF <= kWarpMost ? 32 : (nF <= most ? 8 : 0); }
+    // and the FP64 crossings to one thread lie at the same sizes. Between a warp and eight lanes,
+    // 16 lanes: a step by graphs, us (a warp / 16 / 8 lanes):
+    //              2.6k   3.4k  4.0k   4.4k   5.0k particles  6.0k         9.0k      12.5k     19.8k
+    //   FP32    120/137 130/137 137/142 146/145 158/154  173/163/177 203/188/192 240/212/213 304/249/245
+    //   FP64    134/139 148/140 160/150 174/156 186/169  201/185/199 246/218/224 293/253/265 380/312/315
+    static constexpr int kWarpMost = sizeof(R) == 4 ? 4400 : 3000, kHalfMost = 12288,
+                         kGroupMostA = 65536, kGroupMostBC = 98304, kGroupMostGen = 180000,
+                         kCullMost = 600000;
+    int group_lanes(int most) const {
+        return nF <= kWarpMost ? 32 : (nF <= kHalfMost ? 16 : (nF <= most ? 8 : 0));
+    }
     int list_layout() const { return group_lanes(kGroupMostBC) ? kListGroup : kListThread; }
     int group_grid(int g) const { return blocks(nF, 128 / g); }
 
@@ -969,6 +976,8 @@ template <class R, class RN> class Solver final : public SolverBase {
         const int g = group_lanes(kGroupMostA);
         if (g == 32)
             k_pass_a_g<R, RN, D, TAPE, 32><<<group_grid(32), 128, 0, stream>>>(a);
+        else if (g == 16)
+            k_pass_a_g<R, RN, D, TAPE, 16><<<group_grid(16), 128, 0, stream>>>(a);
         else if (g == 8)
             k_pass_a_g<R, RN, D, TAPE, 8><<<group_grid(8), 128, 0, stream>>>(a);
         else if (TAPE)
@@ -983,6 +992,8 @@ template <class R, class RN> class Solver final : public SolverBase {
         const int g = group_lanes(kGroupMostBC);
         if (g == 32)
             k_pass_b_g<R, RN, D, 32><<<group_grid(32), 128, 0, stream>>>(a);
+        else if (g == 16)
+            k_pass_b_g<R, RN, D, 16><<<group_grid(16), 128, 0, stream>>>(a);
         else if (g == 8)
             k_pass_b_g<R, RN, D, 8><<<group_grid(8), 128, 0, stream>>>(a);
         else if (reg_bound & 1)
@@ -998,8 +1009,12 @@ template <class R, class RN> class Solver final : public SolverBase {
             k_pass_c_g<R, RN, D, false, true, 32><<<group_grid(32), 128, 0, stream>>>(a);
         else if (g == 32)
             k_pass_c_g<R, RN, D, TAPE, false, 32><<<group_grid(32), 128, 0, stream>>>(a);
+        else if (g == 16 && corr)
+            k_pass_c_g<R, RN, D, false, true, 16><<<group_grid(16), 128, 0, stream>>>(a);
         else if (g == 8 && corr)
             k_pass_c_g<R, RN, D, false, true, 8><<<group_grid(8), 128, 0, stream>>>(a);
+        else if (g == 16)
+            k_pass_c_g<R, RN, D, TAPE, false, 16><<<group_grid(16), 128, 0, stream>>>(a);
         else if (g == 8)
             k_pass_c_g<R, RN, D, TAPE, false, 8><<<group_grid(8), 128, 0, stream>>>(a);
         else if (corr)
@@ -1016,6 +1031,8 @@ template <class R, class RN> class Solver final : public SolverBase {
         const int g = group_lanes(kGroupMostGen);
         if (g == 32)
             k_gen_cull_g<R, RN, D, TAPE, CLS, 32><<<group_grid(32), 128, 0, stream>>>(a, pos, prs, typ);
+        else if (g == 16)
+            k_gen_cull_g<R, RN, D, TAPE, CLS, 16><<<group_grid(16), 128, 0, stream>>>(a, pos, prs, typ);
         else if (g == 8)
             k_gen_cull_g<R, RN, D, TAPE, CLS, 8><<<group_grid(8), 128, 0, stream>>>(a, pos, prs, typ);
         else
@@ -1456,6 +1473,8 @@ template <class R, class RN> class Solver final : public SolverBase {
         if (diag_on) k_ph_grd<R, RN, true, CORR><<<gb, block, 0, stream>>>(a);
         else if (g == 32)
             k_pass_c_g<R, RN, false, false, CORR, 32, true><<<group_grid(32), 128, 0, stream>>>(a);
+        else if (g == 16)
+            k_pass_c_g<R, RN, false, false, CORR, 16, true><<<group_grid(16), 128, 0, stream>>>(a);
         else if (g == 8)
             k_pass_c_g<R, RN, false, false, CORR, 8, true><<<group_grid(8), 128, 0, stream>>>(a);
         else k_ph_grd<R, RN, false, CORR><<<gb, block, 0, stream>>>(a);
@@ -1507,6 +1526,8 @@ template <class R, class RN> class Solver final : public SolverBase {
                 if (diag_on) k_ph_vsc<R, RN, true><<<gb, block, 0, stream>>>(a);
                 else if (lanes(kGroupMostA) == 32)
                     k_pass_a_g<R, RN, false, false, 32, true><<<group_grid(32), 128, 0, stream>>>(a);
+                else if (lanes(kGroupMostA) == 16)
+                    k_pass_a_g<R, RN, false, false, 16, true><<<group_grid(16), 128, 0, stream>>>(a);
                 else if (lanes(kGroupMostA) == 8)
                     k_pass_a_g<R, RN, false, false, 8, true><<<group_grid(8), 128, 0, stream>>>(a);
                 else k_ph_vsc<R, RN, false><<<gb, block, 0, stream>>>(a);
@@ -1525,6 +1546,8 @@ template <class R, class RN> class Solver final : public SolverBase {
                 if (diag_on) k_ph_col<R, RN, true><<<gb, block, 0, stream>>>(a);
                 else if (lanes(kGroupMostBC) == 32)
                     k_pass_b_g<R, RN, false, 32, PASS_COL><<<group_grid(32), 128, 0, stream>>>(a);
+                else if (lanes(kGroupMostBC) == 16)
+                    k_pass_b_g<R, RN, false, 16, PASS_COL><<<group_grid(16), 128, 0, stream>>>(a);
                 else if (lanes(kGroupMostBC) == 8)
                     k_pass_b_g<R, RN, false, 8, PASS_COL><<<group_grid(8), 128, 0, stream>>>(a);
                 else k_ph_col<R, RN, false><<<gb, block, 0, stream>>>(a);
@@ -1538,6 +1561,8 @@ template <class R, class RN> class Solver final : public SolverBase {
                 if (diag_on) k_ph_prs<R, RN, true><<<gb, block, 0, stream>>>(a);
                 else if (lanes(kGroupMostBC) == 32)
                     k_pass_b_g<R, RN, false, 32, PASS_PRS><<<group_grid(32), 128, 0, stream>>>(a);
+                else if (lanes(kGroupMostBC) == 16)
+                    k_pass_b_g<R, RN, false, 16, PASS_PRS><<<group_grid(16), 128, 0, stream>>>(a);
                 else if (lanes(kGroupMostBC) == 8)
                     k_pass_b_g<R, RN, false, 8, PASS_PRS><<<group_grid(8), 128, 0, stream>>>(a);
                 else k_ph_prs<R, RN, false><<<gb, block, 0, stream>>>(a);
@@ -2005,12 +2030,11 @@ template <class R, class RN> class Solver final : public SolverBase {
         beside(mirrors, [&] { bin_fluid(t_pos, t_vel, nullptr, t_prs, S.pav, S.pid, t_typ); });
     }
 
-    // lanes per slot: where the pass kernels go from a warp to a group and to one thread per
-    // particle (k_adj_*: times at all sizes)
+    // lanes per slot: a warp, 16 where the pass kernels have several, 4 beyond (AdjLanes: times at
+    // all sizes)
     void back_step(const TapeStep<R>& t) {
-        const int g = group_lanes(kGroupMostBC);
-        if (g == 32) back_step_lanes<32>(t);
-        else if (g == 8) back_step_lanes<16>(t);
+        if (nF <= 5000) back_step_lanes<32>(t);
+        else if (nF <= kGroupMostBC) back_step_lanes<16>(t);
         else back_step_lanes<4>(t);
     }
     template <int G> void back_step_lanes(const TapeStep<R>& t) {

@@ -1,9 +1,9 @@
 """The neighbour passes with several lanes per particle (mps_group.cuh) against the CPU oracle.
 
-Small scenes run the passes with a warp or eight lanes per particle, larger ones with one thread
+Small scenes run the passes with a warp, 16 or eight lanes per particle, larger ones with one thread
 (Solver::group_lanes); every path must give the oracle's state bit for bit. The blocks have odd
 sides, so that a warp's particles span bucket rows and the last warp is ragged; the sizes lie on
-both sides of the line between a warp and eight lanes, and on the line of one thread.
+both sides of the lines between a warp, 16 and eight lanes, and on the line of one thread.
 """
 from __future__ import annotations
 
@@ -40,9 +40,13 @@ def _steps(g, o, n, where):
 @pytest.mark.parametrize("block,tank", [
     ((1, 1, 2), (5, 4, 6)),       # two particles, a nearly empty warp
     ((3, 7, 11), (9, 7, 13)),     # 231
-    ((17, 13, 19), (30, 14, 21)),  # 4199: a warp each
-    ((25, 8, 25), (31, 9, 27)),   # 5000: the last size of a warp each
-    ((23, 17, 13), (40, 17, 15)),  # 5083: eight lanes each
+    ((10, 15, 20), (14, 16, 22)),  # 3000: the last size of a warp each in FP64
+    ((17, 13, 19), (30, 14, 21)),  # 4199: a warp each in FP32, 16 lanes in FP64
+    ((20, 11, 20), (24, 12, 23)),  # 4400: the last size of a warp each in FP32
+    ((25, 8, 25), (31, 9, 27)),   # 5000: the last size of the one-launch bucket builds
+    ((23, 17, 13), (40, 17, 15)),  # 5083: 16 lanes each
+    ((16, 24, 32), (20, 24, 34)),  # 12288: the last size of 16 lanes each
+    ((23, 23, 24), (28, 24, 26)),  # 12696: eight lanes each
 ])
 def test_odd_scenes_equal_the_oracle(block, tank, prec):
     g, o = _pair(block, tank, prec)
@@ -59,7 +63,7 @@ def test_odd_scenes_equal_the_oracle(block, tank, prec):
 @pytest.mark.parametrize("opts", [
     {L.OPT_DIAG: 1}, {L.OPT_LIST_CAPACITY: 9}, {L.OPT_GRADIENT: L.GRAD_CORRECTED}, {L.OPT_CELL_SKIP: 0},
 ])
-@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13)])
+@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13), (23, 23, 24)])
 def test_options_equal_the_oracle(block, opts):
     tank = tuple(b + 3 for b in block)
     g, o = _pair(block, tank, F32)
@@ -78,7 +82,7 @@ def test_options_equal_the_oracle(block, opts):
         o.close()
 
 
-@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13)])
+@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13), (23, 23, 24)])
 def test_scales_outside_the_fast_arithmetic_equal_the_oracle(block):
     """A spacing below 2^-20 takes the walk of one lane per particle inside the same kernels."""
     tank = tuple(b + 3 for b in block)
@@ -111,7 +115,7 @@ def test_nearly_coincident_particles_equal_the_oracle(shift):
         o.close()
 
 
-@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13)])
+@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13), (23, 23, 24)])
 def test_walls_that_moved_and_stopped_equal_the_oracle(block):
     """Walls at rest are told apart by class; a wall that has moved is not, nor once it stops."""
     l0 = 0.02
@@ -139,7 +143,7 @@ def test_walls_that_moved_and_stopped_equal_the_oracle(block):
 
 
 @pytest.mark.parametrize("prec", [F32, F64])
-@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13)])
+@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13), (23, 23, 24)])
 def test_many_wall_normals_equal_the_oracle(block, prec):
     """A rough plate: 14 normals within reach of a particle, more than a particle registers."""
     l0 = 0.02
@@ -168,7 +172,7 @@ def test_many_wall_normals_equal_the_oracle(block, prec):
 
 @pytest.mark.parametrize("corrected", [0, 1])
 @pytest.mark.parametrize("prec", [F32, F64, F32_N64])
-@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13)])
+@pytest.mark.parametrize("block", [(9, 8, 11), (23, 17, 13), (23, 23, 24)])
 def test_methods_one_by_one_equal_the_oracle(block, prec, corrected):
     """Every method on its own, in the reference's order and then without the bucket builds that
     follow a move: the lists are then older than the positions, and one thread walks them."""
