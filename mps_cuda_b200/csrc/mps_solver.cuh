@@ -957,14 +957,19 @@ template <class R, class RN> class Solver final : public SolverBase {
     //   pass C      97 / 19 / 15     104 / 27 / 31     101 / 47 / 66     103 / 75 / 111    120 / 131
     //   two generations and culls
     //              167 / 79 / 52     211 / 86 / 95     205 / 119 / 151   203 / 139 / 209   198 / 207
-    // and the FP64 crossings to one thread lie at the same sizes. Between a warp and eight lanes,
-    // 16 lanes: a step by graphs, us (a warp / 16 / 8 lanes):
+    // and around the lines to one thread (8 lanes / one thread; B and C share a list, so one line):
+    //              48k particles       63k                80k                95k
+    //   FP32 A     117 / 149           148 / 148          -                  -
+    //   FP64 A     179 / 204           228 / 207          -                  -
+    //   a step, FP32  383 / 497        454 / 496          492 / 495          536 / 527
+    //           FP64  528 / 667        636 / 672          679 / 680          740 / 709
+    // Between a warp and eight lanes, 16 lanes; a step by graphs, us (a warp / 16 / 8 lanes):
     //              2.6k   3.4k  4.0k   4.4k   5.0k particles  6.0k         9.0k      12.5k     19.8k
     //   FP32    120/137 130/137 137/142 146/145 158/154  173/163/177 203/188/192 240/212/213 304/249/245
     //   FP64    134/139 148/140 160/150 174/156 186/169  201/185/199 246/218/224 293/253/265 380/312/315
     static constexpr int kWarpMost = sizeof(R) == 4 ? 4400 : 3000, kHalfMost = 12288,
-                         kGroupMostA = 65536, kGroupMostBC = 98304, kGroupMostGen = 180000,
-                         kCullMost = 600000;
+                         kGroupMostA = sizeof(R) == 4 ? 65536 : 56000, kGroupMostBC = 81920,
+                         kGroupMostGen = 180000, kCullMost = 600000;
     int group_lanes(int most) const {
         return nF <= kWarpMost ? 32 : (nF <= kHalfMost ? 16 : (nF <= most ? 8 : 0));
     }

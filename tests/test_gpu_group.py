@@ -194,3 +194,19 @@ def test_methods_one_by_one_equal_the_oracle(block, prec, corrected):
     finally:
         g.close()
         o.close()
+
+
+@pytest.mark.parametrize("prec", [F32, F64])
+@pytest.mark.parametrize("block", [
+    (40, 35, 40),   # 56000 and 65536: the last sizes of several lanes in pass A, FP64 and FP32
+    (32, 32, 64),
+    (40, 32, 64),   # 81920: the last size of several lanes in passes B and C
+    (43, 41, 47),   # 82861: their lists have the one-thread layout
+])
+def test_the_lines_of_one_thread_equal_the_oracle(block, prec):
+    g, o = _pair(block, tuple(b + 3 for b in block), prec)
+    try:
+        _steps(g, o, 2, block)
+    finally:
+        g.close()
+        o.close()
