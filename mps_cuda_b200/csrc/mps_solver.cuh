@@ -1116,7 +1116,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         CK(cudaStreamSynchronize(stream));
         motion_on = nW > 0 && (hmot[0].type != 0 || hmot[1].type != 0);
         walls_moved = walls_moved || motion_on;
-        if (adj) adj->taped = -1;
+        drop_tape();
         invalidate_graph();
     }
 
@@ -1309,6 +1309,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     // restored afterwards, and the choice is kept for later handles of the same precision
     // and size class in this process (tuned_cache).
     void autotune(int trial, int32_t* chosen) override {
+        drop_tape();
         finish_tail();
         struct CandA { int blk, stage, batch; };
         const CandA cand_a[] = {{128, MPS_STAGE_GLOBAL, 4}, {64, MPS_STAGE_GLOBAL, 4},
@@ -1452,6 +1453,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     // full bucket build and mirror generation when the state was set or changed since.
     void step(int n) override {
         if (n <= 0) return;
+        drop_tape();
         const bool use_graph = graph_on && !timing_on;
         if (gexec_diag != diag_on) invalidate_graph();
         gexec_diag = diag_on;
@@ -1488,6 +1490,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     // One method. The group kernels find a particle's candidates in the rows of its current
     // position, so they serve the methods while no particle has moved since the bucket build.
     void phase(int ph) override {
+        drop_tape();
         finish_tail();
         PassArgs<R, RN> a = args(M1, mcs1);
         const int gb = blocks(nF, block);
@@ -1649,6 +1652,7 @@ template <class R, class RN> class Solver final : public SolverBase {
 
     void set_state(const int8_t* typ, const void* pos, const void* vel, const void* acc,
                    const void* prs, const void* pav) override {
+        drop_tape();
         // start from the current state so that omitted arrays keep their values
         store_all((typ ? 0 : kIoTyp) | (pos ? 0 : kIoPos) | (vel ? 0 : kIoVel) |
                   (acc ? 0 : kIoAcc) | (prs ? 0 : kIoPrs) | (pav ? 0 : kIoPav));
@@ -1818,7 +1822,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         int nsteps = 0, every = 0, nck = 0;
         int nbK = 0;  // list capacity the tape was allocated and recorded with
         long long steps_end = 0;
-        int taped = -1;  // the segment the tape holds, if the handle's walls are still its walls
+        int taped = -1;  // the segment the tape holds, while nothing has changed the handle since
         std::vector<Ckpt> ck;  // nck segment starts + the final state
         std::vector<TapeStep<R>> tape;
         V4<R>* unrm = nullptr;
@@ -1828,6 +1832,12 @@ template <class R, class RN> class Solver final : public SolverBase {
         int *am, *inv2, *err;
     };
     std::unique_ptr<AdjState> adj;
+
+    // Steps, methods, a new state or wall motion: the sweep then replays every segment, which
+    // leaves the mirror tables at the rollout's end as well
+    void drop_tape() {
+        if (adj) adj->taped = -1;
+    }
 
     void snapshot(const Ckpt& c) {
         store_all();

@@ -110,6 +110,11 @@ def test_recording_leaves_the_handle_as_the_same_steps_do(block, tank, every):
             h.step(3)
         same(stepped, taped)
         same(stepped, replayed)
+        # a handle that has moved on since replays the whole rollout, as ever
+        grads = [h.adjoint_backward(lam, lam) for h in (taped, replayed)]
+        for a, b in zip(*grads):
+            assert np.max(np.abs(np.subtract(a, b))) <= 1e-8 * np.max(np.abs(a))
+        same(taped, replayed)
     finally:
         for h in hs:
             h.close()
