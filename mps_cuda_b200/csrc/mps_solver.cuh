@@ -1916,7 +1916,8 @@ template <class R, class RN> class Solver final : public SolverBase {
             throw ApiError(MPS_ERR_ARG, "nsteps and checkpoint_every must be positive");
         every = std::min(every, nsteps);
         const int nck = (nsteps + every - 1) / every;
-        if (!adj || adj->nck != nck || adj->every != every) adj_alloc(nck, every);
+        // the tape's lists hold the capacity they were allocated with, and the recording writes them
+        if (!adj || adj->nck != nck || adj->every != every || adj->nbK != nbK) adj_alloc(nck, every);
         adj->nsteps = 0;
         adj->taped = -1;
         // diagnostics, the kernels' times and staged walks belong to the ordinary step
