@@ -2389,6 +2389,7 @@ __global__ void __launch_bounds__(128) k_gen_cull_g(const __grid_constant__ Pass
                                 m.n[e][gr.g][nn[e]][2] = t.z;
                                 m.id[e][gr.g][nn[e]] = j;
                                 m.code[e][gr.g][nn[e]] = code;
+                                fresh = false;  // a NaN normal does not equal its own entry
                             }
                             ++nn[e];
                         }
