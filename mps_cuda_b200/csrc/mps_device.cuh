@@ -53,21 +53,30 @@ __device__ __forceinline__ int scene_of(const SceneDev<R, RN>* sc, int nscene, i
     return lo;
 }
 
+// float to int toward zero, saturating (NaN: an integer of no meaning)
+__device__ __forceinline__ int to_int(float v) { return __float2int_rz(v); }
+__device__ __forceinline__ int to_int(double v) { return __double2int_rz(v); }
+
 // Bucket coordinates, kernel.cu:521-524. Returns false if the index left the grid (then
-// it is clamped to the interior so that the 27-bucket walk stays inside the grid).
+// it is clamped to the interior so that the 27-bucket walk stays inside the grid). The bounds
+// are applied before the 1 is added: beyond 2^31 buckets the conversion saturates, and the sum
+// would overflow.
 template <class R, class RN>
 __device__ __forceinline__ bool cell_of(const SceneDev<R, RN>& sc, R x, R y, R z, int& ix,
                                         int& iy, int& iz) {
-    ix = int((x - sc.minc[0]) * sc.dbinv) + 1;
-    iy = int((y - sc.minc[1]) * sc.dbinv) + 1;
-    iz = int((z - sc.minc[2]) * sc.dbinv) + 1;
-    bool ok = ix >= 1 && ix <= sc.nbx - 2 && iy >= 1 && iy <= sc.nby - 2 && iz >= 1 &&
-              iz <= sc.nbz - 2;
+    ix = to_int((x - sc.minc[0]) * sc.dbinv);
+    iy = to_int((y - sc.minc[1]) * sc.dbinv);
+    iz = to_int((z - sc.minc[2]) * sc.dbinv);
+    const bool ok = ix >= 0 && ix <= sc.nbx - 3 && iy >= 0 && iy <= sc.nby - 3 && iz >= 0 &&
+                    iz <= sc.nbz - 3;
     if (!ok) {
-        ix = min(max(ix, 1), sc.nbx - 2);
-        iy = min(max(iy, 1), sc.nby - 2);
-        iz = min(max(iz, 1), sc.nbz - 2);
+        ix = min(max(ix, 0), sc.nbx - 3);
+        iy = min(max(iy, 0), sc.nby - 3);
+        iz = min(max(iz, 0), sc.nbz - 3);
     }
+    ++ix;
+    ++iy;
+    ++iz;
     return ok;
 }
 
@@ -106,14 +115,17 @@ template <class R, class RN>
 __device__ __forceinline__ int fine_cell(const SceneDev<R, RN>& sc, R x, R y, R z, bool& ok) {
     const R tx = (x - sc.minc[0]) * sc.dbinv, ty = (y - sc.minc[1]) * sc.dbinv,
             tz = (z - sc.minc[2]) * sc.dbinv;
-    int ix = int(tx) + 1, iy = int(ty) + 1, iz = int(tz) + 1;
-    ok = ix >= 1 && ix <= sc.nbx - 2 && iy >= 1 && iy <= sc.nby - 2 && iz >= 1 && iz <= sc.nbz - 2;
-    ix = min(max(ix, 1), sc.nbx - 2);
-    iy = min(max(iy, 1), sc.nby - 2);
-    iz = min(max(iz, 1), sc.nbz - 2);
-    const int sx = min(max(int(R(3) * tx) + 3, 3 * ix), 3 * ix + 2) - 3 * ix;
-    const int sy = min(max(int(R(3) * ty) + 3, 3 * iy), 3 * iy + 2) - 3 * iy;
-    const int sz = min(max(int(R(3) * tz) + 3, 3 * iz), 3 * iz + 2) - 3 * iz;
+    int ix = to_int(tx), iy = to_int(ty), iz = to_int(tz);
+    ok = ix >= 0 && ix <= sc.nbx - 3 && iy >= 0 && iy <= sc.nby - 3 && iz >= 0 && iz <= sc.nbz - 3;
+    ix = min(max(ix, 0), sc.nbx - 3);
+    iy = min(max(iy, 0), sc.nby - 3);
+    iz = min(max(iz, 0), sc.nbz - 3);
+    const int sx = min(max(to_int(R(3) * tx), 3 * ix), 3 * ix + 2) - 3 * ix;
+    const int sy = min(max(to_int(R(3) * ty), 3 * iy), 3 * iy + 2) - 3 * iy;
+    const int sz = min(max(to_int(R(3) * tz), 3 * iz), 3 * iz + 2) - 3 * iz;
+    ++ix;
+    ++iy;
+    ++iz;
     return sc.fbase + 27 * (iz * sc.nbxy + iy * sc.nbx + ix) + 9 * sz + 3 * sy + sx;
 }
 
