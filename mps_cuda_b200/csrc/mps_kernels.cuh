@@ -40,12 +40,10 @@ template <class R, class RN> struct FluidKeySrc {
         int id = pid[t];
         int s = nscene > 1 ? scene_of(sc, nscene, id) : 0;
         V4<R> p = pos[t];
-        const bool fin = isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
-        if (!fin) atomicAdd(&cnt->err_nan, 1);
+        if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) atomicAdd(&cnt->err_nan, 1);
         bool ok;
         const int c = fine_cell(sc[s], p.x, p.y, p.z, ok);
         if (!ok) atomicAdd(&cnt->err_cell, 1);
-        if (!ok || !fin) cnt->off_grid = 1;
         return c;
     }
     __device__ __forceinline__ int id(int t) const { return pid[t]; }
@@ -1755,7 +1753,11 @@ template <class R, class RN> struct GroupSlot {
     V4<R> p;
     RowCtx<R> c;
     int s, pid, row;
-    bool act;
+    // the group walk does not cover the particle: its position is off the grid or not finite, so
+    // that the box around the set would not bound its rows, or the scene's sizes leave the range
+    // of mps_exact.cuh. One lane walks for it, as the kernels of one thread per particle do; the
+    // other particles of the warp keep their sets.
+    bool off;
 };
 // this group's slot, if it is listed
 template <class R, class RN, int G>
@@ -1767,21 +1769,15 @@ __device__ __forceinline__ GroupSlot<R, RN> group_load(const PassArgs<R, RN>& a,
                                                        const V4<R>* pos) {
     GroupSlot<R, RN> t;
     t.s = s;
-    t.act = act;
     t.pid = act ? a.pid[s] : 0;
     t.sc = &a.sc[act && a.nscene > 1 ? scene_of(a.sc, a.nscene, t.pid) : 0];
     t.p = act ? ldg4(pos + s) : V4<R>{R(0), R(0), R(0), R(0)};
     int ix = 0, iy = 0, iz = 0;
-    if (act) cell_of(*t.sc, t.p.x, t.p.y, t.p.z, ix, iy, iz);
+    t.off = act && !(cell_of(*t.sc, t.p.x, t.p.y, t.p.z, ix, iy, iz) && isfinite(t.p.x) &&
+                     isfinite(t.p.y) && isfinite(t.p.z) && t.sc->pairs_ok);
     t.c = row_ctx(*t.sc, t.p.x, t.p.y, t.p.z, ix, iy, iz);
     t.row = t.sc->cbase + iz * t.sc->nbxy + iy * t.sc->nbx;
     return t;
-}
-// whether the group walk does not cover this slot: a position off the grid, whose rows the union
-// would widen, or a scene whose sizes leave the range of mps_exact.cuh
-template <class R, class RN>
-__device__ __forceinline__ bool group_off(const PassArgs<R, RN>& a, int s) {
-    return a.cnt->off_grid != 0 || !scene_ref(a, a.pid[s]).pairs_ok;
 }
 // the scene of a set (its lanes share their bucket row)
 template <class R, class RN>
@@ -1814,13 +1810,13 @@ __global__ void __launch_bounds__(128) k_pass_a_g(const __grid_constant__ PassAr
     const int s = group_slot<R, RN>(gr);
     bool act = group_act<PHASE>(a, s);
     if (!PHASE && s < a.nF && !act && gr.l == 0) pass_a_unlisted(a, s, TAPE);
-    if (act && group_off(a, s)) {
+    const GroupSlot<R, RN> me = group_load(a, s, act, a.pos);
+    if (me.off) {
         if (gr.l == 0) pass_a_single<R, RN, DIAG, TAPE, PHASE>(a, s);
         act = false;
     }
     unsigned pend = __ballot_sync(kFull, act);
     if (pend == 0u) return;
-    const GroupSlot<R, RN> me = group_load(a, s, act, a.pos);
     const SceneDev<R, RN>& sc = *me.sc;
     const V4<R> p = me.p, v = act ? ldg4(a.vel + s) : p;
     const bool nearm = act && near_flag(a.near_m, sc, me.c);
@@ -1975,13 +1971,13 @@ __global__ void __launch_bounds__(128) k_pass_b_g(const __grid_constant__ PassAr
         a.tvel[s] = a.vel[s];
         a.tprs[s] = R(0);
     }
-    if (act && group_off(a, s)) {
+    const GroupSlot<R, RN> me = group_load(a, s, act, a.pos);
+    if (me.off) {
         if (gr.l == 0) pass_b_single<R, RN, DIAG, MODE>(a, s);
         act = false;
     }
     unsigned pend = __ballot_sync(kFull, act);
     if (pend == 0u) return;
-    const GroupSlot<R, RN> me = group_load(a, s, act, a.pos);
     const SceneDev<R, RN>& sc = *me.sc;
     const V4<R> p = me.p, v = act ? ldg4(a.vel + s) : p;
     const bool nearm = act && near_flag(a.near_m, sc, me.c),
@@ -2143,13 +2139,13 @@ __global__ void __launch_bounds__(128) k_pass_c_g(const __grid_constant__ PassAr
         if (TAPE) a.tape_pre[s] = V4<R>{R(0), R(0), R(0), R(kTapeDead)};
     }
     const int n = !PHASE && act ? a.nbcnt[s] : 0;
-    if (act && (n > a.nbK || group_off(a, s))) {  // the walk over the fine rows: any position
+    const GroupSlot<R, RN> me = group_load(a, s, act, a.pos);
+    if (n > a.nbK || me.off) {  // the walk over the fine rows: any position
         if (gr.l == 0) pass_c_single<R, RN, DIAG, TAPE, CORR, PHASE, GA>(a, s);
         act = false;
     }
     unsigned pend = __ballot_sync(kFull, act);
     if (pend == 0u) return;
-    const GroupSlot<R, RN> me = group_load(a, s, act, a.pos);
     const SceneDev<R, RN>& sc = *me.sc;
     const V4<R> p = me.p;
     const R* __restrict__ prs = PHASE ? a.prs : a.tprs;
@@ -2331,7 +2327,7 @@ __global__ void __launch_bounds__(128) k_gen_cull_g(const __grid_constant__ Pass
     bool act = fld && __ldg(a.near_wall + me.row + me.c.ix);
     const R P = act ? (gprs ? gprs[s] : slot_w(s, R(0))) : R(0);
     int nwall = 0;
-    if (act && group_off(a, s)) {
+    if (act && me.off) {
         if (gr.l == 0) nwall = gen_single<R, RN, TAPE>(a, s, p, P);
         act = false;
     }

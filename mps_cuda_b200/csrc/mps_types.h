@@ -91,8 +91,7 @@ struct DevCounters {
     int scan_ticket;      // blocks of the running fine-cell scan that finished (0 between)
     int stage_blocks;     // blocks of a staged pass that walked shared memory (diagnostics)
     int unstaged_blocks;  // ... and those whose neighbourhood did not fit (diagnostics)
-    int off_grid;         // a bucket build met a listed particle outside the grid (sticky)
-    int pad[4];
+    int pad[5];
     // diagnostics: fluid candidates tested by VscTrm's walk and by the list build of
     // ChkCol/MkPrs, and the entries of those lists
     unsigned long long work[3];
