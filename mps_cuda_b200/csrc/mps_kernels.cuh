@@ -1004,8 +1004,8 @@ __device__ __forceinline__ int build_list(const PassArgs<R, RN>& a, const SceneD
 // coordinates. Every step of the row geometry is monotone in the coordinates, so a box
 // corner is never nearer than a particle inside it and the box range covers each
 // particle's own range for that row. Blocks whose rows do not fit (particles in two bucket
-// rows, more than kStageSpan buckets along x, or more candidates than the staging
-// capacity) walk global memory instead, decided uniformly for the block.
+// rows, more than kStageSpan buckets along x, at no finite place, or more candidates than the
+// staging capacity) walk global memory instead, decided uniformly for the block.
 constexpr int kStageRows = 81;                     // 9 x 9 fine rows
 constexpr int kStageSpan = 8;                      // buckets along x, max - min
 constexpr int kStageCols = 3 * kStageSpan + 10;    // fine cells [3 ix_min - 3, 3 ix_max + 5] + end
@@ -1057,7 +1057,9 @@ __device__ bool stage_fluid(const PassArgs<R, RN>& a, StageHdr& h, V4<R>* spos, 
         atomicMax(&h.box[3], ord_bits(c.ry));
         atomicMin(&h.box[4], ord_bits(c.rz));
         atomicMax(&h.box[5], ord_bits(c.rz));
-        atomicMin(&h.smin, scene);
+        // a NaN lies in no order with the others: the box would not bound their rows
+        const bool ordered = isfinite(c.rx) && isfinite(c.ry) && isfinite(c.rz);
+        atomicMin(&h.smin, ordered ? scene : -1);
         atomicMax(&h.smax, scene);
     }
     __syncthreads();
