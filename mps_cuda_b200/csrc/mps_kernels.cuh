@@ -1756,9 +1756,8 @@ template <class R, class RN> struct GroupSlot {
     RowCtx<R> c;
     int s, pid, row;
     // the group walk does not cover the particle: its position is off the grid or not finite, so
-    // that the box around the set would not bound its rows, or the scene's sizes leave the range
-    // of mps_exact.cuh. One lane walks for it, as the kernels of one thread per particle do; the
-    // other particles of the warp keep their sets.
+    // that the box around the set would not bound its rows. One lane walks for it, as the kernels
+    // of one thread per particle do; the other particles of the warp keep their sets.
     bool off;
 };
 // this group's slot, if it is listed
@@ -1776,7 +1775,7 @@ __device__ __forceinline__ GroupSlot<R, RN> group_load(const PassArgs<R, RN>& a,
     t.p = act ? ldg4(pos + s) : V4<R>{R(0), R(0), R(0), R(0)};
     int ix = 0, iy = 0, iz = 0;
     t.off = act && !(cell_of(*t.sc, t.p.x, t.p.y, t.p.z, ix, iy, iz) && isfinite(t.p.x) &&
-                     isfinite(t.p.y) && isfinite(t.p.z) && t.sc->pairs_ok);
+                     isfinite(t.p.y) && isfinite(t.p.z));
     t.c = row_ctx(*t.sc, t.p.x, t.p.y, t.p.z, ix, iy, iz);
     t.row = t.sc->cbase + iz * t.sc->nbxy + iy * t.sc->nbx;
     return t;

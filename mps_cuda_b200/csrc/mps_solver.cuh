@@ -441,6 +441,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     int nbK = kListCap;                    // list capacity in use (MPS_OPT_LIST_CAPACITY)
     std::vector<int> fluid_ids, wall_ids;
     bool lists_valid = false, sorted = false, m1_valid = false, acc_dirty = false;
+    bool pairs_ok = true;  // of every scene (SceneDev::pairs_ok)
     // Captured graphs of a step's body (passes A to C, moving walls), and of the end of the step
     // before it (mirrors, bucket builds) with the body, one per buffer the sorted state starts in:
     // a fluid bucket build moves the state from S to S2, so a graph's baked pointers fit only the
@@ -587,6 +588,7 @@ template <class R, class RN> class Solver final : public SolverBase {
                 throw ApiError(MPS_ERR_OVERFLOW, "the scenes' fine cell grids need more cells "
                                                  "than an int32 index holds");
             derive_scene<R, RN>(p[s], int(cb), int(fb), pb, cnts[s], hsc[s], infos[s]);
+            pairs_ok = pairs_ok && hsc[s].pairs_ok;
             cb += infos[s].nbxyz;
             fb += 27LL * infos[s].nbxyz;
             pb += cnts[s];
@@ -967,10 +969,13 @@ template <class R, class RN> class Solver final : public SolverBase {
     //              2.6k   3.4k  4.0k   4.4k   5.0k particles  6.0k         9.0k      12.5k     19.8k
     //   FP32    120/137 130/137 137/142 146/145 158/154  173/163/177 203/188/192 240/212/213 304/249/245
     //   FP64    134/139 148/140 160/150 174/156 186/169  201/185/199 246/218/224 293/253/265 380/312/315
+    // Handles with a scene whose sizes leave the range of mps_exact.cuh take one thread per
+    // particle at any size: the group walks are in its arithmetic.
     static constexpr int kWarpMost = sizeof(R) == 4 ? 4400 : 3000, kHalfMost = 12288,
                          kGroupMostA = sizeof(R) == 4 ? 65536 : 56000, kGroupMostBC = 81920,
                          kGroupMostGen = 180000, kCullMost = 600000;
     int group_lanes(int most) const {
+        if (!pairs_ok) return 0;
         return nF <= kWarpMost ? 32 : (nF <= kHalfMost ? 16 : (nF <= most ? 8 : 0));
     }
     int list_layout() const { return group_lanes(kGroupMostBC) ? kListGroup : kListThread; }
