@@ -9,8 +9,15 @@
 //   quotient  y' = y + y (1 - b y), q = a y', q' = q + (a - b q) y' with y ~ 1/b
 // (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
 // IBM J. Res. Dev. 34, 1990: with y' the correctly rounded reciprocal and no overflow or
-// underflow in between, q' is the correctly rounded quotient). tests/test_gpu_exact.py compares
-// them with sqrt() and `/` over every significand of the single-precision root and reciprocal.
+// underflow in between, q' is the correctly rounded quotient).
+//
+// What is shown. Single: the root and the reciprocal by trial of every significand
+// (tests/test_gpu_exact.py), so the quotient by the theorem. Double: a reciprocal within one last
+// place becomes the correctly rounded one by one more step, unless every bit of the divisor's
+// significand is set (also Markstein's); that divisor is set apart, and the quotient follows by the
+// theorem. The double root's last step errs by less than 2^-51 last places, and only operands whose
+// exact root lies nearer than that to the middle of two doubles could round wrongly;
+// tests/test_gpu_exact_hard.py tries all of those, and the quotients nearest to a middle.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -62,8 +69,13 @@ __device__ __forceinline__ float rcp_in(float b) {
 }
 __device__ __forceinline__ double rcp_in(double b) {
     double y = rcp_est(b);
-    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);  // the estimate's 20 bits to 40, then to the last
-    return __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);  // the estimate's 20 bits to 40,
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);  // to half a last place and a little,
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);  // to the nearest double
+    // 1 / (2 - 2^-52) lies just above the middle of 1/2 and the next double, where the step ties
+    const int hi = __double2hiint(b), lo = __double2loint(b);
+    const int tie = ((hi | 0xfff00000) & lo) == -1;
+    return __hiloint2double(__double2hiint(y), __double2loint(y) | tie);
 }
 
 // a / b given y = 1 / b, correctly rounded
