@@ -216,16 +216,15 @@ static void derive_scene(const mps_params& p, int cbase, int fbase, int pbase, i
 // Device memory of a handle or of a recorded rollout. A set-up that takes many arrays runs its
 // gets twice, inside plan(): once to add up their sizes, then out of one allocation. The tape of
 // 20 recorded steps of 48 000 particles in FP64 is some 370 arrays of 2.8 GB: one by one 106 ms to
-// allocate and 100 ms to free, at once under 1 and 3 ms; a handle of 48 000 particles in FP32 takes
-// 8.2 and 6.4 ms to create and destroy with one allocation an array, 1.1 and 0.5 at once. Small
-// sets stay apart: the driver serves small requests from blocks that it keeps (480 particles:
-// 0.9 ms either way). A get outside plan() is an allocation of its own.
+// allocate and 100 ms to free, at once under 1 and 3 ms. A handle, us to create / to destroy, with
+// an allocation an array / at once: 480 particles (1.5 MB) 842 / 617, 757 / 413; 3 528 1838 / 1415,
+// 749 / 392; 6 000 2241 / 1658, 813 / 397; 48 000 8200 / 6400, 1140 / 460. A get outside plan() is
+// an allocation of its own.
 struct DevArena {
     std::vector<void*> ptrs;
     bool measuring = false;
     char *next = nullptr, *end = nullptr;  // what is left of the planned allocation
     size_t total = 0;
-    static constexpr size_t kAtOnce = size_t(16) << 20;
     static size_t rounded(size_t bytes) { return (bytes + 255) / 256 * 256; }
     void* allocate(size_t bytes) {
         void* p = nullptr;
@@ -256,10 +255,8 @@ struct DevArena {
         total = 0;
         gets();
         measuring = false;
-        if (total >= kAtOnce) {
-            next = static_cast<char*>(allocate(total));
-            end = next + total;
-        }
+        next = static_cast<char*>(allocate(total));
+        end = next + total;
         gets();
         next = end = nullptr;
     }

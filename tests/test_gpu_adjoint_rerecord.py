@@ -17,9 +17,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("first,second", [(8, 0), (0, 64), (64, 160)])
 @pytest.mark.parametrize("block,tank,every", [
-    ((8, 6, 10), (20, 10, 20), 4),     # every array an allocation of its own
+    ((8, 6, 10), (20, 10, 20), 4),     # a warp per particle
     ((8, 6, 10), (20, 10, 20), 3),     # two segments
-    ((23, 17, 13), (40, 17, 15), 4),   # one allocation for all
+    ((23, 17, 13), (40, 17, 15), 4),   # 16 lanes per particle
 ])
 def test_recording_again_after_a_capacity_change(block, tank, every, first, second):
     l0, n = 0.02, 4
