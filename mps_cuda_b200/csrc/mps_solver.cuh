@@ -966,16 +966,26 @@ template <class R, class RN> class Solver final : public SolverBase {
     //              2.6k   3.4k  4.0k   4.4k   5.0k particles  6.0k         9.0k      12.5k     19.8k
     //   FP32    120/137 130/137 137/142 146/145 158/154  173/163/177 203/188/192 240/212/213 304/249/245
     //   FP64    134/139 148/140 160/150 174/156 186/169  201/185/199 246/218/224 293/253/265 380/312/315
+    // The generation shares the line of B and C. It runs beside another kernel, so the step decides:
+    // eight lanes in the generation alone shorten its launches up to 180 000 particles of a column,
+    // and make the step longer wherever B and C run one thread per particle (112 000 and 180 000 in a
+    // column 560 / 534 and 682 / 640 us with eight lanes / one thread, batches of 102 000 and 203 000
+    // 687 / 600 and 1044 / 876, in FP64 985 / 907 and 1568 / 1399). The more of a scene lies at walls,
+    // the earlier one thread wins, and the line lies between. A step by graphs, us (eight lanes / one
+    // thread in B, C and the generation):
+    //            column, 72k     79k        91k        thin column, 70k  79k        batches, 62k  75k        85k
+    //   FP32     470 / 502       479 / 496  525 / 528  523 / 504         568 / 520  531 / 543     578 / 557  626 / 568
+    //   FP64     634 / 676       650 / 668  716 / 712  725 / 692         785 / 713  709 / 723     792 / 752  863 / 789
     // Handles with a scene whose sizes leave the range of mps_exact.cuh take one thread per
     // particle at any size: the group walks are in its arithmetic.
     static constexpr int kWarpMost = sizeof(R) == 4 ? 4400 : 3000, kHalfMost = 12288,
-                         kGroupMostA = sizeof(R) == 4 ? 65536 : 56000, kGroupMostBC = 81920,
-                         kGroupMostGen = 180000, kCullMost = 600000;
+                         kGroupMostA = sizeof(R) == 4 ? 65536 : 56000, kGroupMost = 73728,
+                         kCullMost = 600000;
     int group_lanes(int most) const {
         if (!pairs_ok) return 0;
         return nF <= kWarpMost ? 32 : (nF <= kHalfMost ? 16 : (nF <= most ? 8 : 0));
     }
-    int list_layout() const { return group_lanes(kGroupMostBC) ? kListGroup : kListThread; }
+    int list_layout() const { return group_lanes(kGroupMost) ? kListGroup : kListThread; }
     int group_grid(int g) const { return blocks(nF, 128 / g); }
 
     // pass A, with the mirror table that `a` names
@@ -996,7 +1006,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         KL();
     }
     template <bool D> void run_pass_b(const PassArgs<R, RN>& a, int bb) {
-        const int g = group_lanes(kGroupMostBC);
+        const int g = group_lanes(kGroupMost);
         if (g == 32)
             k_pass_b_g<R, RN, D, 32><<<group_grid(32), 128, 0, stream>>>(a);
         else if (g == 16)
@@ -1010,7 +1020,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         KL();
     }
     template <bool D, bool TAPE> void run_pass_c(const PassArgs<R, RN>& a, int bc) {
-        const int g = group_lanes(kGroupMostBC);
+        const int g = group_lanes(kGroupMost);
         const bool corr = !TAPE && grad_mode == MPS_GRAD_CORRECTED;
         if (g == 32 && corr)
             k_pass_c_g<R, RN, D, false, true, 32><<<group_grid(32), 128, 0, stream>>>(a);
@@ -1035,7 +1045,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     template <bool D, bool TAPE, bool CLS>
     void launch_gen_cls(const PassArgs<R, RN>& a, int bg, const V4<R>* pos, const R* prs,
                         const int8_t* typ) {
-        const int g = group_lanes(kGroupMostGen);
+        const int g = group_lanes(kGroupMost);
         if (g == 32)
             k_gen_cull_g<R, RN, D, TAPE, CLS, 32><<<group_grid(32), 128, 0, stream>>>(a, pos, prs, typ);
         else if (g == 16)
@@ -1554,11 +1564,11 @@ template <class R, class RN> class Solver final : public SolverBase {
             case MPS_PHASE_CHKCOL:
                 need_lists();
                 if (diag_on) k_ph_col<R, RN, true><<<gb, block, 0, stream>>>(a);
-                else if (lanes(kGroupMostBC) == 32)
+                else if (lanes(kGroupMost) == 32)
                     k_pass_b_g<R, RN, false, 32, PASS_COL><<<group_grid(32), 128, 0, stream>>>(a);
-                else if (lanes(kGroupMostBC) == 16)
+                else if (lanes(kGroupMost) == 16)
                     k_pass_b_g<R, RN, false, 16, PASS_COL><<<group_grid(16), 128, 0, stream>>>(a);
-                else if (lanes(kGroupMostBC) == 8)
+                else if (lanes(kGroupMost) == 8)
                     k_pass_b_g<R, RN, false, 8, PASS_COL><<<group_grid(8), 128, 0, stream>>>(a);
                 else k_ph_col<R, RN, false><<<gb, block, 0, stream>>>(a);
                 KL();
@@ -1569,19 +1579,19 @@ template <class R, class RN> class Solver final : public SolverBase {
             case MPS_PHASE_MKPRS:
                 need_lists();
                 if (diag_on) k_ph_prs<R, RN, true><<<gb, block, 0, stream>>>(a);
-                else if (lanes(kGroupMostBC) == 32)
+                else if (lanes(kGroupMost) == 32)
                     k_pass_b_g<R, RN, false, 32, PASS_PRS><<<group_grid(32), 128, 0, stream>>>(a);
-                else if (lanes(kGroupMostBC) == 16)
+                else if (lanes(kGroupMost) == 16)
                     k_pass_b_g<R, RN, false, 16, PASS_PRS><<<group_grid(16), 128, 0, stream>>>(a);
-                else if (lanes(kGroupMostBC) == 8)
+                else if (lanes(kGroupMost) == 8)
                     k_pass_b_g<R, RN, false, 8, PASS_PRS><<<group_grid(8), 128, 0, stream>>>(a);
                 else k_ph_prs<R, RN, false><<<gb, block, 0, stream>>>(a);
                 KL();
                 break;
             case MPS_PHASE_PRSGRDTRM:
                 need_lists();
-                if (grad_mode == MPS_GRAD_CORRECTED) run_ph_grd<true>(a, gb, lanes(kGroupMostBC));
-                else run_ph_grd<false>(a, gb, lanes(kGroupMostBC));
+                if (grad_mode == MPS_GRAD_CORRECTED) run_ph_grd<true>(a, gb, lanes(kGroupMost));
+                else run_ph_grd<false>(a, gb, lanes(kGroupMost));
                 KL();
                 acc_dirty = true;
                 break;
@@ -2052,7 +2062,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     // all sizes)
     void back_step(const TapeStep<R>& t) {
         if (nF <= 5000) back_step_lanes<32>(t);
-        else if (nF <= kGroupMostBC) back_step_lanes<16>(t);
+        else if (nF <= kGroupMost) back_step_lanes<16>(t);
         else back_step_lanes<4>(t);
     }
     template <int G> void back_step_lanes(const TapeStep<R>& t) {
