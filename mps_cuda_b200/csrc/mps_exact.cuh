@@ -3,7 +3,7 @@
 // The step's pair terms need IEEE square roots and quotients (kernel.cu:1062-1064, 1346-1348,
 // 1731-1735). sqrt() and `/` pay for the whole range of their type: scaling, special values and
 // a branch to a slow path in every pair. A pair's operands lie in a narrow range that is checked
-// once (DivRange below), and inside it a hardware estimate, one Newton step and one residual
+// once (SceneDev::pair_lo), and inside it a hardware estimate, one Newton step and one residual
 // step in fused multiply-adds round correctly:
 //   root      g = x y, g' = g + (x - g^2) y / 2 with y ~ 1/sqrt(x)
 //   quotient  y' = y + y (1 - b y), q = a y', q' = q + (a - b q) y' with y ~ 1/b
@@ -12,11 +12,14 @@
 // underflow in between, q' is the correctly rounded quotient).
 //
 // What is shown. Single: the root and the reciprocal by trial of every significand
-// (tests/test_gpu_exact.py), so the quotient by the theorem. Double: a reciprocal within one last
-// place becomes the correctly rounded one by one more step, unless every bit of the divisor's
-// significand is set (also Markstein's); that divisor is set apart, and the quotient follows by the
-// theorem. The double root's last step errs by less than 2^-51 last places, and only operands whose
-// exact root lies nearer than that to the middle of two doubles could round wrongly;
+// (tests/test_gpu_exact.py), so the quotient by the theorem. Double, with 1 <= b < 2: a reciprocal y
+// within 0.6 last places of 1/b becomes the nearest double by one more step, which before it rounds
+// is short of 1/b by (1 - b y)^2 / b < 1.5 2^-106 / b. A middle m of two doubles has
+// b m = 1 + j 2^-106 with an integer j other than 0, so it lies at least 2^-106 / b from 1/b, and
+// only j = -1 could make the step round wrongly. The significands of b and m, as integers, then
+// multiply to 2^106 - 1, which has one divisor of 53 bits: 2^53 - 1. That divisor b is set apart,
+// and the quotient follows by the theorem. The double root's last step errs by less than 2^-51 last
+// places, and only operands whose exact root lies nearer than that to a middle could round wrongly;
 // tests/test_gpu_exact_hard.py tries all of those, and the quotients nearest to a middle.
 #pragma once
 #include <cuda_runtime.h>
@@ -69,8 +72,8 @@ __device__ __forceinline__ float rcp_in(float b) {
 }
 __device__ __forceinline__ double rcp_in(double b) {
     double y = rcp_est(b);
-    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);  // the estimate's 20 bits to 40,
-    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);  // to half a last place and a little,
+    const double e = __fma_rn(-b, y, 1.0);
+    y = __fma_rn(y, __fma_rn(e, e, e), y);     // y (1 + e + e^2): the estimate's 20 bits to 0.6 places
     y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);  // to the nearest double
     // 1 / (2 - 2^-52) lies just above the middle of 1/2 and the next double, where the step ties
     const int hi = __double2hiint(b), lo = __double2loint(b);
