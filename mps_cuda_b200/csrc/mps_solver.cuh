@@ -966,21 +966,24 @@ template <class R, class RN> class Solver final : public SolverBase {
     //              2.6k   3.4k  4.0k   4.4k   5.0k particles  6.0k         9.0k      12.5k     19.8k
     //   FP32    120/137 130/137 137/142 146/145 158/154  173/163/177 203/188/192 240/212/213 304/249/245
     //   FP64    134/139 148/140 160/150 174/156 186/169  201/185/199 246/218/224 293/253/265 380/312/315
-    // The generation shares the line of B and C. It runs beside another kernel, so the step decides:
-    // eight lanes in the generation alone shorten its launches up to 180 000 particles of a column,
-    // and make the step longer wherever B and C run one thread per particle (112 000 and 180 000 in a
-    // column 560 / 534 and 682 / 640 us with eight lanes / one thread, batches of 102 000 and 203 000
-    // 687 / 600 and 1044 / 876, in FP64 985 / 907 and 1568 / 1399). The more of a scene lies at walls,
-    // the earlier one thread wins, and the line lies between. A step by graphs, us (eight lanes / one
-    // thread in B, C and the generation):
+    // The generation shares the line of B and C where it runs beside other kernels, on the second
+    // stream: eight lanes shorten its launches up to 140 000 particles of a column, but make the step
+    // longer wherever B and C run one thread per particle (112 000 and 180 000 in a column 560 / 534
+    // and 682 / 640 us with eight lanes / one thread in the generation, batches of 102 000 and 203 000
+    // 687 / 600 and 1044 / 876, in FP64 985 / 907 and 1568 / 1399). By itself, after an upload or in the
+    // reference's sequence of methods, it takes eight lanes up to 112 640 (a generation and cull of
+    // 110 000 particles in a wide, a flat and a thin column 72 / 78, 83 / 79 and 108 / 89 us).
+    // The more of a scene lies at walls, the earlier one thread wins; the line is a wide column's,
+    // whose methods one by one also take 814 us with eight lanes at 76 000 particles, 908 with one
+    // thread. A step by graphs, us (eight lanes / one thread in B, C and the generation):
     //            column, 72k     79k        91k        thin column, 70k  79k        batches, 62k  75k        85k
     //   FP32     470 / 502       479 / 496  525 / 528  523 / 504         568 / 520  531 / 543     578 / 557  626 / 568
     //   FP64     634 / 676       650 / 668  716 / 712  725 / 692         785 / 713  709 / 723     792 / 752  863 / 789
     // Handles with a scene whose sizes leave the range of mps_exact.cuh take one thread per
     // particle at any size: the group walks are in its arithmetic.
     static constexpr int kWarpMost = sizeof(R) == 4 ? 4400 : 3000, kHalfMost = 12288,
-                         kGroupMostA = sizeof(R) == 4 ? 65536 : 56000, kGroupMost = 73728,
-                         kCullMost = 600000;
+                         kGroupMostA = sizeof(R) == 4 ? 65536 : 56000, kGroupMost = 81920,
+                         kGroupMostAlone = 112640, kCullMost = 600000;
     int group_lanes(int most) const {
         if (!pairs_ok) return 0;
         return nF <= kWarpMost ? 32 : (nF <= kHalfMost ? 16 : (nF <= most ? 8 : 0));
@@ -1045,7 +1048,7 @@ template <class R, class RN> class Solver final : public SolverBase {
     template <bool D, bool TAPE, bool CLS>
     void launch_gen_cls(const PassArgs<R, RN>& a, int bg, const V4<R>* pos, const R* prs,
                         const int8_t* typ) {
-        const int g = group_lanes(kGroupMost);
+        const int g = group_lanes(stream == side ? kGroupMost : kGroupMostAlone);
         if (g == 32)
             k_gen_cull_g<R, RN, D, TAPE, CLS, 32><<<group_grid(32), 128, 0, stream>>>(a, pos, prs, typ);
         else if (g == 16)

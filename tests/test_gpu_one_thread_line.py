@@ -1,6 +1,6 @@
-"""The sizes on both sides of the line from eight lanes per particle to one thread in ChkCol/MkPrs,
-PrsGrdTrm and mirror generation, in one scene and in a batch, against the CPU oracle; and what a step
-of a batch costs across that line.
+"""Batches on both sides of the line from eight lanes per particle to one thread in ChkCol/MkPrs,
+PrsGrdTrm and mirror generation, against the CPU oracle; the sequence of methods on both sides of its
+line for mirror generation; and what a step of a batch costs across the first line.
 """
 from __future__ import annotations
 
@@ -9,7 +9,7 @@ import time
 import numpy as np
 import pytest
 
-from mps_cuda_b200 import F32, F32_N64, F64, MPS, MPSBatch, SceneDesc, configs, dambreak, dambreak_params
+from mps_cuda_b200 import F32, F64, MPS, MPSBatch, SceneDesc, configs, dambreak, dambreak_params
 from mps_cuda_b200 import _lib as L
 from oracle.oracle import Oracle, params_from
 
@@ -32,29 +32,10 @@ def _batch(scenes):
     return MPSBatch([p for p, _ in scenes], *join, counts=[a[0].size for _, a in scenes])
 
 
-@pytest.mark.parametrize("prec", [F32, F64, F32_N64])
-@pytest.mark.parametrize("block", [
-    (48, 32, 48),  # 73728: the last size of eight lanes
-    (37, 53, 38),  # 74518: one thread
-])
-def test_one_scene_equals_the_oracle(block, prec):
-    p, args = _scene(block, prec)
-    g, o = MPS(p, *args), Oracle(params_from(p), *args)
-    try:
-        g.step(2)
-        o.step(2)
-        a, b = g.state(), o.state()
-        for k in FIELDS:
-            assert np.array_equal(a[k], b[k]), k
-    finally:
-        g.close()
-        o.close()
-
-
 @pytest.mark.parametrize("prec", [F32, F64])
 @pytest.mark.parametrize("blocks", [
-    [(24, 32, 48), (1, 1, 1), (24, 32, 48), (7, 9, 11)],  # 74422 in all: one thread
-    [(24, 32, 48), (31, 29, 41), (1, 1, 5)],  # 73728: eight lanes
+    [(32, 32, 40), (31, 33, 40), (1, 1, 40)],             # 81920 in all: eight lanes
+    [(32, 32, 40), (1, 1, 1), (32, 32, 40), (7, 9, 11)],  # 82614: one thread
 ])
 def test_a_batch_equals_the_oracles(blocks, prec):
     scenes = [_scene(b, prec, seed=3 + i) for i, b in enumerate(blocks)]
@@ -72,6 +53,25 @@ def test_a_batch_equals_the_oracles(blocks, prec):
             at += n
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("prec", [F32, F64])
+@pytest.mark.parametrize("block", [
+    (40, 44, 64),  # 112640: the last size of eight lanes where mirror generation runs by itself
+    (43, 47, 56),  # 113176
+])
+def test_the_methods_equal_the_oracle(block, prec):
+    p, args = _scene(block, prec)
+    g, o = MPS(p, *args), Oracle(params_from(p), *args)
+    try:
+        g.step_by_methods()
+        o.step(1)
+        a, b = g.state(), o.state()
+        for k in FIELDS:
+            assert np.array_equal(a[k], b[k]), k
+    finally:
+        g.close()
+        o.close()
 
 
 def test_a_batch_beyond_the_line_steps_with_one_thread_throughout():
