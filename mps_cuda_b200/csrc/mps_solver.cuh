@@ -19,6 +19,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/mps_b200.h"
@@ -368,14 +369,14 @@ struct mps_handle {
 
 namespace mps {
 
-// Choices of the autotuner, kept per (precision, batched, log2 of the fluid count) for the
-// life of the process: a handle created later in the same class starts from them.
+// Choices of the autotuner, kept per (precision, batched, log2 of the fluid count, lanes per
+// particle of pass A and of the other passes) for the life of the process: a handle created
+// later in the same class starts from them.
 struct TuneKey {
-    int precision, batched, size_class;
+    int precision, batched, size_class, lanes_a, lanes_bc;
     bool operator<(const TuneKey& o) const {
-        if (precision != o.precision) return precision < o.precision;
-        if (batched != o.batched) return batched < o.batched;
-        return size_class < o.size_class;
+        return std::tie(precision, batched, size_class, lanes_a, lanes_bc) <
+               std::tie(o.precision, o.batched, o.size_class, o.lanes_a, o.lanes_bc);
     }
 };
 struct Tuned {
@@ -1048,7 +1049,8 @@ template <class R, class RN> class Solver final : public SolverBase {
     template <bool D, bool TAPE, bool CLS>
     void launch_gen_cls(const PassArgs<R, RN>& a, int bg, const V4<R>* pos, const R* prs,
                         const int8_t* typ) {
-        const int g = group_lanes(stream == side ? kGroupMost : kGroupMostAlone);
+        // steps timed per kernel group run on one stream the kernels that they run on two
+        const int g = group_lanes(stream == side || timing_on ? kGroupMost : kGroupMostAlone);
         if (g == 32)
             k_gen_cull_g<R, RN, D, TAPE, CLS, 32><<<group_grid(32), 128, 0, stream>>>(a, pos, prs, typ);
         else if (g == 16)
@@ -1319,6 +1321,8 @@ template <class R, class RN> class Solver final : public SolverBase {
     //   passes B, C and mirror generation: 128, 96, 64 or 32 threads per block;
     //   then passes B, C and A at their alternate register bound, with the chosen shapes
     //   (pass A with each candidate batch).
+    // A kernel with several lanes per particle has one shape: there is nothing to try but pass A's
+    // against the staged walk.
     // All groups are timed in the same trial steps (they are separate kernels), and every
     // round starts from the handle's state (restored from a snapshot). The state is
     // restored afterwards, and the choice is kept for later handles of the same precision
@@ -1330,8 +1334,10 @@ template <class R, class RN> class Solver final : public SolverBase {
         const CandA cand_a[] = {{128, MPS_STAGE_GLOBAL, 4}, {64, MPS_STAGE_GLOBAL, 4},
                                 {128, MPS_STAGE_GLOBAL, 2}, {64, MPS_STAGE_GLOBAL, 2},
                                 {128, MPS_STAGE_GLOBAL, 8}, {128, MPS_STAGE_POSITIONS, 4}};
+        const CandA cand_a_lanes[] = {{128, MPS_STAGE_GLOBAL, 4}, {128, MPS_STAGE_POSITIONS, 4}};
         const int cand_b[] = {128, 96, 64, 32};
         const int groups_b[] = {MPS_K_PASS_B, MPS_K_PASS_C, MPS_K_GEN};
+        const bool shape_a = !group_lanes(kGroupMostA), shape_b = !group_lanes(kGroupMost);
         double best[MPS_K_COUNT];
         int bestb[MPS_K_COUNT];
         for (int k = 0; k < MPS_K_COUNT; ++k) { best[k] = 1e300; bestb[k] = blk[k]; }
@@ -1343,12 +1349,13 @@ template <class R, class RN> class Solver final : public SolverBase {
         timing_on = true;
         invalidate_graph();
         timing(0, nullptr, nullptr, true);
-        const int nround = int(sizeof(cand_a) / sizeof(cand_a[0]));
+        const int nround = shape_a ? 6 : 2;
         for (int i = 0; i < nround; ++i) {
-            blk[MPS_K_PASS_A] = cand_a[i].blk;
-            stage_mode = cand_a[i].stage;
-            batch_a = cand_a[i].batch;
-            const bool new_b = i < 4;
+            const CandA& ca = shape_a ? cand_a[i] : cand_a_lanes[i];
+            blk[MPS_K_PASS_A] = ca.blk;
+            stage_mode = ca.stage;
+            batch_a = ca.batch;
+            const bool new_b = shape_b && i < 4;
             if (new_b)
                 for (int g : groups_b) blk[g] = cand_b[i];
             // every candidate runs the same steps from the snapshot (a dam break's steps
@@ -1365,9 +1372,9 @@ template <class R, class RN> class Solver final : public SolverBase {
             read(MPS_K_PASS_A, ms);
             if (ms < best[MPS_K_PASS_A]) {
                 best[MPS_K_PASS_A] = ms;
-                bestb[MPS_K_PASS_A] = cand_a[i].blk;
-                best_stage = cand_a[i].stage;
-                best_batch = cand_a[i].batch;
+                bestb[MPS_K_PASS_A] = ca.blk;
+                best_stage = ca.stage;
+                best_batch = ca.batch;
             }
             if (new_b)
                 for (int g : groups_b) {
@@ -1386,14 +1393,14 @@ template <class R, class RN> class Solver final : public SolverBase {
         int regb = 0;
         const int chosen_batch = batch_a;
         const int batches[3] = {chosen_batch, chosen_batch == 2 ? 4 : 2, chosen_batch == 8 ? 4 : 8};
-        for (int r = 0; r < 3; ++r) {
+        for (int r = 0; r < (shape_a ? 3 : 0); ++r) {
             reg_bound = 7;
             batch_a = batches[r];
             load_fluid(true);
             step(trial);
             double ms = 0;
             long long n = 0;
-            if (r == 0) {
+            if (r == 0 && shape_b) {
                 timing(MPS_K_PASS_B, &ms, &n, false);
                 if (n > 0 && ms / n < best[MPS_K_PASS_B]) regb |= 1;
                 ms = 0;
@@ -1425,11 +1432,12 @@ template <class R, class RN> class Solver final : public SolverBase {
     }
 
     // size class of the handle for the tuning cache: precision, batched or not, log2 of the
-    // fluid count
+    // fluid count, and which kernels it runs
     TuneKey tune_key() const {
         int lg = 0;
         while ((2LL << lg) <= (long long)std::max(nF, 1)) ++lg;
-        return TuneKey{precision, nscene > 1 ? 1 : 0, lg};
+        return TuneKey{precision, nscene > 1 ? 1 : 0, lg, group_lanes(kGroupMostA),
+                       group_lanes(kGroupMost)};
     }
 
     int list_capacity() const override { return nbK; }
