@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <array>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <limits>
@@ -1852,7 +1853,7 @@ template <class R, class RN> class Solver final : public SolverBase {
         V4<double> *lx, *lv, *lx_acc, *lG, *lvv, *lxs, *lx_at, *lxs_pid, *lu_pid, *la, *lxa, *lva;
         double *lP, *lP_at, *lkn, *stage;
         R* pmin;
-        int *am, *inv2, *err;
+        int *am, *inv2, *err, *errs;
     };
     std::unique_ptr<AdjState> adj;
 
@@ -1920,6 +1921,7 @@ template <class R, class RN> class Solver final : public SolverBase {
             st->am = a.template get<int>(F);
             st->inv2 = a.template get<int>(T);
             st->err = a.template get<int>(1);
+            st->errs = a.template get<int>(4);
         });
         st->nck = nck;
         st->every = every;
@@ -1982,14 +1984,23 @@ template <class R, class RN> class Solver final : public SolverBase {
         return a;
     }
 
-    // the first mirror generation of a taped segment, as prepare_fused makes it
+    // the first mirror generation of a taped segment, as prepare_fused makes it. Where the handle has
+    // made that generation already, this one adds the normals and leaves the error counters alone.
     void tape_prepare(const TapeStep<R>& t) {
         if (!lists_valid || !sorted) mkbkt(acc_dirty);
         if (acc_dirty) clear_acc();
+        const bool again = m1_valid;
+        static_assert(offsetof(DevCounters, err_nan) - offsetof(DevCounters, err_mirror_slot) == 3 * sizeof(int),
+                      "the four error counters lie side by side");
+        int* const errs = &cnt->err_mirror_slot;
+        if (again)
+            CK(cudaMemcpyAsync(adj->errs, errs, 4 * sizeof(int), cudaMemcpyDeviceToDevice, stream));
         reset_raw();
         PassArgs<R, RN> a = tape_args(M1.pos, M1.slot, mcs1, nb, nbcnt, nullptr);
         run_gen<false, true>(a, block, S.pos, S.prs, S.typ);
         bin_mirrors_n(t.m1pos, t.m1slot, t.m1nrm, t.mcs1);
+        if (again)
+            CK(cudaMemcpyAsync(errs, adj->errs, 4 * sizeof(int), cudaMemcpyDeviceToDevice, stream));
     }
 
     // What follows a taped segment: its end with the mirrors in M1, nothing (another segment is
