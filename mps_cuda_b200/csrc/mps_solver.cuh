@@ -218,15 +218,17 @@ static void derive_scene(const mps_params& p, int cbase, int fbase, int pbase, i
 // Device memory of a handle or of a recorded rollout. A set-up that takes many arrays runs its
 // gets twice, inside plan(): once to add up their sizes, then out of one allocation. The tape of
 // 20 recorded steps of 48 000 particles in FP64 is some 370 arrays of 2.8 GB: one by one 106 ms to
-// allocate and 100 ms to free, at once under 1 and 3 ms. A handle, us to create / to destroy, with
-// an allocation an array / at once: 480 particles (1.5 MB) 842 / 617, 757 / 413; 3 528 1838 / 1415,
-// 749 / 392; 6 000 2241 / 1658, 813 / 397; 48 000 8200 / 6400, 1140 / 460. A get outside plan() is
-// an allocation of its own.
+// allocate and 100 ms to free, at once under 1 and 3 ms. A handle beside another one, us to create /
+// to close, with an allocation an array / at once: 3 528 particles in FP32 (7.4 MB) 980 + 690 /
+// 770 + 395, 6 000 1020 + 684 / 815 + 400, 48 000 8200 + 6400 / 1140 + 460. Small sets stay apart,
+// as the driver serves small requests from blocks that it keeps: 2 016 in FP64 (6.3 MB) 583 + 380 /
+// 780 + 400, 480 512 + 345 / 740 + 390. A get outside plan() is an allocation of its own.
 struct DevArena {
     std::vector<void*> ptrs;
     bool measuring = false;
     char *next = nullptr, *end = nullptr;  // what is left of the planned allocation
     size_t total = 0;
+    static constexpr size_t kAtOnce = size_t(13) << 19;
     static size_t rounded(size_t bytes) { return (bytes + 255) / 256 * 256; }
     void* allocate(size_t bytes) {
         void* p = nullptr;
@@ -257,8 +259,10 @@ struct DevArena {
         total = 0;
         gets();
         measuring = false;
-        next = static_cast<char*>(allocate(total));
-        end = next + total;
+        if (total >= kAtOnce) {
+            next = static_cast<char*>(allocate(total));
+            end = next + total;
+        }
         gets();
         next = end = nullptr;
     }
