@@ -22,7 +22,15 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmps_b200.so")
 SOURCES = ["mps_api.cu", "mps_inst_f32.cu", "mps_inst_f64.cu", "mps_inst_mix.cu",
            "mps_noalloc.cu", "mps_scene.cpp", "mps_io.cpp", "mps_output.cu", "mps_peaks.cu"]
-HEADERS = ["mps_types.h", "mps_exact.cuh", "mps_device.cuh", "mps_group.cuh", "mps_kernels.cuh", "mps_adjoint.cuh", "mps_solver.cuh"]
+HEADERS = ["mps_types.h", "mps_exact.cuh", "mps_device.cuh", "mps_group.cuh", "mps_kernels.cuh",
+           "mps_lanes.cuh", "mps_adjoint.cuh", "mps_solver.cuh"]
+# the kernels with several lanes per particle: one unit for each precision and number of lanes
+LANES = [(f"mps_lanes_{name}_{lanes}", ["-DMPS_REAL=" + real, "-DMPS_DENSITY=" + density,
+                                        f"-DMPS_LANES={lanes}"])
+         for name, real, density in (("f32", "float", "float"), ("f64", "double", "double"),
+                                     ("mix", "float", "double"))
+         for lanes in (32, 16, 8)]
+UNITS = [(src, src, []) for src in SOURCES] + [("mps_lanes.cu", name, d) for name, d in LANES]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -34,7 +42,7 @@ def nvcc_path() -> str:
 
 
 def _inputs():
-    files = [os.path.join(CSRC, f) for f in SOURCES + HEADERS]
+    files = [os.path.join(CSRC, f) for f in SOURCES + ["mps_lanes.cu"] + HEADERS]
     files.append(os.path.join(ROOT, "include", "mps_b200.h"))
     files.append(os.path.abspath(__file__))
     return files
@@ -59,15 +67,15 @@ def build(force: bool = False, verbose: bool = False, extra: list[str] | None = 
     objdir = os.path.join(HERE, "_build")
     os.makedirs(objdir, exist_ok=True)
     procs = []
-    for src in SOURCES:
-        obj = os.path.join(objdir, src + ".o")
-        cmd = [nvcc, *ARCH, *COMMON, "-Xptxas", "-warn-spills", "-c", os.path.join(CSRC, src),
-               "-o", obj]
+    for src, name, defines in UNITS:
+        obj = os.path.join(objdir, name + ".o")
+        cmd = [nvcc, *ARCH, *COMMON, *defines, "-Xptxas", "-warn-spills", "-c",
+               os.path.join(CSRC, src), "-o", obj]
         if extra:
             cmd += extra
         if verbose:
             print(" ".join(cmd), file=sys.stderr)
-        procs.append((src, obj, subprocess.Popen(cmd, cwd=CSRC, stdout=subprocess.PIPE,
+        procs.append((name, obj, subprocess.Popen(cmd, cwd=CSRC, stdout=subprocess.PIPE,
                                                  stderr=subprocess.STDOUT, text=True)))
     objs, errors = [], []
     for src, obj, pr in procs:

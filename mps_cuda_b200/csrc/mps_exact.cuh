@@ -77,7 +77,7 @@ __device__ __forceinline__ double rcp_in(double b) {
     y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);  // to the nearest double
     // 1 / (2 - 2^-52) lies just above the middle of 1/2 and the next double, where the step ties
     const int hi = __double2hiint(b), lo = __double2loint(b);
-    const int tie = ((hi | 0xfff00000) & lo) == -1;
+    const int tie = ((hi | int(0xfff00000u)) & lo) == -1;
     return __hiloint2double(__double2hiint(y), __double2loint(y) | tie);
 }
 

@@ -26,6 +26,7 @@
 #include "../../include/mps_b200.h"
 #include "mps_adjoint.cuh"
 #include "mps_kernels.cuh"
+#include "mps_lanes.cuh"
 
 namespace mps {
 
@@ -995,17 +996,17 @@ template <class R, class RN> class Solver final : public SolverBase {
         return nF <= kWarpMost ? 32 : (nF <= kHalfMost ? 16 : (nF <= most ? 8 : 0));
     }
     int list_layout() const { return group_lanes(kGroupMost) ? kListGroup : kListThread; }
-    int group_grid(int g) const { return blocks(nF, 128 / g); }
+    template <class F> static void with_lanes(int g, F&& f) {
+        if (g == 32) f(Lanes<R, RN, 32>());
+        else if (g == 16) f(Lanes<R, RN, 16>());
+        else f(Lanes<R, RN, 8>());
+    }
 
     // pass A, with the mirror table that `a` names
     template <bool D, bool TAPE> void run_pass_a(const PassArgs<R, RN>& a, int ba) {
         const int g = group_lanes(kGroupMostA);
-        if (g == 32)
-            k_pass_a_g<R, RN, D, TAPE, 32><<<group_grid(32), 128, 0, stream>>>(a);
-        else if (g == 16)
-            k_pass_a_g<R, RN, D, TAPE, 16><<<group_grid(16), 128, 0, stream>>>(a);
-        else if (g == 8)
-            k_pass_a_g<R, RN, D, TAPE, 8><<<group_grid(8), 128, 0, stream>>>(a);
+        if (g)
+            with_lanes(g, [&](auto ln) { ln.pass_a(a, D, TAPE, stream); });
         else if (TAPE)
             k_pass_a<R, RN, D, TAPE><<<blocks(nF, ba), ba, 0, stream>>>(a);
         else if (reg_bound & 4)
@@ -1016,12 +1017,8 @@ template <class R, class RN> class Solver final : public SolverBase {
     }
     template <bool D> void run_pass_b(const PassArgs<R, RN>& a, int bb) {
         const int g = group_lanes(kGroupMost);
-        if (g == 32)
-            k_pass_b_g<R, RN, D, 32><<<group_grid(32), 128, 0, stream>>>(a);
-        else if (g == 16)
-            k_pass_b_g<R, RN, D, 16><<<group_grid(16), 128, 0, stream>>>(a);
-        else if (g == 8)
-            k_pass_b_g<R, RN, D, 8><<<group_grid(8), 128, 0, stream>>>(a);
+        if (g)
+            with_lanes(g, [&](auto ln) { ln.pass_b(a, D, stream); });
         else if (reg_bound & 1)
             k_pass_b<R, RN, D, true><<<blocks(nF, bb), bb, 0, stream>>>(a);
         else
@@ -1031,18 +1028,8 @@ template <class R, class RN> class Solver final : public SolverBase {
     template <bool D, bool TAPE> void run_pass_c(const PassArgs<R, RN>& a, int bc) {
         const int g = group_lanes(kGroupMost);
         const bool corr = !TAPE && grad_mode == MPS_GRAD_CORRECTED;
-        if (g == 32 && corr)
-            k_pass_c_g<R, RN, D, false, true, 32><<<group_grid(32), 128, 0, stream>>>(a);
-        else if (g == 32)
-            k_pass_c_g<R, RN, D, TAPE, false, 32><<<group_grid(32), 128, 0, stream>>>(a);
-        else if (g == 16 && corr)
-            k_pass_c_g<R, RN, D, false, true, 16><<<group_grid(16), 128, 0, stream>>>(a);
-        else if (g == 8 && corr)
-            k_pass_c_g<R, RN, D, false, true, 8><<<group_grid(8), 128, 0, stream>>>(a);
-        else if (g == 16)
-            k_pass_c_g<R, RN, D, TAPE, false, 16><<<group_grid(16), 128, 0, stream>>>(a);
-        else if (g == 8)
-            k_pass_c_g<R, RN, D, TAPE, false, 8><<<group_grid(8), 128, 0, stream>>>(a);
+        if (g)
+            with_lanes(g, [&](auto ln) { ln.pass_c(a, D, TAPE, corr, stream); });
         else if (corr)
             k_pass_c<R, RN, D, false, true><<<blocks(nF, bc), bc, 0, stream>>>(a);
         else if (!TAPE && (reg_bound & 2))
@@ -1056,12 +1043,8 @@ template <class R, class RN> class Solver final : public SolverBase {
                         const int8_t* typ) {
         // steps timed per kernel group run on one stream the kernels that they run on two
         const int g = group_lanes(stream == side || timing_on ? kGroupMost : kGroupMostAlone);
-        if (g == 32)
-            k_gen_cull_g<R, RN, D, TAPE, CLS, 32><<<group_grid(32), 128, 0, stream>>>(a, pos, prs, typ);
-        else if (g == 16)
-            k_gen_cull_g<R, RN, D, TAPE, CLS, 16><<<group_grid(16), 128, 0, stream>>>(a, pos, prs, typ);
-        else if (g == 8)
-            k_gen_cull_g<R, RN, D, TAPE, CLS, 8><<<group_grid(8), 128, 0, stream>>>(a, pos, prs, typ);
+        if (g)
+            with_lanes(g, [&](auto ln) { ln.gen(a, D, TAPE, CLS, pos, prs, typ, stream); });
         else
             k_gen_cull<R, RN, D, TAPE, CLS><<<blocks(nF, bg), bg, 0, stream>>>(a, pos, prs, typ);
     }
@@ -1506,12 +1489,7 @@ template <class R, class RN> class Solver final : public SolverBase {
 
     template <bool CORR> void run_ph_grd(const PassArgs<R, RN>& a, int gb, int g) {
         if (diag_on) k_ph_grd<R, RN, true, CORR><<<gb, block, 0, stream>>>(a);
-        else if (g == 32)
-            k_pass_c_g<R, RN, false, false, CORR, 32, true><<<group_grid(32), 128, 0, stream>>>(a);
-        else if (g == 16)
-            k_pass_c_g<R, RN, false, false, CORR, 16, true><<<group_grid(16), 128, 0, stream>>>(a);
-        else if (g == 8)
-            k_pass_c_g<R, RN, false, false, CORR, 8, true><<<group_grid(8), 128, 0, stream>>>(a);
+        else if (g) with_lanes(g, [&](auto ln) { ln.grd(a, CORR, stream); });
         else k_ph_grd<R, RN, false, CORR><<<gb, block, 0, stream>>>(a);
     }
 
@@ -1560,12 +1538,8 @@ template <class R, class RN> class Solver final : public SolverBase {
             case MPS_PHASE_VSCTRM:
                 need_lists();
                 if (diag_on) k_ph_vsc<R, RN, true><<<gb, block, 0, stream>>>(a);
-                else if (lanes(kGroupMostA) == 32)
-                    k_pass_a_g<R, RN, false, false, 32, true><<<group_grid(32), 128, 0, stream>>>(a);
-                else if (lanes(kGroupMostA) == 16)
-                    k_pass_a_g<R, RN, false, false, 16, true><<<group_grid(16), 128, 0, stream>>>(a);
-                else if (lanes(kGroupMostA) == 8)
-                    k_pass_a_g<R, RN, false, false, 8, true><<<group_grid(8), 128, 0, stream>>>(a);
+                else if (const int g = lanes(kGroupMostA))
+                    with_lanes(g, [&](auto ln) { ln.vsc(a, stream); });
                 else k_ph_vsc<R, RN, false><<<gb, block, 0, stream>>>(a);
                 KL();
                 acc_dirty = true;
@@ -1580,12 +1554,8 @@ template <class R, class RN> class Solver final : public SolverBase {
             case MPS_PHASE_CHKCOL:
                 need_lists();
                 if (diag_on) k_ph_col<R, RN, true><<<gb, block, 0, stream>>>(a);
-                else if (lanes(kGroupMost) == 32)
-                    k_pass_b_g<R, RN, false, 32, PASS_COL><<<group_grid(32), 128, 0, stream>>>(a);
-                else if (lanes(kGroupMost) == 16)
-                    k_pass_b_g<R, RN, false, 16, PASS_COL><<<group_grid(16), 128, 0, stream>>>(a);
-                else if (lanes(kGroupMost) == 8)
-                    k_pass_b_g<R, RN, false, 8, PASS_COL><<<group_grid(8), 128, 0, stream>>>(a);
+                else if (const int g = lanes(kGroupMost))
+                    with_lanes(g, [&](auto ln) { ln.col(a, stream); });
                 else k_ph_col<R, RN, false><<<gb, block, 0, stream>>>(a);
                 KL();
                 k_ph_upchkcol<R, RN><<<gb, block, 0, stream>>>(a);
@@ -1595,12 +1565,8 @@ template <class R, class RN> class Solver final : public SolverBase {
             case MPS_PHASE_MKPRS:
                 need_lists();
                 if (diag_on) k_ph_prs<R, RN, true><<<gb, block, 0, stream>>>(a);
-                else if (lanes(kGroupMost) == 32)
-                    k_pass_b_g<R, RN, false, 32, PASS_PRS><<<group_grid(32), 128, 0, stream>>>(a);
-                else if (lanes(kGroupMost) == 16)
-                    k_pass_b_g<R, RN, false, 16, PASS_PRS><<<group_grid(16), 128, 0, stream>>>(a);
-                else if (lanes(kGroupMost) == 8)
-                    k_pass_b_g<R, RN, false, 8, PASS_PRS><<<group_grid(8), 128, 0, stream>>>(a);
+                else if (const int g = lanes(kGroupMost))
+                    with_lanes(g, [&](auto ln) { ln.prs(a, stream); });
                 else k_ph_prs<R, RN, false><<<gb, block, 0, stream>>>(a);
                 KL();
                 break;

@@ -1,12 +1,17 @@
-"""What a handle costs to create and to close: a small scene's no more than a larger one's."""
+"""What a handle costs to create and to close: a small scene's no more than a larger one's, and the
+first of a precision no more than its module takes to load without the kernels of several lanes.
+"""
 from __future__ import annotations
 
+import subprocess
+import sys
 import time
 
 import numpy as np
 import pytest
 
 from mps_cuda_b200 import F32, F64, MPS, SceneDesc, dambreak, dambreak_params
+from mps_cuda_b200.build import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +40,24 @@ def test_a_small_handle_costs_no_more_than_a_larger_one(prec):
             MPS(*a).close()
             best[i] = min(best[i], time.perf_counter() - t0)
     assert best[0] < 1.4 * best[1], best
+
+
+FIRST = """
+import sys, time
+sys.path.insert(0, {root!r})
+from tests.test_gpu_create import F32, F64, MPS, _args
+MPS(*_args((8, 6, 10), F32)).close()
+args = _args((8, 6, 10), F64)
+t0 = time.perf_counter()
+h = MPS(*args)
+print(1e3 * (time.perf_counter() - t0))
+h.close()
+"""
+
+
+def test_the_first_handle_of_a_precision_loads_no_more_than_it_runs():
+    """28 ms with all kernels in one module, 6.5 with those of several lanes in their own."""
+    code = FIRST.format(root=ROOT)
+    run = lambda: float(subprocess.run([sys.executable, "-c", code], check=True, capture_output=True,
+                                       text=True, timeout=120).stdout)
+    assert min(run() for _ in range(3)) < 14.0
