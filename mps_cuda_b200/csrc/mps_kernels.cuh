@@ -9,10 +9,11 @@
 //
 // Fused step (kernel.cu:1904-1935 in three neighbour passes):
 //   pass A: VscTrm + UpPcl1 (+ChkPcl)                            reads x^n, v^n, M1
-//   pass B: ChkCol + MkPrs + GenMRR/MRRinout at (x*, P)          reads x*, v*, walls, M1
-//   pass C: PrsGrdTrm + UpPcl2 (+ChkPcl) + GenMRR/MRRinout at (x^{n+1}, P)  reads x*, P, M2
-// Mirrors produced by pass C are the next step's first generation: GenMRR at the start of
-// the next step (kernel.cu:1906-1908) would read the same positions and pressures.
+//   pass B: ChkCol + MkPrs                                       reads x*, v*, walls, M1
+//   pass C: PrsGrdTrm + UpPcl2 (+ChkPcl)                         reads x*, P, M2
+// GenMRR and MRRinout (k_gen_cull, k_ph_cull) run at (x*, P) between B and C, M2, and at
+// (x^{n+1}, P) after C, the next step's M1: GenMRR at the start of the next step
+// (kernel.cu:1906-1908) would read the same positions and pressures.
 #pragma once
 #include <climits>
 #include <type_traits>

@@ -1,5 +1,7 @@
 // mps_lanes.cu -- the kernels with MPS_LANES lanes per particle, for state in MPS_REAL and number
 // density in MPS_DENSITY. Compiled once for each.
+#include <algorithm>
+
 #include "mps_lanes.cuh"
 
 namespace mps {

@@ -463,8 +463,8 @@ template <class R, class RN> class Solver final : public SolverBase {
     // state, so a state replaced in between (mps_set_state) wastes no build.
     bool tail_pending = false;
     // the handle's second stream (MPS_OPT_OVERLAP), created with the handle, at the device's
-    // highest priority: the work forked to it (the step end's fluid bucket build, the second
-    // mirror generation) gets SMs while the main stream's long kernel has blocks pending;
+    // highest priority: the work forked to it (the step end's mirrors, the second mirror
+    // generation) gets SMs while the main stream's long kernel has blocks pending;
     // the fork and join events
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
